@@ -28,6 +28,10 @@ __device__ __forceinline__ uint32_t pk_addmax(uint32_t a, uint32_t b, uint32_t c
 __device__ __forceinline__ uint32_t pk_max_relu(uint32_t a, uint32_t b) {
   return __vimax_s16x2_relu(a, b);  // max(a, b, 0)
 }
+__device__ __forceinline__ uint32_t pk_addmax_relu(uint32_t a, uint32_t b, uint32_t c) {
+  return __viaddmax_s16x2_relu(a, b, c);  // max(a + b, c, 0)
+}
+__device__ __forceinline__ uint32_t pk_max3(uint32_t a, uint32_t b, uint32_t c) { return __vimax3_s16x2(a, b, c); }
 __device__ __forceinline__ uint32_t pk_max(uint32_t a, uint32_t b) { return __vmaxs2(a, b); }
 __device__ __forceinline__ uint32_t pk_add(uint32_t a, uint32_t b) { return __vadd2(a, b); }
 

@@ -24,17 +24,28 @@
 // its slot records loaded one task ahead, so the loads are off the critical
 // path.
 //
-// Recurrence per cell (literally Gotoh's, as the reference's scalar kernel
-// src/simd.rs:361-374):
-//   H = max(Hdiag + S, E, F, 0)
-//   E' = max(E - extend, H - open)        (E of the next column)
-//   F' = max(F - extend, H - open)        (F of the next row)
-// with DPX ops: t = viaddmax(Hdiag, S, E); H = vimax_relu(t, F);
-// Ho = vadd2(H, -open); E' = viaddmax(E, -ext, Ho); F' = viaddmax(F, -ext, Ho).
+// Recurrence per cell: Gotoh's (the reference's scalar kernel,
+// src/simd.rs:361-374), with both gap states opened from the match state
+//   t = max(Hdiag + S, E, 0);  H = max(t, F)
+//   E' = max(E - x, t - open)        (E of the next column)
+//   F' = max(F - x, t - open)        (F of the next row),  x = min(open, extend)
+// Every H equals the literal recurrence's.  Reopening a gap out of itself
+// costs open where extending costs extend, so opening from H instead of t only
+// matters for open < extend, which x covers; a gap in one sequence directly
+// followed by one in the other scores the same in either order, and the order
+// E then F is kept (t holds E).  The maximum is always reached in some t (a gap
+// never raises it), so `best` follows t.  With H out of the F chain the serial
+// part of a row is one operation (F') instead of three; what bounds the kernel
+// is the ALU pipe: 5.5 operations a cell pair (t, H, half a three-way best, E',
+// F', prmt), the packed add runs beside them on the multiply pipe.  Measured, B200:
+// the 1.2 M-pair PSSM plan 24.93 -> 24.61 ms, 4 M exhaustive pairs 75.6 -> 74.1 ms, one
+// 250 x 300 call 88.7 -> 83.2 us.  Scores by byte dot products on the multiply
+// pipe instead of prmt measured no faster (6.3 against 6.4 T cells/s in a bare cell
+// loop: the third register operand of both pipes' instructions is what limits then).
 //
-// Exactness.  The adds wrap instead of saturating.  If no H anywhere exceeds
+// Exactness.  The adds wrap instead of saturating.  If no t anywhere exceeds
 // T = 32767 - max(0, max score), no sum can leave the int16 range (E, F >=
-// -open-extend, S is int8), so the result is exact; otherwise the first H
+// -open-extend, S is int8), so the result is exact; otherwise the first t
 // above T was itself computed exactly and the pair is flagged for the exact
 // 32-bit kernel.  Rows past the query and columns past a target score 0, which
 // cannot raise the maximum when open, extend >= 0 (the only gap costs this
@@ -203,7 +214,7 @@ __global__ void __launch_bounds__(WARPS * 32) sw16_kernel(const Sw16Params prm) 
   const int grp = lane / G;
   uint2* bnd = prm.scratch + static_cast<size_t>((blockIdx.x * WARPS + warp) * NG + grp) * prm.scratch_stride;
   const uint32_t MOPEN = pk_splat(-prm.open);
-  const uint32_t MEXT = pk_splat(-prm.ext);
+  const uint32_t MEXT = pk_splat(-min(prm.ext, prm.open));
   const uint32_t E0 = MOPEN;  // E of the first column: max(0 - open, -inf)
   const uint32_t F0 = MOPEN;  // F of the first row
   const uint32_t SENTW = 0x15151515u;
@@ -330,17 +341,20 @@ __global__ void __launch_bounds__(WARPS * 32) sw16_kernel(const Sw16Params prm) 
         load_rows8<R>(rows + resB * m_pad, wb);
         uint32_t hd = j == 0 ? hup_prev : h_in[j - 1];
         uint32_t F = f_in[j];
+        uint32_t t_odd = 0;
 #pragma unroll
         for (int k = 0; k < R; ++k) {
           const uint32_t S = prmt(wa[k >> 2], wb[k >> 2], sel_pair(k & 3));
-          const uint32_t t = pk_addmax(hd, S, E[k]);
-          const uint32_t H = pk_max_relu(t, F);
-          best = pk_max(best, H);
-          const uint32_t Ho = pk_add(H, MOPEN);
-          E[k] = pk_addmax(E[k], MEXT, Ho);
-          F = pk_addmax(F, MEXT, Ho);
+          const uint32_t t = pk_addmax_relu(hd, S, E[k]);
+          const uint32_t To = pk_add(t, MOPEN);
           hd = Hp[k];
-          Hp[k] = H;
+          Hp[k] = pk_max(t, F);
+          E[k] = pk_addmax(E[k], MEXT, To);
+          F = pk_addmax(F, MEXT, To);
+          if (k & 1)
+            best = pk_max3(best, t_odd, t);
+          else
+            t_odd = t;
         }
         my_h[j] = Hp[R - 1];
         my_f[j] = F;
