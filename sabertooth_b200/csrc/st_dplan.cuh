@@ -370,9 +370,4 @@ __global__ void __launch_bounds__(256) dp_iota_kernel(uint32_t* v, uint32_t n) {
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) v[i] = i;
 }
 
-__global__ void __launch_bounds__(256) dp_fill_zline_kernel(uint2* z, uint32_t n, uint32_t v) {
-  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) z[i] = make_uint2(0u, v);
-}
-
 }  // namespace st

@@ -251,7 +251,7 @@ static const Sw16Class kClasses[] = {
     ST_CLASS(4, 24, 4),  ST_CLASS(8, 24, 4),  ST_CLASS(16, 24, 4), ST_CLASS(32, 24, 4),
     ST_CLASS_W(4, 28, 4, 4), ST_CLASS_W(8, 28, 4, 4), ST_CLASS_W(16, 28, 4, 4),
     ST_CLASS_W(4, 32, 4, 4), ST_CLASS_W(8, 32, 4, 4), ST_CLASS_W(16, 32, 4, 4),
-    ST_CLASS(32, 16, 2),
+    ST_CLASS(32, 16, 2), ST_CLASS_W(32, 32, 4, 4),
 };
 #undef ST_CLASS
 #undef ST_CLASS_W
@@ -1699,10 +1699,6 @@ static int plan_build(st_ctx* c, const st_pair* pairs, uint64_t n, int32_t open,
     cp.o_wt = carve(cp.wt.size() * sizeof(Sw16WarpTask));
     cp.o_slots = carve(cp.slots.size() * sizeof(Sw16Slot));
   }
-  uint32_t zcols = 64;
-  for (auto& cp : cps)
-    for (auto& w : cp.wt) zcols = std::max(zcols, w.ncols + 8);
-  const size_t o_zline = carve(static_cast<size_t>(zcols) * sizeof(uint2));
   const size_t data_bytes = off;
   const size_t o_cnt = carve((kNumClasses + 2) * 4);
   for (auto& cp : cps) {
@@ -1742,12 +1738,6 @@ static int plan_build(st_ctx* c, const st_pair* pairs, uint64_t n, int32_t open,
     memcpy(h + o_pr, pr.data(), n * 4);
   }
   if (!list32.empty()) memcpy(h + o_list, list32.data(), list32.size() * 4);
-  {
-    // input of a first pass: H = 0 above the query, F = first-row F
-    uint2* z = reinterpret_cast<uint2*>(h + o_zline);
-    const uint2 v = make_uint2(0u, pk_splat(-open));
-    for (uint32_t i = 0; i < zcols; ++i) z[i] = v;
-  }
   {
     // counters: [0, kNumClasses) class work, [kNumClasses] 32-bit work, [kNumClasses+1] list count
     uint32_t* ci = reinterpret_cast<uint32_t*>(h + o_cinit);
@@ -1818,7 +1808,6 @@ static int plan_build(st_ctx* c, const st_pair* pairs, uint64_t n, int32_t open,
     prm.ovf_pairs = d_list;
     prm.work_counter = counters + cp.cls;
     prm.scratch = reinterpret_cast<uint2*>(dbase + cp.o_scratch);
-    prm.zline = reinterpret_cast<const uint2*>(dbase + o_zline);
     prm.scratch_stride = cp.scratch_stride;
     prm.open = open;
     prm.ext = ext;
@@ -2208,13 +2197,11 @@ static int dplan_build(st_ctx* c, const st_pair* pairs, uint64_t n, int32_t open
   // stage 2: sizes known; task arrays, scratch, emission, LPT order
   uint64_t n_slots = 0, n_wt = 0, n_cta = 0;
   uint64_t cta_begin[kNumClasses];
-  uint32_t zcols = 64;
   for (int k = 0; k < kNumClasses; ++k) {
     cta_begin[k] = n_cta;
     n_slots += static_cast<uint64_t>(tot.n_wt[k]) * (64 / kClasses[k].G);
     n_wt += tot.n_wt[k];
     n_cta += tot.n_cta[k];
-    if (tot.n_cta[k]) zcols = std::max(zcols, tot.max_cols[k] + 8);
   }
   for (int k = 0; k < kNumClasses; ++k) {
     if (!tot.n_cta[k]) continue;
@@ -2262,8 +2249,7 @@ static int dplan_build(st_ctx* c, const st_pair* pairs, uint64_t n, int32_t open
   const size_t p_slots = carve(n_slots * sizeof(Sw16Slot)), p_wt = carve(n_wt * sizeof(Sw16WarpTask)),
                p_craw = carve(n_cta * sizeof(Sw16CtaTask)), p_cta = carve(n_cta * sizeof(Sw16CtaTask)),
                p_ck0 = carve(n_cta * 8), p_ck1 = carve(n_cta * 8), p_ci0 = carve(n_cta * 4),
-               p_ci1 = carve(n_cta * 4), p_z = carve(static_cast<size_t>(zcols) * sizeof(uint2)),
-               p_tmp = carve(t_lpt);
+               p_ci1 = carve(n_cta * 4), p_tmp = carve(t_lpt);
   for (auto& cp : plan->classes) {
     if (!cp.scratch_stride) continue;
     const size_t groups = static_cast<size_t>(cp.grid) * kClasses[cp.cls].W * (32 / kClasses[cp.cls].G);
@@ -2294,10 +2280,8 @@ static int dplan_build(st_ctx* c, const st_pair* pairs, uint64_t n, int32_t open
     o.cta_idx_sorted = ci.Current();
     dp_gather_cta_kernel<<<static_cast<uint32_t>((n_cta + 255) / 256), 256, 0, s1>>>(o);
   }
-  uint2* zline = reinterpret_cast<uint2*>(a + p_z);
-  dp_fill_zline_kernel<<<(zcols + 255) / 256, 256, 0, s1>>>(zline, zcols, pk_splat(-open));
   ST_CUDA(cudaGetLastError());
-  c->launches += 3;
+  c->launches += 2;
   ST_CUDA(cudaEventRecord(c->plan_ev, s1));
   ST_CUDA(cudaStreamWaitEvent(st, c->plan_ev, 0));
 
@@ -2319,7 +2303,6 @@ static int dplan_build(st_ctx* c, const st_pair* pairs, uint64_t n, int32_t open
     prm.ovf_pairs = w.list32;
     prm.work_counter = counters + cp.cls;
     prm.scratch = reinterpret_cast<uint2*>(a + cp.o_scratch);
-    prm.zline = zline;
     prm.scratch_stride = cp.scratch_stride;
     prm.open = open;
     prm.ext = ext;
@@ -2853,7 +2836,7 @@ struct SwCall {
   int32_t open = 0, ext = 0;
   bool use16 = false, wait = false;
   size_t tbytes = 0, o_off = 0, o_len = 0, o_pt = 0, o_pq = 0, o_pc = 0, o_pr = 0, o_cta = 0, o_wt = 0, o_slots = 0,
-         o_cnt = 0, o_list = 0, o_zline = 0, total = 0;
+         o_cnt = 0, o_list = 0, total = 0;
   DeviceProfiles pv;
 };
 
@@ -2871,7 +2854,7 @@ static int sw_score_prepare(st_ctx* c, CallSlot* sl, uint32_t profile, uint32_t 
   }
   // staging block (one host->device copy per call):
   //   [target codes, padded] [db offset u64] [db length u32] [pair: target u32, query u32, center i32, radius i32]
-  //   [cta task] [warp task] [slots x64] [counters x(kNumClasses+2)] [32-bit list u32] [first-pass boundary]
+  //   [cta task] [warp task] [slots x64] [counters x(kNumClasses+2)] [32-bit list u32]
   // and, behind it in the pinned block only, the score and kernel tag the kernels write
   w->profile = profile;
   w->n = n;
@@ -2892,9 +2875,6 @@ static int sw_score_prepare(st_ctx* c, CallSlot* sl, uint32_t profile, uint32_t 
   w->o_slots = o; o += 64 * sizeof(Sw16Slot);
   w->o_cnt = o; o += (kNumClasses + 2) * 4;
   w->o_list = o; o += 4;
-  o = up16(o);
-  w->o_zline = o; o += (static_cast<size_t>(std::max<uint32_t>(32, static_cast<uint32_t>(up16(n)))) +
-                        static_cast<size_t>(32 * 4 + 16)) * sizeof(uint2);
   w->total = up16(o);
   w->use16 = pm.fits8 && gaps16_ok(open, ext);
   w->k = 0;
@@ -2960,11 +2940,6 @@ static int sw_score_launch(CallSlot* sl, const uint8_t* target, const SwCall& w,
   uint32_t* cnt = reinterpret_cast<uint32_t*>(h + w.o_cnt);
   if (!w.use16) cnt[kNumClasses + 1] = 1;  // the pair goes straight to the 32-bit list
   *reinterpret_cast<uint32_t*>(h + w.o_list) = 0;
-  {
-    uint2* z = reinterpret_cast<uint2*>(h + w.o_zline);
-    const size_t nz = (w.total - w.o_zline) / sizeof(uint2);
-    for (size_t i = 0; i < nz; ++i) z[i] = make_uint2(0u, pk_splat(-w.open));
-  }
   *res_off = w.total;
   int32_t* h_res = sl->pin.as<int32_t>(*res_off);
   h_res[0] = 0;
@@ -2996,7 +2971,6 @@ static int sw_score_launch(CallSlot* sl, const uint8_t* target, const SwCall& w,
     prm.ovf_pairs = d_list;
     prm.work_counter = d_cnt + w.k;
     prm.scratch = sl->scratch.as<uint2>();
-    prm.zline = reinterpret_cast<const uint2*>(d + w.o_zline);
     prm.scratch_stride = w.sstride;
     prm.open = w.open;
     prm.ext = w.ext;

@@ -88,16 +88,16 @@ struct Sw16Params {
   uint32_t* ovf_pairs;
   uint32_t* work_counter; // next CTA task (reset before each launch)
   uint2* scratch;         // pass boundary rows, scratch_stride entries per group
-  const uint2* zline;     // (H, F) = (0, first-row F) for every column: the input of a first pass
   uint32_t scratch_stride;
   int32_t open, ext;
 };
 
 constexpr uint32_t kNoPair = 0xFFFFFFFFu;
 
-// control word: column (16 bits) | pass (8) | task slot (3) | last step of the task | idle
-constexpr uint32_t kCtlLast = 1u << 27;
-constexpr uint32_t kCtlIdle = 1u << 28;
+// control word: events, with the pass (bits 16-23) and the task slot (24-26) they belong to
+constexpr uint32_t kCtlLast = 1u << 27;   // last step of the task
+constexpr uint32_t kCtlFirst = 1u << 28;  // first step of a pass
+constexpr uint32_t kCtlMore = 1u << 29;   // a pass that is not the last: its bottom row is kept
 constexpr int kSlotRing = 8;
 
 template <int G, int R, int C>
@@ -144,6 +144,17 @@ __device__ __forceinline__ uint32_t load_codes(const uint8_t* t, uint32_t len16,
   if constexpr (C == 4) return __ldg(reinterpret_cast<const uint32_t*>(t + c));
   else if constexpr (C == 2) return __ldg(reinterpret_cast<const uint16_t*>(t + c));
   else return __ldg(t + c);
+}
+
+// acc + (byte j of bytes) * mul: the 16-bit x byte dot product with mul in the half that meets byte j
+// (bits 16-31 for odd j) and zero in the other.
+__device__ __forceinline__ uint32_t dot_byte(int j, uint32_t mul, uint32_t bytes, uint32_t acc) {
+  uint32_t d;
+  if (j < 2)
+    asm("dp2a.lo.u32.u32 %0, %1, %2, %3;" : "=r"(d) : "r"(mul), "r"(bytes), "r"(acc));
+  else
+    asm("dp2a.hi.u32.u32 %0, %1, %2, %3;" : "=r"(d) : "r"(mul), "r"(bytes), "r"(acc));
+  return d;
 }
 
 template <int C>
@@ -198,8 +209,18 @@ __device__ __forceinline__ Sw16Pair2 load_pair2(const Sw16Params& prm, uint32_t 
 // Persistent kernel: CTAs pull CTA tasks (one query each) from a global
 // counter and stage the query's int8 profile in shared memory; each warp then
 // streams the CTA task's warp tasks, claimed from a shared counter.
+//
+// Beside the cells a step costs its 3 + 2C shuffles, the residues' row offsets
+// (one dot product each, dot_byte) and the feeder's loads; the decisions of the
+// stream (pass, task, idle) are taken only at the end of a pass, and the first
+// pass reads no boundary line.  Registers are the other lever: asking for three
+// CTAs of four warps (R >= 28, up to 168 registers) or three of eight (R = 8)
+// and two of eight otherwise lets the profile loads of a column be issued ahead
+// of its rows.  Streamed cells/s of single classes on the 1.2 M-pair PSSM batch,
+// before -> after: <8,32> 5.23 -> 5.79 T, <16,32> 5.13 -> 5.77, <16,24> 5.40 -> 5.67,
+// <8,24> 5.41 -> 5.60, <16,20> 5.20 -> 5.54, <8,8> 4.57 -> 4.68 (4.25 with two CTAs).
 template <int G, int R, int C, int WARPS>
-__global__ void __launch_bounds__(WARPS * 32) sw16_kernel(const Sw16Params prm) {
+__global__ void __launch_bounds__(WARPS * 32, WARPS == 4 || R == 8 ? 3 : 2) sw16_kernel(const Sw16Params prm) {
   using Tile = Sw16Tile<G, R, C>;
   constexpr int NG = Tile::kGroups;
   constexpr uint32_t FULL = 0xFFFFFFFFu;
@@ -271,13 +292,19 @@ __global__ void __launch_bounds__(WARPS * 32) sw16_kernel(const Sw16Params prm) 
     Sw16WarpTask wt_nxt = have_nxt ? prm.warp_tasks[w_nxt] : Sw16WarpTask{0, 0};
     Sw16Pair2 nxt{};
     if (have_nxt && feeder) nxt = load_pair2(prm, wt_nxt.slot_begin, grp);
-    int u_col = 0, u_pass = 0, u_seq = 0, drain = 0;
     if (feeder) {
       s_pair[warp][grp][0][0] = cur.pA;
       s_pair[warp][grp][0][1] = cur.pB;
       s_best[warp][grp][0][0] = 0;
       s_best[warp][grp][0][1] = 0;
     }
+    // Lane 0's position: column u_col of pass u_pass of task u_seq.  The control word of an ordinary step is
+    // u_ctl; the first and the last step of a pass add their events, so an ordinary step takes no decisions
+    // beyond comparing its column with the pass's end.
+    int u_col = 0, u_pass = 0, u_seq = 0, drain = 0;
+    int u_end = static_cast<int>(wt_cur.ncols);  // columns of the pass
+    uint32_t u_ctl = P > 1 ? kCtlMore : 0u;
+    uint32_t u_last = P > 1 ? 0u : kCtlLast;     // the event of the pass's last step
 
     // per-lane wavefront state
     uint32_t Hp[R], E[R];
@@ -287,8 +314,11 @@ __global__ void __launch_bounds__(WARPS * 32) sw16_kernel(const Sw16Params prm) 
       E[k] = E0;
     }
     uint32_t best = 0, hup_prev = 0;
+    uint32_t row0 = static_cast<uint32_t>(gl * R);  // this lane's first row of its pass
+    uint32_t my_col = 0;                            // its column
+    const uint32_t mul_lo = m_pad, mul_hi = m_pad << 16;
     // outgoing registers: a lane's outputs for the lane below (the feeder: lane 0's next inputs)
-    uint32_t my_ctl = kCtlIdle, my_rA = SENTW, my_rB = SENTW;
+    uint32_t my_ctl = 0, my_rA = SENTW, my_rB = SENTW;
     uint32_t my_h[C], my_f[C];
 #pragma unroll
     for (int j = 0; j < C; ++j) {
@@ -296,7 +326,7 @@ __global__ void __launch_bounds__(WARPS * 32) sw16_kernel(const Sw16Params prm) 
       my_f[j] = F0;
     }
     if (feeder) {  // lane 0's first step: column 0, pass 0 of the first task
-      my_ctl = 0u;
+      my_ctl = kCtlFirst | u_ctl;
       my_rA = load_codes<C>(cur.tA, cur.lenA, 0);
       my_rB = load_codes<C>(cur.tB, cur.lenB, 0);
     }
@@ -316,29 +346,81 @@ __global__ void __launch_bounds__(WARPS * 32) sw16_kernel(const Sw16Params prm) 
       my_ctl = ctl;
       my_rA = rA;
       my_rB = rB;
-      const int col = static_cast<int>(ctl & 0xFFFFu);
-      const int pass = static_cast<int>((ctl >> 16) & 0xFFu);
-      // first column of a pass (or idle): left border H = 0, first-column E. The
-      // groups of a warp move in step, so lane l of every group resets on the
-      // same steps: the branch is skipped on the other steps of a pass.
-      if (__any_sync(FULL, col == 0)) {
-        if (col == 0) {
+      // lane 0's next step (uniform across the warp)
+      uint32_t n_ctl = u_ctl;
+      u_col += C;
+      if (u_col == u_end) {
+        if (have) {
+          n_ctl = kCtlFirst;
+          if (++u_pass == P) {  // task done: the pre-claimed task becomes current, claim the one after
+            u_pass = 0;
+            ++u_seq;
+            have = have_nxt;
+            wt_cur = wt_nxt;
+            cur = nxt;
+            if (have) {
+              const int slot = u_seq & (kSlotRing - 1);
+              if (feeder) {
+                s_pair[warp][grp][slot][0] = cur.pA;
+                s_pair[warp][grp][slot][1] = cur.pB;
+                s_best[warp][grp][slot][0] = 0;
+                s_best[warp][grp][slot][1] = 0;
+              }
+              w_nxt = claim();
+              have_nxt = w_nxt < task.wt_end;
+              if (have_nxt) {
+                wt_nxt = prm.warp_tasks[w_nxt];
+                if (feeder) nxt = load_pair2(prm, wt_nxt.slot_begin, grp);
+              }
+              u_end = static_cast<int>(wt_cur.ncols);
+            }
+          }
+          if (have) {
+            const uint32_t at = (static_cast<uint32_t>(u_pass) << 16) |
+                                (static_cast<uint32_t>(u_seq & (kSlotRing - 1)) << 24);
+            u_ctl = u_pass + 1 < P ? kCtlMore : 0u;
+            u_last = u_pass + 1 < P ? 0u : kCtlLast | at;
+            n_ctl |= u_ctl | at;
+            u_col = 0;
+          } else {  // idle steps until the last lane has finished
+            cur.lenA = cur.lenB = 0;
+            u_ctl = u_last = n_ctl = 0u;
+            u_col = 0;
+            u_end = -C;
+          }
+        }
+      } else if (u_col + C == u_end) {
+        n_ctl |= u_last;
+      }
+      if (!have) ++drain;
+      uint32_t nA = SENTW, nB = SENTW;
+      if (feeder) {  // its residues, on their way while this step is computed
+        nA = load_codes<C>(cur.tA, cur.lenA, u_col);
+        nB = load_codes<C>(cur.tB, cur.lenB, u_col);
+      }
+      // first column of a pass: left border H = 0, first-column E. The groups of a
+      // warp move in step, so lane l of every group resets on the same steps: the
+      // branch is skipped on the other steps of a pass.
+      if (__any_sync(FULL, (ctl & kCtlFirst) != 0)) {
+        if (ctl & kCtlFirst) {
 #pragma unroll
           for (int k = 0; k < R; ++k) {
             Hp[k] = 0;
             E[k] = E0;
           }
           hup_prev = 0;
+          my_col = 0;
+          row0 = ((ctl >> 16) & 0xFFu) * (G * R) + gl * R;
         }
       }
-      const int8_t* rows = prof_s + pass * (G * R) + gl * R;
 #pragma unroll
       for (int j = 0; j < C; ++j) {
-        const uint32_t resA = (rA >> (8 * j)) & 0xFFu;
-        const uint32_t resB = (rB >> (8 * j)) & 0xFFu;
+        // row0 + residue * m_pad: one 16-bit x byte dot product picks the byte and multiplies it
+        const uint32_t oA = dot_byte(j, j & 1 ? mul_hi : mul_lo, rA, row0);
+        const uint32_t oB = dot_byte(j, j & 1 ? mul_hi : mul_lo, rB, row0);
         uint32_t wa[Tile::kWords], wb[Tile::kWords];
-        load_rows8<R>(rows + resA * m_pad, wa);
-        load_rows8<R>(rows + resB * m_pad, wb);
+        load_rows8<R>(prof_s + oA, wa);
+        load_rows8<R>(prof_s + oB, wb);
         uint32_t hd = j == 0 ? hup_prev : h_in[j - 1];
         uint32_t F = f_in[j];
         uint32_t t_odd = 0;
@@ -387,56 +469,23 @@ __global__ void __launch_bounds__(WARPS * 32) sw16_kernel(const Sw16Params prm) 
         }
       }
       // the bottom row of a pass that is not the last goes to the scratch line
-      if (feeder && !(ctl & kCtlIdle) && pass + 1 < P) store_bnd<C>(bnd + col, my_h, my_f);
+      if (feeder && (ctl & kCtlMore)) store_bnd<C>(bnd + my_col, my_h, my_f);
+      my_col += C;
       __syncwarp();
-
-      // advance lane 0's stream position (uniform across the warp)
-      if (have) {
-        u_col += C;
-        if (u_col == static_cast<int>(wt_cur.ncols)) {
-          u_col = 0;
-          if (++u_pass == P) {  // task done: the pre-claimed task becomes current, claim the one after
-            u_pass = 0;
-            ++u_seq;
-            have = have_nxt;
-            w_cur = w_nxt;
-            wt_cur = wt_nxt;
-            cur = nxt;
-            if (have) {
-              const int slot = u_seq & (kSlotRing - 1);
-              if (feeder) {
-                s_pair[warp][grp][slot][0] = cur.pA;
-                s_pair[warp][grp][slot][1] = cur.pB;
-                s_best[warp][grp][slot][0] = 0;
-                s_best[warp][grp][slot][1] = 0;
-              }
-              w_nxt = claim();
-              have_nxt = w_nxt < task.wt_end;
-              if (have_nxt) {
-                wt_nxt = prm.warp_tasks[w_nxt];
-                if (feeder) nxt = load_pair2(prm, wt_nxt.slot_begin, grp);
-              }
-            }
-          }
-        }
-      } else {
-        ++drain;
-      }
-      if (!have && drain >= G) break;
+      if (drain >= G) break;  // the last lane has done the last step
       // the feeder's outgoing registers become lane 0's inputs for the next step
       if (feeder) {
-        if (have) {
-          const bool last = (u_pass == P - 1) && (u_col + C == static_cast<int>(wt_cur.ncols));
-          my_ctl = static_cast<uint32_t>(u_col) | (static_cast<uint32_t>(u_pass) << 16) |
-                   (static_cast<uint32_t>(u_seq & (kSlotRing - 1)) << 24) | (last ? kCtlLast : 0u);
-          my_rA = load_codes<C>(cur.tA, cur.lenA, u_col);
-          my_rB = load_codes<C>(cur.tB, cur.lenB, u_col);
-          load_bnd<C>((u_pass > 0 ? bnd : prm.zline) + u_col, my_h, my_f);
-        } else {
-          my_ctl = kCtlIdle;
-          my_rA = SENTW;
-          my_rB = SENTW;
-          load_bnd<C>(prm.zline, my_h, my_f);
+        my_ctl = n_ctl;
+        my_rA = nA;
+        my_rB = nB;
+        if (u_pass > 0) {
+          load_bnd<C>(bnd + u_col, my_h, my_f);
+        } else {  // above the query's first row: H = 0, first-row F
+#pragma unroll
+          for (int j = 0; j < C; ++j) {
+            my_h[j] = 0;
+            my_f[j] = F0;
+          }
         }
       }
     }

@@ -57,13 +57,13 @@ inline float tuning_default_rate(int G, int R, int C) {
     int G, R;
     float rate;
   } kRates[] = {
-      {4, 8, 3.826f}, {8, 8, 4.573f}, {16, 8, 4.578f}, {32, 8, 4.483f},
-      {4, 12, 3.832f}, {8, 12, 4.817f}, {16, 12, 4.879f}, {32, 12, 4.665f},
-      {4, 16, 3.986f}, {8, 16, 4.959f}, {16, 16, 5.011f}, {32, 16, 4.788f},
-      {4, 20, 4.451f}, {8, 20, 5.240f}, {16, 20, 5.198f}, {32, 20, 5.069f},
-      {4, 24, 4.680f}, {8, 24, 5.405f}, {16, 24, 5.399f}, {32, 24, 5.128f},
-      {4, 28, 5.289f}, {8, 28, 5.362f}, {16, 28, 4.958f}, {4, 32, 5.194f},
-      {8, 32, 5.233f}, {16, 32, 5.126f},
+      {4, 8, 3.737f}, {8, 8, 4.675f}, {16, 8, 4.779f}, {32, 8, 4.641f},
+      {4, 12, 3.677f}, {8, 12, 4.824f}, {16, 12, 4.983f}, {32, 12, 4.887f},
+      {4, 16, 4.073f}, {8, 16, 5.130f}, {16, 16, 5.240f}, {32, 16, 5.070f},
+      {4, 20, 4.443f}, {8, 20, 5.446f}, {16, 20, 5.541f}, {32, 20, 5.424f},
+      {4, 24, 4.677f}, {8, 24, 5.595f}, {16, 24, 5.670f}, {32, 24, 5.477f},
+      {4, 28, 5.082f}, {8, 28, 5.273f}, {16, 28, 5.294f}, {4, 32, 5.581f},
+      {8, 32, 5.792f}, {16, 32, 5.771f}, {32, 32, 5.663f},
   };
   for (const auto& r : kRates)
     if (r.G == G && r.R == R) return r.rate;
