@@ -1,6 +1,6 @@
 // Device-side planning of a batch of (profile, target) pairs for the packed
 // 16-bit kernel: the same plan the host planner builds (pairs grouped by
-// query, targets longest first, a tile class per query from the class rates,
+// query, targets longest first, a tile class per query from the class rates and its critical path,
 // warp tasks of 64/G targets, CTA tasks capped at one CTA's share of their
 // class, CTA tasks longest first), built on the GPU so that a large batch
 // needs no host pass over its pairs beyond validation.
@@ -9,8 +9,10 @@
 //   classify   pair -> route (empty / 16-bit / 32-bit), SoA copies for the
 //              32-bit kernel, a sort key (query, target length descending)
 //   sort       radix sort of the keys (stable: equal keys keep pair order)
-//   pick       per query: tile class by estimated time, warp-task count,
-//              per-class totals (atomics)
+//   estimate   per query and class: the chip's time for the query's streamed
+//              cells; the batch's time with every query in its cheapest class
+//   pick       per query: tile class by that time and its critical path
+//              (tune_objective), warp-task count, per-class totals (atomics)
 //   split      per query: CTA-task count under the class's cost cap
 //   order      queries sorted by class, exclusive scans of slots, warp tasks
 //              and CTA tasks in that order (class segments are contiguous)
@@ -23,6 +25,7 @@
 #include "../../include/sabertooth_b200.h"
 #include "st_common.cuh"
 #include "st_sw16.cuh"
+#include "st_tuning.h"
 
 namespace st {
 
@@ -53,6 +56,7 @@ struct DpTotals {
   uint32_t max_cols[kDpMaxClasses];        // widest warp task
   uint32_t max_cols_multi[kDpMaxClasses];  // widest warp task of a query with several passes
   unsigned long long cost[kDpMaxClasses];  // sum of warp-task costs (the CTA-task cap)
+  unsigned long long batch_ps;             // the batch's time with every query in its cheapest class
 };
 
 struct DpIn {
@@ -73,6 +77,7 @@ struct DpWork {
   unsigned long long *keys, *keys_alt;
   uint32_t *vals, *vals_alt;  // after the sort: vals_sorted = pair ids grouped by query
   const uint32_t* vals_sorted;
+  const unsigned long long* keys_sorted;
   uint32_t* list32;      // 32-bit list (static entries first, 16-bit overflows appended by the kernels)
   uint32_t* list_count;  // device count of list32
   // per query
@@ -83,6 +88,7 @@ struct DpWork {
   uint32_t *a_slots, *a_wt, *a_cta;  // counts in class order, then their exclusive scans
   uint32_t *o_slots, *o_wt, *o_cta;
   DpTotals* totals;
+  double* est;  // per query and class: the chip's time for the query, picoseconds
 };
 
 struct DpOut {
@@ -129,6 +135,11 @@ __device__ __forceinline__ DpShape dp_shape(const DpClass& k, uint32_t m) {
   s.minc = s.P > 1 ? max(32u, dp_up16(k.C * k.G)) : 32u;
   s.step_cost = k.R * k.C + 8;
   return s;
+}
+
+// Cost of a warp task whose longest target has tl residues: its wavefront steps, each of step_cost.
+__device__ __forceinline__ unsigned long long dp_wt_cost(const DpClass& c, const DpShape& sh, uint32_t tl) {
+  return static_cast<unsigned long long>(sh.P) * (max(sh.minc, dp_up4(tl)) / c.C) * sh.step_cost;
 }
 
 __device__ __forceinline__ unsigned long long dp_warp_sum(unsigned long long v) {
@@ -182,7 +193,52 @@ __global__ void __launch_bounds__(256) dp_list_keys_kernel(const DpIn in, const 
   }
 }
 
-// ---- pick: one warp per query ----
+// Length of a query's j-th target, longest first, from its sort key.
+struct DpLens {
+  const unsigned long long* key;
+  uint32_t tmask;
+  __device__ __forceinline__ uint32_t operator()(uint32_t j) const {
+    return tmask - (static_cast<uint32_t>(key[j]) & tmask);
+  }
+};
+__device__ __forceinline__ DpLens dp_lens(const DpIn& in, const DpWork& w, uint32_t q) {
+  return DpLens{w.keys_sorted + w.qstart[q], (in.tbits >= 32) ? 0xFFFFFFFFu : ((1u << in.tbits) - 1)};
+}
+
+// ---- estimate: one CTA per query, a warp per class ----
+// Streamed cells over the rate for every class (as tuning_estimate), and the batch's total of the cheapest.
+__global__ void __launch_bounds__(256) dp_estimate_kernel(const DpIn in, const DpWork w, const DpClasses cls) {
+  __shared__ double s_est[kDpMaxClasses];
+  const uint32_t q = blockIdx.x;
+  const uint32_t np = w.qcnt[q];
+  if (np == 0) return;
+  const int lane = threadIdx.x & 31;
+  const uint32_t m = in.prof.qlen[q];
+  const DpLens tl = dp_lens(in, w, q);
+  for (int k = threadIdx.x >> 5; k < cls.n; k += blockDim.x >> 5) {
+    const DpClass& c = cls.c[k];
+    const DpShape sh = dp_shape(c, m);
+    double v = 1e300;
+    if (sh.mpad <= c.max_mpad) {
+      const uint32_t nw = (np + c.S - 1) / c.S;
+      unsigned long long cols = 0;
+      for (uint32_t x = lane; x < nw; x += 32) cols += max(sh.minc, dp_up4(tl(x * c.S)));
+      cols = dp_warp_sum(cols);
+      v = static_cast<double>(cols) * c.S * sh.mpad;
+      v = c.rate > 0.0f ? v / c.rate : v * 1e150;
+    }
+    if (lane == 0) s_est[k] = w.est[static_cast<size_t>(q) * kDpMaxClasses + k] = v;
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    double best = 0.0;
+    for (int k = 0; k < cls.n; ++k)
+      if (s_est[k] < 1e140 && (best == 0.0 || s_est[k] < best)) best = s_est[k];
+    atomicAdd(&w.totals->batch_ps, static_cast<unsigned long long>(best));
+  }
+}
+
+// ---- pick: one warp per query, a lane per class ----
 __global__ void __launch_bounds__(256) dp_pick_kernel(const DpIn in, const DpWork w, const DpClasses cls) {
   const uint32_t q = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
@@ -195,51 +251,49 @@ __global__ void __launch_bounds__(256) dp_pick_kernel(const DpIn in, const DpWor
     w.nwt[q] = 0;
   }
   if (np == 0) return;
-  const uint32_t* v = w.vals_sorted + w.qstart[q];
-  auto tl_at = [&](uint32_t j) { return in.db.length[w.pt[v[j]]]; };
+  const DpLens tl = dp_lens(in, w, q);
   unsigned long long sum = 0;
-  for (uint32_t j = lane; j < np; j += 32) sum += tl_at(j);
+  for (uint32_t j = lane; j < np; j += 32) sum += tl(j);
   sum = dp_warp_sum(sum);
   const uint32_t m = in.prof.qlen[q];
   const uint32_t mean_n = static_cast<uint32_t>(sum / np);
+  const double* est = w.est + static_cast<size_t>(q) * kDpMaxClasses;
   int best = -1;
   const int forced = cls.table[dp_mbin(m)][dp_nbin(mean_n)];
-  if (forced >= 0 && forced < cls.n && dp_shape(cls.c[forced], m).mpad <= cls.c[forced].max_mpad) best = forced;
-  // least streamed cells / rate over the classes with a rate; if none of them
-  // stages this query, least streamed cells over every class that does
-  for (int pass = 0; pass < 2 && best < 0; ++pass) {
-    double bt = 1e300;
-    for (int k = 0; k < cls.n; ++k) {
-      const DpClass& c = cls.c[k];
-      if (pass == 0 && !(c.rate > 0.0f)) continue;
+  if (forced >= 0 && forced < cls.n && est[forced] < 1e300) {
+    best = forced;
+  } else {
+    double v = 1e300;
+    if (lane < cls.n && est[lane] < 1e300) {
+      const DpClass& c = cls.c[lane];
       const DpShape sh = dp_shape(c, m);
-      if (sh.mpad > c.max_mpad) continue;
-      const uint32_t nw = (np + c.S - 1) / c.S;
-      unsigned long long cols = 0;
-      for (uint32_t x = lane; x < nw; x += 32) cols += max(sh.minc, dp_up4(tl_at(x * c.S)));
-      cols = dp_warp_sum(cols);
-      const double t = static_cast<double>(cols) * c.S * sh.mpad / (pass == 0 ? c.rate : 1.0f);
-      if (t < bt) {
-        bt = t;
-        best = k;
+      v = tune_objective(est[lane], tune_crit_ps(c.G, c.R, c.C, sh.P, max(sh.minc, dp_up4(tl(0)))),
+                         static_cast<double>(w.totals->batch_ps));
+    }
+    int k = lane;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      const double ov = __shfl_xor_sync(0xFFFFFFFFu, v, o);
+      const int ok = __shfl_xor_sync(0xFFFFFFFFu, k, o);
+      if (ov < v || (ov == v && ok < k)) {
+        v = ov;
+        k = ok;
       }
     }
+    if (v < 1e300) best = k;
   }
   if (best < 0) return;  // cannot happen: the 16-bit route admits only queries some class stages
   const DpClass& c = cls.c[best];
   const DpShape sh = dp_shape(c, m);
   const uint32_t nw = (np + c.S - 1) / c.S;
   unsigned long long cost = 0;
-  for (uint32_t x = lane; x < nw; x += 32) {
-    const uint32_t nc = max(sh.minc, dp_up4(tl_at(x * c.S)));
-    cost += static_cast<unsigned long long>(sh.P) * (nc / c.C) * sh.step_cost;
-  }
+  for (uint32_t x = lane; x < nw; x += 32) cost += dp_wt_cost(c, sh, tl(x * c.S));
   cost = dp_warp_sum(cost);
   if (lane == 0) {
     w.qclass[q] = static_cast<uint32_t>(best);
     w.qkey[q] = static_cast<uint32_t>(best);
     w.nwt[q] = nw;
-    const uint32_t nc0 = max(sh.minc, dp_up4(tl_at(0)));
+    const uint32_t nc0 = max(sh.minc, dp_up4(tl(0)));
     atomicAdd(&w.totals->n_query[best], 1u);
     atomicAdd(&w.totals->n_wt[best], nw);
     atomicAdd(&w.totals->cost[best], cost);
@@ -249,50 +303,73 @@ __global__ void __launch_bounds__(256) dp_pick_kernel(const DpIn in, const DpWor
   }
 }
 
-// CTA tasks of one query: consecutive warp tasks; a task ends at 128 warp
-// tasks or, once it holds W of them, when its cost would pass the cap.
-// f(w0, w1, cost) for each, in order.
+// CTA tasks of one query, by one warp: consecutive warp tasks in units of tune_cta_unit; a task ends at 128 warp
+// tasks or where the query's running cost passes a multiple of the class's cap (its cost over two CTAs on every
+// SM).  f(t, w0, w1, cost) is called once for each task t by some lane; returns the number of tasks.
 template <class F>
-__device__ __forceinline__ void dp_for_each_cta(const DpClass& c, const DpShape& sh, uint32_t nw,
-                                                const uint32_t* v, const uint32_t* pt, const uint32_t* len,
-                                                unsigned long long cap, F&& f) {
-  uint32_t w0 = 0;
-  unsigned long long acc = 0;
-  for (uint32_t x = 0; x < nw; ++x) {
-    const uint32_t nc = max(sh.minc, dp_up4(len[pt[v[x * c.S]]]));
-    const unsigned long long cw = static_cast<unsigned long long>(sh.P) * (nc / c.C) * sh.step_cost;
-    const uint32_t cnt = x - w0;
-    if (cnt == 128u || (cnt >= c.W && acc + cw > cap)) {
-      f(w0, x, acc);
-      w0 = x;
-      acc = 0;
+__device__ __forceinline__ uint32_t dp_for_each_cta(const DpClasses& cls, const DpTotals* tot, uint32_t k,
+                                                    const DpShape& sh, uint32_t nw, const DpLens& tl, F&& f) {
+  const DpClass& c = cls.c[k];
+  const int lane = threadIdx.x & 31;
+  unsigned long long wt_total = lane < cls.n ? tot->n_wt[lane] : 0u;
+  wt_total = dp_warp_sum(wt_total);
+  const uint32_t unit = tune_cta_unit(wt_total, cls.sms, c.W);
+  const unsigned long long cap = max(1ull, tot->cost[k] / (2ull * cls.sms));
+  unsigned long long base = 0;         // cost of the warp tasks before this round's
+  unsigned long long last_bucket = 0;  // of the last unit of the round before
+  unsigned long long open_cost = 0;    // running cost at the start of the open task
+  uint32_t n = 0, open_w = 0;          // tasks begun, first warp task of the open one
+  for (uint32_t x0 = 0; x0 < nw; x0 += 32) {
+    const uint32_t x = x0 + lane;
+    const unsigned long long cw = x < nw ? dp_wt_cost(c, sh, tl(x * c.S)) : 0ull;
+    unsigned long long incl = cw;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const unsigned long long y = __shfl_up_sync(0xFFFFFFFFu, incl, o);
+      if (lane >= o) incl += y;
     }
-    acc += cw;
+    const unsigned long long excl = base + incl - cw;
+    const unsigned long long bucket = excl / cap;
+    unsigned long long before = __shfl_up_sync(0xFFFFFFFFu, bucket, unit);
+    if (lane < static_cast<int>(unit)) before = last_bucket;
+    const bool begin = x < nw && x % unit == 0 && (x == 0 || bucket != before || x % 128u == 0);
+    const uint32_t mask = __ballot_sync(0xFFFFFFFFu, begin);
+    const uint32_t lower = mask & ((1u << lane) - 1u);
+    // the task before mine: begun by the next lower lane of the ballot, or the open one
+    const int prev = lower ? 31 - __clz(lower) : 0;
+    const unsigned long long pc = __shfl_sync(0xFFFFFFFFu, excl, prev);
+    if (begin && x > 0)
+      f(n + __popc(lower) - 1, lower ? x0 + prev : open_w, x, excl - (lower ? pc : open_cost));
+    if (mask) {
+      const int top = 31 - __clz(mask);
+      open_w = x0 + top;
+      open_cost = __shfl_sync(0xFFFFFFFFu, excl, top);
+      n += __popc(mask);
+    }
+    base += __shfl_sync(0xFFFFFFFFu, incl, 31);
+    last_bucket = __shfl_sync(0xFFFFFFFFu, bucket, 32 - unit);
   }
-  if (nw > w0) f(w0, nw, acc);
+  if (lane == 0 && n) f(n - 1, open_w, nw, base - open_cost);
+  return n;
 }
 
-__device__ __forceinline__ unsigned long long dp_cap(const DpClasses& cls, const DpTotals* t, uint32_t k) {
-  const unsigned long long cap = t->cost[k] / (2ull * cls.sms);
-  return cap ? cap : 1ull;
-}
-
-// ---- split: one thread per query ----
+// ---- split: one warp per query ----
 __global__ void __launch_bounds__(256) dp_split_kernel(const DpIn in, const DpWork w, const DpClasses cls) {
-  const uint32_t q = blockIdx.x * blockDim.x + threadIdx.x;
+  const uint32_t q = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const int lane = threadIdx.x & 31;
   if (q >= in.n_prof) return;
   const uint32_t k = w.qclass[q];
   if (k == kDpNoClass) {
-    w.ncta[q] = 0;
+    if (lane == 0) w.ncta[q] = 0;
     return;
   }
-  const DpClass& c = cls.c[k];
-  const DpShape sh = dp_shape(c, in.prof.qlen[q]);
-  uint32_t n = 0;
-  dp_for_each_cta(c, sh, w.nwt[q], w.vals_sorted + w.qstart[q], w.pt, in.db.length, dp_cap(cls, w.totals, k),
-                  [&](uint32_t, uint32_t, unsigned long long) { ++n; });
-  w.ncta[q] = n;
-  atomicAdd(&w.totals->n_cta[k], n);
+  const DpShape sh = dp_shape(cls.c[k], in.prof.qlen[q]);
+  const uint32_t n = dp_for_each_cta(cls, w.totals, k, sh, w.nwt[q], dp_lens(in, w, q),
+                                     [](uint32_t, uint32_t, uint32_t, unsigned long long) {});
+  if (lane == 0) {
+    w.ncta[q] = n;
+    atomicAdd(&w.totals->n_cta[k], n);
+  }
 }
 
 // ---- counts in class order (one thread per position of the class-sorted queries) ----
@@ -348,17 +425,14 @@ __global__ void __launch_bounds__(256) dp_emit_kernel(const DpIn in, const DpWor
     }
     out.wt[o_wt + x] = Sw16WarpTask{sb, ncols};
   }
-  if (lane == 0) {
-    uint32_t t = o_cta;
-    const unsigned long long kmask = (1ull << 44) - 1;
-    dp_for_each_cta(c, sh, nw, v, w.pt, in.db.length, dp_cap(cls, w.totals, k),
-                    [&](uint32_t w0, uint32_t w1, unsigned long long cost) {
-                      out.cta_raw[t] = Sw16CtaTask{q, o_wt + w0, o_wt + w1, sh.mpad};
-                      out.cta_key[t] = (static_cast<unsigned long long>(k) << 44) | (kmask - min(cost, kmask));
-                      out.cta_idx[t] = t;
-                      ++t;
-                    });
-  }
+  const unsigned long long kmask = (1ull << 44) - 1;
+  dp_for_each_cta(cls, w.totals, k, sh, nw, dp_lens(in, w, q),
+                  [&](uint32_t j, uint32_t w0, uint32_t w1, unsigned long long cost) {
+                    const uint32_t t = o_cta + j;
+                    out.cta_raw[t] = Sw16CtaTask{q, o_wt + w0, o_wt + w1, sh.mpad};
+                    out.cta_key[t] = (static_cast<unsigned long long>(k) << 44) | (kmask - min(cost, kmask));
+                    out.cta_idx[t] = t;
+                  });
 }
 
 __global__ void __launch_bounds__(256) dp_gather_cta_kernel(const DpOut out) {

@@ -394,6 +394,7 @@ struct st_ctx {
     std::vector<uint8_t> route;
     std::vector<uint64_t> qstart, n32;
     std::vector<uint32_t> hist;  // per-thread query histograms of the grouping
+    std::vector<double> est;
     std::vector<Sw16Slot> slots[32];
     std::vector<Sw16WarpTask> wt[32];
     std::vector<Sw16CtaTask> cta[32];
@@ -1473,8 +1474,10 @@ static int plan_build(st_ctx* c, const st_pair* pairs, uint64_t n, int32_t open,
     if (qstart[q + 1] > qstart[q]) qlist.push_back(q);
   std::vector<int> qclass(qlist.size());
   std::vector<uint64_t> qsum(qlist.size());
-  int toolong = -1;
-#pragma omp parallel for schedule(dynamic, 8)
+  std::vector<double>& est = ps.est;  // per query and class: the chip's time for it, picoseconds
+  est.resize(qlist.size() * kNumClasses);
+  double batch_ps = 0.0;              // the batch's time with every query in its cheapest class
+#pragma omp parallel for schedule(dynamic, 8) reduction(+ : batch_ps)
   for (int64_t k = 0; k < static_cast<int64_t>(qlist.size()); ++k) {
     const uint32_t q = qlist[k];
     uint32_t* v0 = byq.data() + qstart[q];
@@ -1487,18 +1490,22 @@ static int plan_build(st_ctx* c, const st_pair* pairs, uint64_t n, int32_t open,
       tl_desc[it - v0] = tlen[*it];
       sum_n += tlen[*it];
     }
+    qsum[k] = sum_n;
+    batch_ps += tuning_estimate(&c->tuning, c->profs[q].m, tl_desc.data(), tl_desc.size(), &est[k * kNumClasses]);
+  }
+  int toolong = -1;
+  for (size_t k = 0; k < qlist.size(); ++k) {
+    const uint32_t q = qlist[k];
     const uint32_t m = c->profs[q].m;
-    const uint32_t mean_n = static_cast<uint32_t>(sum_n / (v1 - v0));
-    int cls = tuning_pick_batch(&c->tuning, m, tl_desc.data(), tl_desc.size(), mean_n);
-    if (cls < 0) cls = tuning_pick_single(&c->tuning, m, mean_n);  // no class has a rate: the wavefront model
+    const uint64_t np = qstart[q + 1] - qstart[q];
+    const uint32_t mean_n = static_cast<uint32_t>(qsum[k] / np);
+    int cls = tuning_pick_batch(&c->tuning, m, tlen[byq[qstart[q]]], mean_n, &est[k * kNumClasses], batch_ps);
+    if (cls < 0) cls = tuning_pick_single(&c->tuning, m, mean_n);  // no class stages it: the wavefront model
     const uint32_t rows = kClasses[cls].G * kClasses[cls].R;
     const uint32_t P = (m + rows - 1) / rows;
-    if (static_cast<uint64_t>(kProfRows) * P * rows > static_cast<uint64_t>(g_class_smem[cls])) {
-#pragma omp critical
+    if (static_cast<uint64_t>(kProfRows) * P * rows > static_cast<uint64_t>(g_class_smem[cls]))
       toolong = static_cast<int>(m);
-    }
     qclass[k] = cls;
-    qsum[k] = sum_n;
   }
   if (toolong >= 0) return fail(ST_EINVAL, "query of %d rows does not fit the shared-memory profile", toolong);
   tc.lap("sort+pick");
@@ -1510,12 +1517,12 @@ static int plan_build(st_ctx* c, const st_pair* pairs, uint64_t n, int32_t open,
     cps[k].cta.swap(ps.cta[k]);
   }
   // Emission. A query's pairs (sorted by target length, longest first) form
-  // warp tasks of S = 64/G pairs; consecutive warp tasks form CTA tasks. A CTA
-  // task ends at 128 warp tasks, or (once it holds a warp task for each warp)
-  // when its estimated cost would pass the class's cap: one CTA's share of the
-  // class's total cost on a grid of two CTAs per SM. The cap keeps a long
+  // warp tasks of S = 64/G pairs; consecutive warp tasks form CTA tasks, in units
+  // of tune_cta_unit warp tasks. A CTA task ends at 128 warp tasks, or where the
+  // query's running cost passes a multiple of the class's cap: one CTA's share of
+  // the class's total cost on a grid of two CTAs per SM. The cap keeps a long
   // query from becoming one CTA task longer than the rest of the launch (the
-  // tail); a looser split would pay the ramp, drain and barrier wait of a CTA
+  // tail); a finer split would pay the ramp, drain and barrier wait of a CTA
   // task more often.
   // Passes: warp-task counts and costs, CTA-task counts, offsets, parallel fill.
   struct QEmit {
@@ -1565,23 +1572,28 @@ static int plan_build(st_ctx* c, const st_pair* pairs, uint64_t n, int32_t open,
   std::vector<uint64_t> cap(kNumClasses, 0);
   for (size_t k = 0; k < qlist.size(); ++k) cap[qclass[k]] += qe[k].cost;
   for (int k = 0; k < kNumClasses; ++k) cap[k] = std::max<uint64_t>(1, cap[k] / (2 * c->sms));
+  uint64_t wt_total = 0;
+  for (size_t k = 0; k < qlist.size(); ++k) wt_total += qe[k].n_wt;
   // calls f(w0, w1, cost) for each CTA task of query k, in order
   auto for_each_cta = [&](int64_t k, const QShape& sh, auto&& f) {
     const uint32_t n_wt = qe[k].n_wt;
     const uint64_t cp = cap[qclass[k]];
+    const uint32_t unit = tune_cta_unit(wt_total, c->sms, kClasses[qclass[k]].W);
     uint32_t w0 = 0;
-    uint64_t acc = 0;
+    uint64_t acc = 0, start = 0, bucket = 0;
     for (uint32_t w = 0; w < n_wt; ++w) {
-      const uint64_t cw = wt_cost(sh, wt_cols(k, sh, w));
-      const uint32_t cnt = w - w0;
-      if (cnt == kMaxWtPerCta || (cnt >= static_cast<uint32_t>(kClasses[qclass[k]].W) && acc + cw > cp)) {
-        f(w0, w, acc);
-        w0 = w;
-        acc = 0;
+      if (w % unit == 0) {
+        const uint64_t bk = acc / cp;
+        if (w > 0 && (bk != bucket || w % kMaxWtPerCta == 0)) {
+          f(w0, w, acc - start);
+          w0 = w;
+          start = acc;
+        }
+        bucket = bk;
       }
-      acc += cw;
+      acc += wt_cost(sh, wt_cols(k, sh, w));
     }
-    if (n_wt > w0) f(w0, n_wt, acc);
+    if (n_wt > w0) f(w0, n_wt, acc - start);
   };
 #pragma omp parallel for schedule(dynamic, 16)
   for (int64_t k = 0; k < static_cast<int64_t>(qlist.size()); ++k) {
@@ -2098,7 +2110,7 @@ static int dplan_build(st_ctx* c, const st_pair* pairs, uint64_t n, int32_t open
                o_qk1 = carve(np1 * 4), o_qi0 = carve(np1 * 4), o_qi1 = carve(np1 * 4), o_as = carve(np1 * 4),
                o_aw = carve(np1 * 4), o_ac = carve(np1 * 4), o_os = carve(np1 * 4), o_ow = carve(np1 * 4),
                o_oc = carve(np1 * 4), o_tot = carve(sizeof(DpTotals)), o_sq = carve(np1 * 4),
-               o_sf = carve(np1), o_tmp = carve(t_tmp);
+               o_sf = carve(np1), o_est = carve(np1 * kDpMaxClasses * sizeof(double)), o_tmp = carve(t_tmp);
   ST_TRY(pool_get(c, off, work));
   char* b = work.as<char>();
   DpWork w{};
@@ -2130,6 +2142,7 @@ static int dplan_build(st_ctx* c, const st_pair* pairs, uint64_t n, int32_t open
   w.o_wt = reinterpret_cast<uint32_t*>(b + o_ow);
   w.o_cta = reinterpret_cast<uint32_t*>(b + o_oc);
   w.totals = reinterpret_cast<DpTotals*>(b + o_tot);
+  w.est = reinterpret_cast<double*>(b + o_est);
   void* tmp = b + o_tmp;
   in.pairs = reinterpret_cast<const st_pair*>(b + o_pairs);
 
@@ -2173,11 +2186,13 @@ static int dplan_build(st_ctx* c, const st_pair* pairs, uint64_t n, int32_t open
   cub::DoubleBuffer<uint32_t> vb(w.vals, w.vals_alt);
   ST_CUDA(cub::DeviceRadixSort::SortPairs(tmp, t_sort, kb, vb, static_cast<int>(n), 0, key_bits, s1));
   w.vals_sorted = vb.Current();
+  w.keys_sorted = kb.Current();
   ST_CUDA(cub::DeviceScan::ExclusiveSum(tmp, t_scan, w.qcnt, w.qstart, static_cast<int>(np1), s1));
   const uint32_t gq32 = static_cast<uint32_t>((static_cast<uint64_t>(n_prof) * 32 + 255) / 256);
   const uint32_t gq = static_cast<uint32_t>((np1 + 255) / 256);
+  dp_estimate_kernel<<<n_prof, 256, 0, s1>>>(in1, w, cls);
   dp_pick_kernel<<<gq32, 256, 0, s1>>>(in1, w, cls);
-  dp_split_kernel<<<gq, 256, 0, s1>>>(in1, w, cls);
+  dp_split_kernel<<<gq32, 256, 0, s1>>>(in1, w, cls);
   cub::DoubleBuffer<uint32_t> qk(w.qkey, w.qkey_alt), qi(w.qid, w.qid_alt);
   ST_CUDA(cub::DeviceRadixSort::SortPairs(tmp, t_qsort, qk, qi, static_cast<int>(n_prof), 0, 6, s1));
   w.qid_sorted = qi.Current();
@@ -2186,7 +2201,7 @@ static int dplan_build(st_ctx* c, const st_pair* pairs, uint64_t n, int32_t open
   ST_CUDA(cub::DeviceScan::ExclusiveSum(tmp, t_scan, w.a_wt, w.o_wt, static_cast<int>(np1), s1));
   ST_CUDA(cub::DeviceScan::ExclusiveSum(tmp, t_scan, w.a_cta, w.o_cta, static_cast<int>(np1), s1));
   ST_CUDA(cudaGetLastError());
-  c->launches += 5;
+  c->launches += 6;
   DpTotals tot;
   uint32_t n_list32 = 0;  // pairs the classify stage sent to the 32-bit kernel
   ST_CUDA(cudaMemcpyAsync(&tot, w.totals, sizeof(DpTotals), cudaMemcpyDeviceToHost, s1));
@@ -2217,28 +2232,6 @@ static int dplan_build(st_ctx* c, const st_pair* pairs, uint64_t n, int32_t open
   plan->scratch32_stride = max_m > static_cast<uint32_t>(kSw32Rows) ? max_len : 0;
   plan->n_static32 = n_list32;
   ST_TRY(grid_sw32(c, n_list32, n, plan->scratch32_stride, &plan->grid32));
-  if (n_list32 > 1) {
-    // the 32-bit list longest first (the packed band kernel scores neighbouring entries together), in the
-    // stage-1 buffers that are free now: both key buffers and the value buffer the pair sort left unused
-    uint32_t* vfree = w.vals_sorted == w.vals ? w.vals_alt : w.vals;
-    size_t t_ls = 0;
-    {
-      cub::DoubleBuffer<ull> lk(nullptr, nullptr);
-      cub::DoubleBuffer<uint32_t> lv(nullptr, nullptr);
-      ST_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, t_ls, lk, lv, static_cast<int>(n_list32), 0, 48, s1));
-    }
-    if (t_ls <= t_tmp) {
-      const uint32_t gl = static_cast<uint32_t>(std::min<uint64_t>((n_list32 + 255) / 256,
-                                                                   static_cast<uint64_t>(c->sms) * 8));
-      dp_list_keys_kernel<<<gl, 256, 0, s1>>>(in, w, n_list32, w.keys, vfree);
-      cub::DoubleBuffer<ull> lk(w.keys, w.keys_alt);
-      cub::DoubleBuffer<uint32_t> lv(vfree, w.list32);
-      ST_CUDA(cub::DeviceRadixSort::SortPairs(tmp, t_ls, lk, lv, static_cast<int>(n_list32), 0, 48, s1));
-      if (lv.Current() != w.list32)
-        ST_CUDA(cudaMemcpyAsync(w.list32, lv.Current(), static_cast<size_t>(n_list32) * 4, cudaMemcpyDeviceToDevice,
-                                s1));
-    }
-  }
   size_t t_lpt = 0;
   {
     cub::DoubleBuffer<ull> ck(nullptr, nullptr);
@@ -2279,6 +2272,28 @@ static int dplan_build(st_ctx* c, const st_pair* pairs, uint64_t n, int32_t open
     ST_CUDA(cub::DeviceRadixSort::SortPairs(a + p_tmp, t_lpt, ck, ci, static_cast<int>(n_cta), 0, 44 + 6, s1));
     o.cta_idx_sorted = ci.Current();
     dp_gather_cta_kernel<<<static_cast<uint32_t>((n_cta + 255) / 256), 256, 0, s1>>>(o);
+  }
+  if (n_list32 > 1) {
+    // the 32-bit list longest first (the packed band kernel scores neighbouring entries together), in the
+    // stage-1 buffers that are free after the emission: both key buffers and the value buffer the pair sort left
+    uint32_t* vfree = w.vals_sorted == w.vals ? w.vals_alt : w.vals;
+    size_t t_ls = 0;
+    {
+      cub::DoubleBuffer<ull> lk(nullptr, nullptr);
+      cub::DoubleBuffer<uint32_t> lv(nullptr, nullptr);
+      ST_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, t_ls, lk, lv, static_cast<int>(n_list32), 0, 48, s1));
+    }
+    if (t_ls <= t_tmp) {
+      const uint32_t gl = static_cast<uint32_t>(std::min<uint64_t>((n_list32 + 255) / 256,
+                                                                   static_cast<uint64_t>(c->sms) * 8));
+      dp_list_keys_kernel<<<gl, 256, 0, s1>>>(in, w, n_list32, w.keys, vfree);
+      cub::DoubleBuffer<ull> lk(w.keys, w.keys_alt);
+      cub::DoubleBuffer<uint32_t> lv(vfree, w.list32);
+      ST_CUDA(cub::DeviceRadixSort::SortPairs(tmp, t_ls, lk, lv, static_cast<int>(n_list32), 0, 48, s1));
+      if (lv.Current() != w.list32)
+        ST_CUDA(cudaMemcpyAsync(w.list32, lv.Current(), static_cast<size_t>(n_list32) * 4, cudaMemcpyDeviceToDevice,
+                                s1));
+    }
   }
   ST_CUDA(cudaGetLastError());
   c->launches += 2;

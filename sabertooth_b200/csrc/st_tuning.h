@@ -1,12 +1,12 @@
 // Tile-class selection for the packed 16-bit kernel: lanes per alignment (G),
 // query rows per lane (R) and columns per step (C).
 //
-// Batches: each query takes the class with the least estimated time, its
-// streamed cells (padded rows x padded columns x slots, from its own target
-// lengths) divided by the class's measured rate (streamed cells per second,
-// calibrated by st_autotune; built-in B200 figures by default, 0 = class not
-// considered).  A table entry per (query length, mean target length) bin, set
-// by the caller, forces a class for that bin.
+// Batches: each query takes the class with the least estimated cost to the
+// batch: the chip's time for its streamed cells (padded rows x padded columns x
+// slots, from its own target lengths, over the class's measured rate; built-in
+// B200 figures, replaced by st_autotune, 0 = class not considered), plus what its
+// critical path exceeds the whole batch by.  A table entry per (query length,
+// mean target length) bin, set by the caller, forces a class for that bin.
 //
 // Single alignments (the per-call path) use a model of the wavefront: a task
 // streams P * ncols / C + G - 1 steps, each costing about R * C row updates
@@ -14,6 +14,12 @@
 #pragma once
 #include <algorithm>
 #include <cstdint>
+
+#ifdef __CUDACC__
+#define TUNE_HD __host__ __device__
+#else
+#define TUNE_HD
+#endif
 
 constexpr int kTuneMBins = 10;  // query length: <=32, <=64, ..., <=8192, >8192
 constexpr int kTuneNBins = 8;   // mean target length: <=64, <=128, ..., <=4096, >4096
@@ -100,21 +106,63 @@ inline double tune_streamed(int c, uint32_t m, const uint32_t* tlen_desc, size_t
   return cols * S * P * rows;
 }
 
-// The class with the least estimated time for one query of a batch.
-inline int tuning_pick_batch(const Tuning* t, uint32_t m, const uint32_t* tlen_desc, size_t n, uint32_t mean_n) {
+// Critical path: the time of the wavefront that streams a query's longest target, alone on its scheduler, in
+// picoseconds.  A step of a lone warp takes about 700 cycles (the shuffles, the profile loads, the dependent
+// rows) plus 11.5 for each of its R*C cell pairs; measured at 1,965 MHz on 4,000-column targets: 1,090 cycles for
+// R = 8, 1,380 for 16, 1,780 for 24, 2,200 for 32 (C = 4), 990 for R = 16, C = 2.
+TUNE_HD inline double tune_crit_ps(uint32_t G, uint32_t R, uint32_t C, uint32_t P, uint32_t ncols) {
+  return (static_cast<double>(P) * (ncols / C) + G) * (700.0 + 11.5 * (R * C)) * (1e6 / 1965.0);
+}
+
+// What a query costs the batch in a class: the chip's time for its cells, plus what its critical path adds when
+// that is longer than the whole batch (batch_ps: the batch's time with every query in its cheapest class).  Large
+// batches are all cell time and take the classes of few lanes, which pad least; in a small one the chip waits
+// for the longest wavefront, so a query of many rows takes more lanes and fewer passes.  1.5: a warp that shares
+// its scheduler at the start and ends alone runs between once and 2.6 times its lone time.
+TUNE_HD inline double tune_objective(double est_ps, double crit_ps, double batch_ps) {
+  const double over = 1.5 * crit_ps - batch_ps;
+  return est_ps + (over > 0.0 ? over : 0.0);
+}
+
+// Warp tasks per unit of a CTA task: a CTA's warps, fewer (a power of two) when the batch has not that many for
+// two CTAs on every SM, so that a small batch spreads over the chip.
+TUNE_HD inline uint32_t tune_cta_unit(uint64_t wt_total, uint32_t sms, uint32_t W) {
+  uint32_t u = W;
+  while (u > 1 && static_cast<uint64_t>(u) * 2 * sms > wt_total) u >>= 1;
+  return u;
+}
+
+// est[c] = the chip's time (ps) for the query in class c: streamed cells over the rate; a class without a rate
+// counts 1e150 times its cells (taken only when no class with a rate stages the query), one that cannot stage it
+// 1e300.  Returns the least time over the classes with a rate (0: none).
+inline double tuning_estimate(const Tuning* t, uint32_t m, const uint32_t* tlen_desc, size_t n, double* est) {
+  double best = 0.0;
+  for (int c = 0; c < st_tuning_num_classes(); ++c) {
+    const double v = tune_streamed(c, m, tlen_desc, n);
+    est[c] = v >= 1e300 ? 1e300 : (t->rate[c] > 0.0f ? v / t->rate[c] : v * 1e150);
+    if (est[c] < 1e140 && (best == 0.0 || est[c] < best)) best = est[c];
+  }
+  return best;
+}
+
+// The class of one query of a batch (longest: its longest target); -1 when none stages it.
+inline int tuning_pick_batch(const Tuning* t, uint32_t m, uint32_t longest, uint32_t mean_n, const double* est,
+                             double batch_ps) {
   const int forced = t->table[tune_mbin(m)][tune_nbin(mean_n)];
-  if (forced >= 0 && forced < st_tuning_num_classes() && tune_streamed(forced, m, tlen_desc, n) < 1e300) return forced;
-  // classes with a rate first; if none of them stages this query, least streamed cells over all
+  if (forced >= 0 && forced < st_tuning_num_classes() && est[forced] < 1e300) return forced;
   int best = -1;
-  for (int pass = 0; pass < 2 && best < 0; ++pass) {
-    double bt = 1e299;
-    for (int c = 0; c < st_tuning_num_classes() && c < kMaxTileClasses; ++c) {
-      if (pass == 0 && !(t->rate[c] > 0.0f)) continue;
-      const double v = tune_streamed(c, m, tlen_desc, n) / (pass == 0 ? t->rate[c] : 1.0f);
-      if (v < bt) {
-        bt = v;
-        best = c;
-      }
+  double bt = 1e300;
+  for (int c = 0; c < st_tuning_num_classes(); ++c) {
+    if (est[c] >= 1e300) continue;
+    int G, R, C;
+    st_tuning_class_shape(c, &G, &R, &C);
+    const uint32_t rows = static_cast<uint32_t>(G * R), P = (m + rows - 1) / rows;
+    const uint32_t minc = P > 1 ? std::max<uint32_t>(32, (static_cast<uint32_t>(C * G) + 15) & ~15u) : 32u;
+    const double crit = tune_crit_ps(G, R, C, P, std::max<uint32_t>(minc, (longest + 3) & ~3u));
+    const double v = tune_objective(est[c], crit, batch_ps);
+    if (v < bt) {
+      bt = v;
+      best = c;
     }
   }
   return best;
