@@ -405,8 +405,9 @@ int st_calibrate_profiles(st_ctx* ctx, const uint32_t* profiles, uint32_t n_prof
  * Score plus end cell, the first optimum in column-major order (smallest target
  * position, then smallest query position): QueryProfile::sw_score_end_with
  * (src/simd.rs:301-326, tie rule :375-381).  Positions are 0-based and
- * inclusive; -1 when the score is 0 (the reference returns None).  Computed by
- * the exact 32-bit kernel.  Unbanded pairs only. */
+ * inclusive; -1 when the score is 0 (the reference returns None).  A single
+ * call runs the exact 32-bit kernel; batches run the packed 16-bit kernel with
+ * its exact 32-bit rescore.  Unbanded pairs only. */
 int st_sw_score_end(st_ctx* ctx, uint32_t profile, const uint8_t* target, uint32_t n, int32_t open, int32_t ext,
                     int32_t* score, int32_t* q_end, int32_t* t_end);
 /* Batched: ends[2i], ends[2i+1] = (query end, target end) of pair i. */

@@ -66,6 +66,7 @@ struct DpIn {
   DeviceProfiles prof;
   uint32_t n_prof;
   uint32_t max_m16;  // longest query the 16-bit classes stage; longer ones take the 32-bit kernel
+  uint32_t max_n16;  // longest target of a 16-bit pair
   uint32_t g16;      // gap costs inside the 16-bit kernel's range
   uint32_t tbits;    // bits of the sort key's target-length field
 };
@@ -164,7 +165,7 @@ __global__ void __launch_bounds__(256) dp_classify_kernel(const DpIn in, const D
     const uint32_t tl = in.db.length[t];
     unsigned long long key = sentinel;
     if (m != 0 && tl != 0) {
-      if (radius < 0 && in.g16 && in.prof.fits8[q] && m <= in.max_m16) {
+      if (radius < 0 && in.g16 && in.prof.fits8[q] && m <= in.max_m16 && tl <= in.max_n16) {
         key = (static_cast<unsigned long long>(q) << in.tbits) | (tmask - tl);
         atomicAdd(&w.qcnt[q], 1u);
       } else {

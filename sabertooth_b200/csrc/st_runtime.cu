@@ -256,6 +256,24 @@ static const Sw16Class kClasses[] = {
 #undef ST_CLASS
 #undef ST_CLASS_W
 constexpr int kNumClasses = sizeof(kClasses) / sizeof(kClasses[0]);
+
+// The tile classes built for end cells too: 64 to 512 rows a pass, so that every query length has a class that
+// pads little; eight warps a CTA and at most 16 rows a lane, which leaves registers for the row masks.
+struct Sw16EndFns {
+  int G, R;
+  Sw16Fn fwd, rev;
+};
+#define ST_END(g, r) {g, r, sw16_kernel<g, r, 4, kWarps16, kSw16End>, sw16_kernel<g, r, 4, kWarps16, kSw16RevEnd>}
+static const Sw16EndFns kEndFns[] = {ST_END(8, 8), ST_END(32, 8), ST_END(8, 16), ST_END(16, 16), ST_END(32, 16)};
+#undef ST_END
+static const Sw16EndFns* end_fns(int cls) {
+  if (kClasses[cls].C != 4) return nullptr;
+  for (const auto& f : kEndFns)
+    if (f.G == kClasses[cls].G && f.R == kClasses[cls].R) return &f;
+  return nullptr;
+}
+constexpr uint32_t kEndMaxLen = 65535;  // an end cell's column travels in 16 bits
+
 static_assert(kNumClasses <= kMaxTileClasses, "tile classes exceed the tuning arrays");
 
 int st_tuning_num_classes() { return kNumClasses; }
@@ -618,6 +636,13 @@ static int set_smem_limits(int device) {
     g_class_smem[i] = std::min<int>(kMaxSmem, optin - static_cast<int>(fa.sharedSizeBytes));
     ST_CUDA(cudaFuncSetAttribute(kClasses[i].fn, cudaFuncAttributeMaxDynamicSharedMemorySize, g_class_smem[i]));
   }
+  for (const auto& f : kEndFns)
+    for (Sw16Fn fn : {f.fwd, f.rev}) {
+      cudaFuncAttributes fa;
+      ST_CUDA(cudaFuncGetAttributes(&fa, reinterpret_cast<const void*>(fn)));
+      ST_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                   std::min<int>(kMaxSmem, optin - static_cast<int>(fa.sharedSizeBytes))));
+    }
   cudaFuncAttributes fa_t, fa_f;
   ST_CUDA(cudaFuncGetAttributes(&fa_t, reinterpret_cast<const void*>(ungapped_kernel<true>)));
   ST_CUDA(cudaFuncGetAttributes(&fa_f, reinterpret_cast<const void*>(ungapped_kernel<false>)));
@@ -1151,6 +1176,14 @@ static uint64_t band_cells(uint32_t m, uint32_t n, int64_t c, int64_t r) {
   return static_cast<uint64_t>(total);
 }
 
+// The tile classes a plan may take, a bit each.
+static uint32_t class_mask(bool ends) {
+  uint32_t m = 0;
+  for (int k = 0; k < kNumClasses; ++k)
+    if (!ends || end_fns(k)) m |= 1u << k;
+  return m;
+}
+
 struct ClassPlan {
   int cls = -1;
   std::vector<Sw16CtaTask> cta;
@@ -1309,8 +1342,10 @@ static int fork_set(st_ctx* c, int i, st_ctx::ForkSet** out) {
 // Builds a plan for `n` pairs. Its initialised data is staged in pinned block
 // `slot` of the context's ring and uploaded on `up`; the block is reused only
 // after that copy has finished (an event per block).
+// With `ends` the plan is for the end-cell modes: their tile classes only, targets they can address.
 static int plan_build(st_ctx* c, const st_pair* pairs, uint64_t n, int32_t open, int32_t ext, int32_t* d_scores,
-                      uint32_t* d_kernels, st_plan** out, bool capture, cudaStream_t up, int slot) {
+                      uint32_t* d_kernels, st_plan** out, bool capture, cudaStream_t up, int slot,
+                      bool ends = false) {
   if (!c->has_db) return fail(ST_ESTATE, "no target database uploaded (st_db_upload)");
   if (n > 0xFFFFFFF0ull) return fail(ST_EINVAL, "too many pairs (%llu)", static_cast<unsigned long long>(n));
   ST_TRY(sync_profiles(c));
@@ -1324,8 +1359,10 @@ static int plan_build(st_ctx* c, const st_pair* pairs, uint64_t n, int32_t open,
   const bool g16 = gaps16_ok(open, ext);
   // the longest query whose int8 profile fits the shared memory of some 16-bit class;
   // longer ones take the 32-bit kernel
+  const uint32_t max_n16 = ends ? kEndMaxLen : UINT32_MAX;
   uint32_t max_m16 = 0;
   for (int k = 0; k < kNumClasses; ++k) {
+    if (ends && !end_fns(k)) continue;
     const uint32_t rows = static_cast<uint32_t>(kClasses[k].G * kClasses[k].R);
     const uint32_t smem = static_cast<uint32_t>(std::min<int>(g_class_smem[k], 216 * 1024));  // the models' limit
     max_m16 = std::max(max_m16, smem / kProfRows / rows * rows);
@@ -1379,7 +1416,7 @@ static int plan_build(st_ctx* c, const st_pair* pairs, uint64_t n, int32_t open,
     } else {
       const uint64_t mc = static_cast<uint64_t>(pm.m) * tl;
       cells += mc;
-      if (g16 && pm.fits8 && pm.m <= max_m16) {
+      if (g16 && pm.fits8 && pm.m <= max_m16 && tl <= max_n16) {
         route[i] = 1;
       } else {
         route[i] = 2;
@@ -1491,7 +1528,8 @@ static int plan_build(st_ctx* c, const st_pair* pairs, uint64_t n, int32_t open,
       sum_n += tlen[*it];
     }
     qsum[k] = sum_n;
-    batch_ps += tuning_estimate(&c->tuning, c->profs[q].m, tl_desc.data(), tl_desc.size(), &est[k * kNumClasses]);
+    batch_ps += tuning_estimate(&c->tuning, c->profs[q].m, tl_desc.data(), tl_desc.size(), &est[k * kNumClasses],
+                                class_mask(ends));
   }
   int toolong = -1;
   for (size_t k = 0; k < qlist.size(); ++k) {
@@ -2040,7 +2078,8 @@ static int bits_for(uint64_t x) {
 static int upload_host(st_ctx* c, void* dst, const void* src, size_t bytes, cudaStream_t s);
 
 static int dplan_build(st_ctx* c, const st_pair* pairs, uint64_t n, int32_t open, int32_t ext, int32_t* d_scores,
-                       uint32_t* d_kernels, uint32_t max_len, uint32_t max_m, DevMem& work, st_plan** out) {
+                       uint32_t* d_kernels, uint32_t max_len, uint32_t max_m, DevMem& work, st_plan** out,
+                       bool ends = false) {
   cudaStream_t st = c->stream;
   TraceClock tc("dplan");
   const uint32_t n_prof = static_cast<uint32_t>(c->profs.size());
@@ -2066,7 +2105,7 @@ static int dplan_build(st_ctx* c, const st_pair* pairs, uint64_t n, int32_t open
     d.rows = d.G * d.R;
     d.S = 64 / d.G;
     const uint32_t smem = static_cast<uint32_t>(std::min<int>(g_class_smem[k], 216 * 1024));
-    d.max_mpad = smem / kProfRows / d.rows * d.rows;
+    d.max_mpad = ends && !end_fns(k) ? 0u : smem / kProfRows / d.rows * d.rows;
     d.rate = c->tuning.rate[k];
     max_m16 = std::max(max_m16, d.max_mpad);
   }
@@ -2078,6 +2117,7 @@ static int dplan_build(st_ctx* c, const st_pair* pairs, uint64_t n, int32_t open
   in.prof = prof_view(c);
   in.n_prof = n_prof;
   in.max_m16 = max_m16;
+  in.max_n16 = ends ? kEndMaxLen : UINT32_MAX;
   in.g16 = g16 ? 1u : 0u;
   in.tbits = static_cast<uint32_t>(bits_for(max_len));
   const int key_bits = std::min(64, bits_for(n_prof) + static_cast<int>(in.tbits));
@@ -2662,126 +2702,203 @@ extern "C" int st_sw_score_pairs(st_ctx* c, const st_pair* pairs, uint64_t n, in
 
 // ---------------------------------------------------------------------------
 // end cells and alignment spans (sw_score_end_with + the reverse pass of
-// align_canonical), exact 32-bit kernel
+// align_canonical)
 // ---------------------------------------------------------------------------
-// Scores n pairs (targets in `db`, unbanded) in end mode and, with `span`,
-// runs the reverse pass from each end cell. Outputs go to host buffers:
-// scores[i]; ends[2i..2i+1] = (query end, target end); with span,
-// starts[2i..2i+1] = (query start, target start); -1 where the score is 0.
-static int end_pairs_run(st_ctx* c, const DeviceDb& db, const uint32_t* pq_h, const uint32_t* pt_h, uint64_t n,
-                         uint32_t max_m, uint32_t max_len, int32_t open, int32_t ext, bool span, int32_t* scores,
-                         int32_t* ends, int32_t* starts) {
-  if (n == 0) return ST_OK;
-  if (n > 0xFFFFFFF0ull) return fail(ST_EINVAL, "too many pairs");
+// Score and end cell of one pair whose target is `db`'s only sequence, by the exact 32-bit kernel:
+// end[0], end[1] = (query end, target end), -1 where the score is 0.
+static int end_single_run(st_ctx* c, const DeviceDb& db, uint32_t profile, uint32_t max_m, uint32_t max_len,
+                          int32_t open, int32_t ext, int32_t* score, int32_t* end) {
   uint32_t grid = 0;
   const uint32_t sstride = max_m > static_cast<uint32_t>(kSw32Rows) ? max_len : 0;
-  ST_TRY(grid_sw32(c, n, n, sstride, &grid));
-  size_t off = 0;
-  auto carve = [&](size_t bytes) {
-    const size_t o = off;
-    off = (off + bytes + 255) & ~static_cast<size_t>(255);
-    return o;
+  ST_TRY(grid_sw32(c, 1, 1, sstride, &grid));
+  // inputs (one copy): query, target, list entry, no band, list count, work counter; outputs behind them
+  struct In {
+    uint32_t q, t, entry;
+    int32_t zero;
+    uint32_t count, work;
+    int32_t score, eq, et;
   };
-  const size_t o_pq = carve(n * 4), o_pt = carve(n * 4), o_zero = carve(n * 4), o_list = carve(n * 4),
-               o_cnt = carve(16), o_s = carve(n * 4), o_eq = carve(n * 4), o_et = carve(n * 4), o_rs = carve(n * 4),
-               o_sq = carve(n * 4), o_st = carve(n * 4),
-               o_scr = carve(sstride ? static_cast<size_t>(grid) * kWarps32 * sstride * sizeof(int2) : 16);
-  const size_t up_bytes = o_zero;  // pq, pt travel in one copy
+  const size_t o_scr = (sizeof(In) + 255) & ~static_cast<size_t>(255);
   DevMem a;
-  ST_TRY(pool_get(c, off, a));
+  ST_TRY(pool_get(c, o_scr + (sstride ? static_cast<size_t>(grid) * kWarps32 * sstride * sizeof(int2) : 16), a));
   struct Back {
     st_ctx* c;
     DevMem* m;
     ~Back() { pool_put_after(c, std::move(*m), c->stream); }
   } back{c, &a};
-  char* d = a.as<char>();
-  ST_TRY(c->pin.reserve(up_bytes + 16));
+  ST_TRY(c->pin.reserve(sizeof(In)));
   ST_CUDA(cudaStreamSynchronize(c->stream));  // the pinned block may still feed an earlier copy
-  char* h = c->pin.as<char>();
-  memcpy(h + o_pq, pq_h, n * 4);
-  memcpy(h + o_pt, pt_h, n * 4);
-  ST_CUDA(cudaMemcpyAsync(d, h, up_bytes, cudaMemcpyHostToDevice, c->stream));
-  ST_CUDA(cudaMemsetAsync(d + o_zero, 0, n * 4, c->stream));
-  ST_CUDA(cudaMemsetAsync(d + o_cnt, 0, 16, c->stream));
-  uint32_t* cnt = reinterpret_cast<uint32_t*>(d + o_cnt);  // [0] list count, [1], [2] work counters
-  const uint32_t n32 = static_cast<uint32_t>(n);
-  ST_CUDA(cudaMemcpyAsync(cnt, &n32, 4, cudaMemcpyHostToDevice, c->stream));
-  dp_iota_kernel<<<static_cast<uint32_t>(std::min<uint64_t>((n + 255) / 256, 65535)), 256, 0, c->stream>>>(
-      reinterpret_cast<uint32_t*>(d + o_list), n32);
+  In* h = c->pin.as<In>();
+  *h = In{profile, 0, 0, 0, 1, 0, 0, -1, -1};
+  In* d = a.as<In>();
+  ST_CUDA(cudaMemcpyAsync(d, h, sizeof(In), cudaMemcpyHostToDevice, c->stream));
   Sw32Params p{};
   p.db = db;
   p.prof = prof_view(c);
-  p.list = reinterpret_cast<const uint32_t*>(d + o_list);
-  p.list_count = cnt;
-  p.pair_query = reinterpret_cast<const uint32_t*>(d + o_pq);
-  p.pair_target = reinterpret_cast<const uint32_t*>(d + o_pt);
-  p.pair_center = reinterpret_cast<const int32_t*>(d + o_zero);
-  p.pair_radius = reinterpret_cast<const int32_t*>(d + o_zero);  // unused in the end modes
-  p.scores = reinterpret_cast<int32_t*>(d + o_s);
+  p.list = &d->entry;
+  p.list_count = &d->count;
+  p.pair_query = &d->q;
+  p.pair_target = &d->t;
+  p.pair_center = &d->zero;
+  p.pair_radius = &d->zero;  // unused in the end modes
+  p.scores = &d->score;
   p.kernels = nullptr;
-  p.work_counter = cnt + 1;
-  p.scratch = reinterpret_cast<int2*>(d + o_scr);
+  p.work_counter = &d->work;
+  p.scratch = reinterpret_cast<int2*>(a.as<char>() + o_scr);
   p.scratch_stride = sstride;
   p.open = open;
   p.ext = ext;
-  p.end_q = reinterpret_cast<int32_t*>(d + o_eq);
-  p.end_t = reinterpret_cast<int32_t*>(d + o_et);
+  p.end_q = &d->eq;
+  p.end_t = &d->et;
   sw32_end_kernel<kWarps32, kSw32End><<<grid, kWarps32 * 32, 0, c->stream>>>(p);
-  c->launches += 2;
-  if (span) {
-    Sw32Params r = p;
-    r.rev_q = p.end_q;
-    r.rev_t = p.end_t;
-    r.scores = reinterpret_cast<int32_t*>(d + o_rs);
-    r.end_q = reinterpret_cast<int32_t*>(d + o_sq);
-    r.end_t = reinterpret_cast<int32_t*>(d + o_st);
-    r.work_counter = cnt + 2;
-    sw32_end_kernel<kWarps32, kSw32RevEnd><<<grid, kWarps32 * 32, 0, c->stream>>>(r);
-    ++c->launches;
-  }
+  ++c->launches;
   ST_CUDA(cudaGetLastError());
-  std::vector<int32_t> eq(n), et(n), rs, sq, st;
-  ST_CUDA(cudaMemcpyAsync(scores, d + o_s, n * 4, cudaMemcpyDeviceToHost, c->stream));
-  ST_CUDA(cudaMemcpyAsync(eq.data(), d + o_eq, n * 4, cudaMemcpyDeviceToHost, c->stream));
-  ST_CUDA(cudaMemcpyAsync(et.data(), d + o_et, n * 4, cudaMemcpyDeviceToHost, c->stream));
-  if (span) {
-    rs.resize(n);
-    sq.resize(n);
-    st.resize(n);
-    ST_CUDA(cudaMemcpyAsync(rs.data(), d + o_rs, n * 4, cudaMemcpyDeviceToHost, c->stream));
-    ST_CUDA(cudaMemcpyAsync(sq.data(), d + o_sq, n * 4, cudaMemcpyDeviceToHost, c->stream));
-    ST_CUDA(cudaMemcpyAsync(st.data(), d + o_st, n * 4, cudaMemcpyDeviceToHost, c->stream));
-  }
+  ST_CUDA(cudaMemcpyAsync(h, d, sizeof(In), cudaMemcpyDeviceToHost, c->stream));
   ST_CUDA(cudaStreamSynchronize(c->stream));
-  for (uint64_t i = 0; i < n; ++i) {
-    ends[2 * i] = eq[i];
-    ends[2 * i + 1] = et[i];
-    if (!span) continue;
-    if (scores[i] > 0 && rs[i] != scores[i])  // impossible: the best alignment ending at the end cell lies in the prefix
-      return fail(ST_ECUDA, "pair %llu: reverse pass scored %d, forward %d", static_cast<unsigned long long>(i),
-                  rs[i], scores[i]);
-    starts[2 * i] = scores[i] > 0 ? eq[i] - sq[i] : -1;
-    starts[2 * i + 1] = scores[i] > 0 ? et[i] - st[i] : -1;
-  }
+  *score = h->score;
+  end[0] = h->eq;
+  end[1] = h->et;
   return ST_OK;
 }
 
+// One end-cell pass of a plan: every 16-bit class (side by side on the fork set), then the exact 32-bit kernel over
+// its list, which holds the pairs that are not eligible for 16 bits and those the forward pass found above the
+// headroom.
+static int end_pass(st_plan* p, st_ctx::ForkSet* fs, cudaStream_t st, bool rev, const Sw16Params& arrays,
+                    const Sw32Params& p32) {
+  std::vector<const ClassPlan*> order;
+  for (const auto& cp : p->classes) order.push_back(&cp);
+  std::stable_sort(order.begin(), order.end(),
+                   [](const ClassPlan* a, const ClassPlan* b) { return a->cells > b->cells; });
+  if (order.size() > 1) ST_CUDA(cudaEventRecord(fs->ev[0], st));
+  for (size_t i = 0; i < order.size(); ++i) {
+    const ClassPlan& cp = *order[i];
+    cudaStream_t s = st;
+    if (i) {
+      s = fs->s[i - 1];
+      ST_CUDA(cudaStreamWaitEvent(s, fs->ev[0], 0));
+    }
+    Sw16Params prm = cp.prm;
+    prm.scores = arrays.scores;
+    prm.end_q = arrays.end_q;
+    prm.end_t = arrays.end_t;
+    prm.rev_q = arrays.rev_q;
+    prm.rev_t = arrays.rev_t;
+    prm.rev_score = arrays.rev_score;
+    const Sw16EndFns* f = end_fns(cp.cls);
+    (rev ? f->rev : f->fwd)<<<cp.grid, kClasses[cp.cls].W * 32, cp.smem, s>>>(prm);
+    ST_CUDA(cudaGetLastError());
+  }
+  for (size_t i = 1; i < order.size(); ++i) {
+    ST_CUDA(cudaEventRecord(fs->ev[i], fs->s[i - 1]));
+    ST_CUDA(cudaStreamWaitEvent(st, fs->ev[i], 0));
+  }
+  if (rev)
+    sw32_end_kernel<kWarps32, kSw32RevEnd><<<p->grid32, kWarps32 * 32, 0, st>>>(p32);
+  else
+    sw32_end_kernel<kWarps32, kSw32End><<<p->grid32, kWarps32 * 32, 0, st>>>(p32);
+  ST_CUDA(cudaGetLastError());
+  p->ctx->launches += order.size() + 1;
+  return ST_OK;
+}
+
+// Batched end cells and spans: the pairs are planned like a scoring batch, over the tile classes that track end
+// cells.  The forward pass gives every pair's score and end cell, the reverse pass runs the same tasks over the
+// reversed prefixes; both write into one block that comes back in one copy.  One warp a pair in exact 32-bit cells
+// before (about 20 instructions a cell): see kEndFns for the classes and st_sw16.cuh for the tracking.
 static int end_pairs_entry(st_ctx* c, const st_pair* pairs, uint64_t n, int32_t open, int32_t ext, bool span,
                            int32_t* scores, int32_t* ends, int32_t* starts) {
   if (n && (!pairs || !scores || !ends || (span && !starts))) return fail(ST_EINVAL, "null argument");
   if (!c->has_db) return fail(ST_ESTATE, "no target database uploaded (st_db_upload)");
   uint32_t max_len = 0, max_m = 0;
   ST_TRY(validate_pairs(c, pairs, n, &max_len, &max_m));
-  std::vector<uint32_t> pq(n), pt(n);
-  for (uint64_t i = 0; i < n; ++i) {
-    if (pairs[i].band_radius >= 0)
-      return fail(ST_EINVAL, "pair %llu: end cells are defined for full local alignments (band_radius < 0)",
-                  static_cast<unsigned long long>(i));
-    pq[i] = pairs[i].profile;
-    pt[i] = pairs[i].target;
-  }
+  int64_t banded = INT64_MAX;
+#pragma omp parallel for schedule(static) reduction(min : banded) if (n > 65536)
+  for (int64_t i = 0; i < static_cast<int64_t>(n); ++i)
+    if (pairs[i].band_radius >= 0) banded = std::min<int64_t>(banded, i);
+  if (banded != INT64_MAX)
+    return fail(ST_EINVAL, "pair %llu: end cells are defined for full local alignments (band_radius < 0)",
+                static_cast<unsigned long long>(banded));
+  if (n == 0) return ST_OK;
+  if (n > 0xFFFFFFF0ull) return fail(ST_EINVAL, "too many pairs");
   ST_TRY(sync_profiles(c));
-  return end_pairs_run(c, db_view(c), pq.data(), pt.data(), n, max_m, max_len, open, ext, span, scores, ends, starts);
+  // [scores] [query ends] [target ends] and with spans [reverse scores] [the same of the reverse pass]
+  const int k_out = span ? 6 : 3;
+  DevMem out, work;
+  st_plan* plan = nullptr;
+  struct Back {  // on every exit: nothing queued still uses the buffers when they return to the pool
+    st_ctx* c;
+    DevMem *a, *b;
+    st_plan** p;
+    bool idle;
+    ~Back() {
+      if (!idle) {
+        for (auto s : c->forks[0].s)
+          if (s) cudaStreamSynchronize(s);
+        cudaStreamSynchronize(c->stream);
+      }
+      if (*p) plan_free(*p);
+      pool_put(c, std::move(*a));
+      pool_put(c, std::move(*b));
+    }
+  } back{c, &out, &work, &plan, false};
+  ST_TRY(pool_get(c, n * 4 * k_out, out));
+  int32_t* d = out.as<int32_t>();
+  int32_t *d_s = d, *d_eq = d + n, *d_et = d + 2 * n, *d_rs = d + 3 * n, *d_sq = d + 4 * n, *d_st = d + 5 * n;
+  if (use_device_plan(n))
+    ST_TRY(dplan_build(c, pairs, n, open, ext, d_s, nullptr, max_len, max_m, work, &plan, true));
+  else
+    ST_TRY(plan_build(c, pairs, n, open, ext, d_s, nullptr, &plan, false, c->stream, 0, true));
+  cudaStream_t st = c->stream;
+  st_ctx::ForkSet* fs = nullptr;
+  ST_TRY(fork_set(c, 0, &fs));
+  ST_CUDA(cudaMemsetAsync(d_s, 0, n * 4, st));
+  ST_CUDA(cudaMemsetAsync(d_eq, 0xFF, n * 8, st));  // -1: a pair without a positive score has no cells
+  ST_CUDA(cudaMemcpyAsync(plan->counters, plan->counters_init, (kNumClasses + 2) * 4, cudaMemcpyDeviceToDevice, st));
+  Sw16Params a16{};
+  a16.scores = d_s;
+  a16.end_q = d_eq;
+  a16.end_t = d_et;
+  Sw32Params p32 = plan->p32;
+  p32.end_q = d_eq;
+  p32.end_t = d_et;
+  ST_TRY(end_pass(plan, fs, st, false, a16, p32));
+  if (span) {
+    ST_CUDA(cudaMemsetAsync(d_rs, 0, n * 4, st));
+    ST_CUDA(cudaMemsetAsync(d_sq, 0xFF, n * 8, st));
+    // the work counters start over; the 32-bit list keeps what the forward pass added to it
+    ST_CUDA(cudaMemsetAsync(plan->counters, 0, (kNumClasses + 1) * 4, st));
+    a16.rev_q = p32.rev_q = d_eq;
+    a16.rev_t = p32.rev_t = d_et;
+    a16.rev_score = d_s;
+    a16.scores = p32.scores = d_rs;
+    a16.end_q = p32.end_q = d_sq;
+    a16.end_t = p32.end_t = d_st;
+    ST_TRY(end_pass(plan, fs, st, true, a16, p32));
+  }
+  ST_CUDA(cudaStreamSynchronize(st));  // the pinned block may still feed an earlier copy
+  ST_TRY(c->pin.reserve(n * 4 * k_out));
+  const int32_t* h = c->pin.as<int32_t>();
+  ST_CUDA(cudaMemcpyAsync(c->pin.p, d, n * 4 * k_out, cudaMemcpyDeviceToHost, st));
+  ST_CUDA(cudaStreamSynchronize(st));
+  back.idle = true;
+  int64_t bad = INT64_MAX;
+#pragma omp parallel for schedule(static) reduction(min : bad) if (n > 65536)
+  for (int64_t i = 0; i < static_cast<int64_t>(n); ++i) {
+    const int32_t s = h[i], eq = h[n + i], et = h[2 * n + i];
+    scores[i] = s;
+    ends[2 * i] = eq;
+    ends[2 * i + 1] = et;
+    if (!span) continue;
+    // impossible: the best alignment ending at the end cell lies in the prefix
+    if (s > 0 && h[3 * n + i] != s) bad = std::min<int64_t>(bad, i);
+    starts[2 * i] = s > 0 ? eq - h[4 * n + i] : -1;
+    starts[2 * i + 1] = s > 0 ? et - h[5 * n + i] : -1;
+  }
+  if (bad != INT64_MAX)
+    return fail(ST_ECUDA, "pair %llu: reverse pass scored %d, forward %d", static_cast<unsigned long long>(bad),
+                h[3 * n + bad], h[bad]);
+  return ST_OK;
 }
 
 extern "C" int st_sw_score_end_pairs(st_ctx* c, const st_pair* pairs, uint64_t n, int32_t open, int32_t ext,
@@ -2822,9 +2939,8 @@ extern "C" int st_sw_score_end(st_ctx* c, uint32_t profile, const uint8_t* targe
   db.offset = reinterpret_cast<const uint64_t*>(a.as<char>() + tb);
   db.length = reinterpret_cast<const uint32_t*>(a.as<char>() + tb + 8);
   db.n_seqs = 1;
-  const uint32_t t0 = 0;
   int32_t ends[2];
-  ST_TRY(end_pairs_run(c, db, &profile, &t0, 1, m, n, open, ext, false, score, ends, nullptr));
+  ST_TRY(end_single_run(c, db, profile, m, n, open, ext, score, ends));
   *q_end = ends[0];
   *t_end = ends[1];
   return ST_OK;

@@ -43,6 +43,17 @@
 // pipe instead of prmt measured no faster (6.3 against 6.4 T cells/s in a bare cell
 // loop: the third register operand of both pipes' instructions is what limits then).
 //
+// End cells.  In the end modes a column's maximum is compared with a threshold
+// before anything else is done: the best score seen by this lane or by the lanes
+// above it (their g travels with the columns), less one, as an equal score may
+// come first by its column.  Only a column above it looks for the row and
+// updates the lane's optimum, ordered by score, column, row; the fold takes the
+// first over the lanes.  The reverse pass knows its score, so only the optimum
+// itself passes its threshold; it stages the query backwards, reads the target
+// backwards from the end cell, and masks the rows before the prefix to score 0,
+// which leaves H = 0 and the gap states of a first row, the prefix's border.
+// 4,000 spans of 280 x 280 cells took 4.0 ms with one warp a pair in 32 bits.
+//
 // Exactness.  The adds wrap instead of saturating.  If no t anywhere exceeds
 // T = 32767 - max(0, max score), no sum can leave the int16 range (E, F >=
 // -open-extend, S is int8), so the result is exact; otherwise the first t
@@ -90,7 +101,19 @@ struct Sw16Params {
   uint2* scratch;         // pass boundary rows, scratch_stride entries per group
   uint32_t scratch_stride;
   int32_t open, ext;
+  // end-cell modes: end cell (query, target) of each pair, -1 for a zero score; in the reverse mode the end of
+  // the reversed prefix [0, rev_q] x [0, rev_t] whose forward score is rev_score
+  int32_t* end_q = nullptr;
+  int32_t* end_t = nullptr;
+  const int32_t* rev_q = nullptr;
+  const int32_t* rev_t = nullptr;
+  const int32_t* rev_score = nullptr;
 };
+
+// What a pass reports: the score; the score and its end cell, the first optimum in column-major order
+// (src/simd.rs:375-381); or the end cell of the reversed prefixes (the start search of align_canonical,
+// src/align.rs:848-866), whose score is known.
+enum Sw16Mode { kSw16Score = 0, kSw16End = 1, kSw16RevEnd = 2 };
 
 constexpr uint32_t kNoPair = 0xFFFFFFFFu;
 
@@ -146,6 +169,17 @@ __device__ __forceinline__ uint32_t load_codes(const uint8_t* t, uint32_t len16,
   else return __ldg(t + c);
 }
 
+// Four residues of a target read backwards from position last: positions last - c .. last - c - 3 (sentinels
+// below position 0), from two aligned words.
+__device__ __forceinline__ uint32_t load_codes_rev(const uint8_t* t, int last, int c) {
+  const int p = last - c;
+  if (p < 0) return 0x15151515u;
+  const uint32_t* w = reinterpret_cast<const uint32_t*>(t) + (p >> 2);
+  const uint32_t hi = __ldg(w), lo = p >= 4 ? __ldg(w - 1) : 0x15151515u;
+  const uint32_t s = static_cast<uint32_t>(p & 3);
+  return __byte_perm(lo, hi, 0x1234u + s * 0x1111u);  // bytes s + 4, s + 3, s + 2, s + 1 of the eight
+}
+
 // acc + (byte j of bytes) * mul: the 16-bit x byte dot product with mul in the half that meets byte j
 // (bits 16-31 for odd j) and zero in the other.
 __device__ __forceinline__ uint32_t dot_byte(int j, uint32_t mul, uint32_t bytes, uint32_t acc) {
@@ -189,8 +223,10 @@ __device__ __forceinline__ void store_bnd(uint2* b, const uint32_t (&h)[C], cons
 struct Sw16Pair2 {
   const uint8_t* tA;
   const uint8_t* tB;
-  uint32_t lenA, lenB;
+  uint32_t lenA, lenB;  // reverse mode: residues of the prefix
   uint32_t pA, pB;
+  int32_t sA, sB;       // reverse mode: the forward scores
+  uint32_t offA, offB;  // and the rows of the reversed query before the prefix
 };
 
 __device__ __forceinline__ Sw16Pair2 load_pair2(const Sw16Params& prm, uint32_t slot_begin, int grp) {
@@ -206,6 +242,27 @@ __device__ __forceinline__ Sw16Pair2 load_pair2(const Sw16Params& prm, uint32_t 
   return r;
 }
 
+// The reverse mode's view: the prefix of each half and its score (0: nothing to search, the pair scored 0 or is
+// in the 32-bit list).
+__device__ __forceinline__ void load_rev(const Sw16Params& prm, uint32_t p, uint32_t m, int32_t thresh, uint32_t& len,
+                                         int32_t& score, uint32_t& off) {
+  len = 0;
+  score = 0;
+  off = 0;
+  if (p == kNoPair) return;
+  const int32_t s = prm.rev_score[p];
+  if (s <= 0 || s > thresh) return;
+  score = s;
+  len = static_cast<uint32_t>(prm.rev_t[p]) + 1;
+  off = m - 1 - static_cast<uint32_t>(prm.rev_q[p]);
+}
+
+// Bytes of word v (rows 4v .. 4v+3 of a lane) that lie at or past row nz, as a byte mask.
+__device__ __forceinline__ uint32_t rows_from(int nz, int v) {
+  const int k = nz - 4 * v;
+  return k <= 0 ? 0xFFFFFFFFu : (k >= 4 ? 0u : 0xFFFFFFFFu << (8 * k));
+}
+
 // Persistent kernel: CTAs pull CTA tasks (one query each) from a global
 // counter and stage the query's int8 profile in shared memory; each warp then
 // streams the CTA task's warp tasks, claimed from a shared counter.
@@ -219,8 +276,9 @@ __device__ __forceinline__ Sw16Pair2 load_pair2(const Sw16Params& prm, uint32_t 
 // of its rows.  Streamed cells/s of single classes on the 1.2 M-pair PSSM batch,
 // before -> after: <8,32> 5.23 -> 5.79 T, <16,32> 5.13 -> 5.77, <16,24> 5.40 -> 5.67,
 // <8,24> 5.41 -> 5.60, <16,20> 5.20 -> 5.54, <8,8> 4.57 -> 4.68 (4.25 with two CTAs).
-template <int G, int R, int C, int WARPS>
-__global__ void __launch_bounds__(WARPS * 32, WARPS == 4 || R == 8 ? 3 : 2) sw16_kernel(const Sw16Params prm) {
+template <int G, int R, int C, int WARPS, int MODE = kSw16Score>
+__global__ void __launch_bounds__(WARPS * 32, WARPS == 4 || (R == 8 && MODE == kSw16Score) ? 3 : 2)
+    sw16_kernel(const Sw16Params prm) {
   using Tile = Sw16Tile<G, R, C>;
   constexpr int NG = Tile::kGroups;
   constexpr uint32_t FULL = 0xFFFFFFFFu;
@@ -228,6 +286,11 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 4 || R == 8 ? 3 : 2) sw16
   __shared__ uint32_t s_task, s_next;
   __shared__ int32_t s_best[WARPS][NG][kSlotRing][2];
   __shared__ uint32_t s_pair[WARPS][NG][kSlotRing][2];
+  constexpr bool kEnds = MODE != kSw16Score;
+  // end-cell modes: (score, inverted column and row) of a task's two targets, largest first; the reverse mode's
+  // (forward score, rows before the prefix)
+  __shared__ unsigned long long s_end[kEnds ? WARPS : 1][kEnds ? NG : 1][kSlotRing][2];
+  __shared__ int2 s_rev[MODE == kSw16RevEnd ? WARPS : 1][MODE == kSw16RevEnd ? NG : 1][kSlotRing][2];
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
@@ -249,6 +312,7 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 4 || R == 8 ? 3 : 2) sw16
     const uint32_t q = task.query;
     const uint32_t m_pad = task.m_pad;
     const int P = static_cast<int>(m_pad / (G * R));
+    const uint32_t m = MODE == kSw16RevEnd ? prm.prof.qlen[q] : 0u;
     {  // stage the profile: 22 residue rows of m_pad int8 scores, zero past the stored stride
       const uint32_t chunks_per_row = m_pad / 16;
       const uint32_t stride = prm.prof.stride8[q];
@@ -257,7 +321,14 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 4 || R == 8 ? 3 : 2) sw16
         const uint32_t r = idx / chunks_per_row;
         const uint32_t i = (idx - r * chunks_per_row) * 16;
         uint4 v = make_uint4(0, 0, 0, 0);
-        if (i < stride) v = *reinterpret_cast<const uint4*>(src + static_cast<size_t>(r) * stride + i);
+        if constexpr (MODE == kSw16RevEnd) {  // the query backwards
+          int8_t* b = reinterpret_cast<int8_t*>(&v);
+#pragma unroll
+          for (int k = 0; k < 16; ++k)
+            if (i + k < m) b[k] = src[static_cast<size_t>(r) * stride + (m - 1 - i - k)];
+        } else {
+          if (i < stride) v = *reinterpret_cast<const uint4*>(src + static_cast<size_t>(r) * stride + i);
+        }
         *reinterpret_cast<uint4*>(prof_s + static_cast<size_t>(r) * m_pad + i) = v;
       }
     }
@@ -284,20 +355,43 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 4 || R == 8 ? 3 : 2) sw16
       __syncthreads();
       continue;
     }
+    auto load_pairs = [&](uint32_t slot_begin) {
+      Sw16Pair2 r = load_pair2(prm, slot_begin, grp);
+      if constexpr (MODE == kSw16RevEnd) {
+        load_rev(prm, r.pA, m, thresh, r.lenA, r.sA, r.offA);
+        load_rev(prm, r.pB, m, thresh, r.lenB, r.sB, r.offB);
+      }
+      return r;
+    };
+    auto load_step = [&](const uint8_t* t, uint32_t len, int c) -> uint32_t {
+      if constexpr (MODE == kSw16RevEnd) return load_codes_rev(t, static_cast<int>(len) - 1, c);
+      else return load_codes<C>(t, len, c);
+    };
+    // a task enters the ring (the group's feeder)
+    auto open_slot = [&](int slot, const Sw16Pair2& r) {
+      s_pair[warp][grp][slot][0] = r.pA;
+      s_pair[warp][grp][slot][1] = r.pB;
+      if constexpr (kEnds) {
+        s_end[warp][grp][slot][0] = 0;
+        s_end[warp][grp][slot][1] = 0;
+        if constexpr (MODE == kSw16RevEnd) {
+          s_rev[warp][grp][slot][0] = make_int2(r.sA, static_cast<int>(r.offA));
+          s_rev[warp][grp][slot][1] = make_int2(r.sB, static_cast<int>(r.offB));
+        }
+      } else {
+        s_best[warp][grp][slot][0] = 0;
+        s_best[warp][grp][slot][1] = 0;
+      }
+    };
     Sw16WarpTask wt_cur = prm.warp_tasks[w_cur];
     Sw16Pair2 cur{};
-    if (feeder) cur = load_pair2(prm, wt_cur.slot_begin, grp);
+    if (feeder) cur = load_pairs(wt_cur.slot_begin);
     uint32_t w_nxt = claim();
     bool have_nxt = w_nxt < task.wt_end;
     Sw16WarpTask wt_nxt = have_nxt ? prm.warp_tasks[w_nxt] : Sw16WarpTask{0, 0};
     Sw16Pair2 nxt{};
-    if (have_nxt && feeder) nxt = load_pair2(prm, wt_nxt.slot_begin, grp);
-    if (feeder) {
-      s_pair[warp][grp][0][0] = cur.pA;
-      s_pair[warp][grp][0][1] = cur.pB;
-      s_best[warp][grp][0][0] = 0;
-      s_best[warp][grp][0][1] = 0;
-    }
+    if (have_nxt && feeder) nxt = load_pairs(wt_nxt.slot_begin);
+    if (feeder) open_slot(0, cur);
     // Lane 0's position: column u_col of pass u_pass of task u_seq.  The control word of an ordinary step is
     // u_ctl; the first and the last step of a pass add their events, so an ordinary step takes no decisions
     // beyond comparing its column with the pass's end.
@@ -317,6 +411,15 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 4 || R == 8 ? 3 : 2) sw16
     uint32_t row0 = static_cast<uint32_t>(gl * R);  // this lane's first row of its pass
     uint32_t my_col = 0;                            // its column
     const uint32_t mul_lo = m_pad, mul_hi = m_pad << 16;
+    // end-cell modes: this lane's first optimum per half as score and column << 16 | row; thr: only a cell above
+    // it is looked at; g: the best score of the lanes above and of this one
+    int32_t endsA = 0, endsB = 0;
+    uint32_t endA = 0, endB = 0, thr = 0, g = 0;
+    uint32_t maskA[kEnds ? Tile::kWords : 1], maskB[kEnds ? Tile::kWords : 1];
+    if constexpr (MODE == kSw16RevEnd) {
+#pragma unroll
+      for (int v = 0; v < Tile::kWords; ++v) maskA[v] = maskB[v] = 0xFFFFFFFFu;
+    }
     // outgoing registers: a lane's outputs for the lane below (the feeder: lane 0's next inputs)
     uint32_t my_ctl = 0, my_rA = SENTW, my_rB = SENTW;
     uint32_t my_h[C], my_f[C];
@@ -327,8 +430,8 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 4 || R == 8 ? 3 : 2) sw16
     }
     if (feeder) {  // lane 0's first step: column 0, pass 0 of the first task
       my_ctl = kCtlFirst | u_ctl;
-      my_rA = load_codes<C>(cur.tA, cur.lenA, 0);
-      my_rB = load_codes<C>(cur.tB, cur.lenB, 0);
+      my_rA = load_step(cur.tA, cur.lenA, 0);
+      my_rB = load_step(cur.tB, cur.lenB, 0);
     }
     __syncwarp();
 
@@ -343,6 +446,8 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 4 || R == 8 ? 3 : 2) sw16
         h_in[j] = __shfl_sync(FULL, my_h[j], src_lane);
         f_in[j] = __shfl_sync(FULL, my_f[j], src_lane);
       }
+      uint32_t g_in = 0;
+      if constexpr (MODE == kSw16End) g_in = __shfl_sync(FULL, g, src_lane);
       my_ctl = ctl;
       my_rA = rA;
       my_rB = rB;
@@ -359,18 +464,12 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 4 || R == 8 ? 3 : 2) sw16
             wt_cur = wt_nxt;
             cur = nxt;
             if (have) {
-              const int slot = u_seq & (kSlotRing - 1);
-              if (feeder) {
-                s_pair[warp][grp][slot][0] = cur.pA;
-                s_pair[warp][grp][slot][1] = cur.pB;
-                s_best[warp][grp][slot][0] = 0;
-                s_best[warp][grp][slot][1] = 0;
-              }
+              if (feeder) open_slot(u_seq & (kSlotRing - 1), cur);
               w_nxt = claim();
               have_nxt = w_nxt < task.wt_end;
               if (have_nxt) {
                 wt_nxt = prm.warp_tasks[w_nxt];
-                if (feeder) nxt = load_pair2(prm, wt_nxt.slot_begin, grp);
+                if (feeder) nxt = load_pairs(wt_nxt.slot_begin);
               }
               u_end = static_cast<int>(wt_cur.ncols);
             }
@@ -395,8 +494,8 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 4 || R == 8 ? 3 : 2) sw16
       if (!have) ++drain;
       uint32_t nA = SENTW, nB = SENTW;
       if (feeder) {  // its residues, on their way while this step is computed
-        nA = load_codes<C>(cur.tA, cur.lenA, u_col);
-        nB = load_codes<C>(cur.tB, cur.lenB, u_col);
+        nA = load_step(cur.tA, cur.lenA, u_col);
+        nB = load_step(cur.tB, cur.lenB, u_col);
       }
       // first column of a pass: left border H = 0, first-column E. The groups of a
       // warp move in step, so lane l of every group resets on the same steps: the
@@ -411,7 +510,34 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 4 || R == 8 ? 3 : 2) sw16
           hup_prev = 0;
           my_col = 0;
           row0 = ((ctl >> 16) & 0xFFu) * (G * R) + gl * R;
+          if constexpr (kEnds) {
+            const bool begin = (ctl & 0x00FF0000u) == 0;  // the task's first pass
+            if (begin) {
+              endsA = endsB = 0;
+              endA = endB = 0;
+              g = 0;
+            }
+            if constexpr (MODE == kSw16RevEnd) {
+              // only the known score is looked for; the rows before the prefix score 0 (H = 0, as above a query)
+              const int slot = static_cast<int>((ctl >> 24) & 7u);
+              const int2 a = s_rev[warp][grp][slot][0], b = s_rev[warp][grp][slot][1];
+              thr = (a.x > 0 ? static_cast<uint32_t>(a.x - 1) : 32767u) |
+                    ((b.x > 0 ? static_cast<uint32_t>(b.x - 1) : 32767u) << 16);
+#pragma unroll
+              for (int v = 0; v < Tile::kWords; ++v) {
+                maskA[v] = rows_from(a.y - static_cast<int>(row0), v);
+                maskB[v] = rows_from(b.y - static_cast<int>(row0), v);
+              }
+            } else {
+              // a later pass may reach the same score in an earlier column
+              thr = static_cast<uint32_t>(max(endsA - 1, 0)) | (static_cast<uint32_t>(max(endsB - 1, 0)) << 16);
+            }
+          }
         }
+      }
+      if constexpr (MODE == kSw16End) {
+        if (gl != 0) g = pk_max(g, g_in);
+        thr = pk_max(thr, pk_add(g, 0xFFFFFFFFu));  // g - 1: an equal score may come first by its column
       }
 #pragma unroll
       for (int j = 0; j < C; ++j) {
@@ -421,9 +547,17 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 4 || R == 8 ? 3 : 2) sw16
         uint32_t wa[Tile::kWords], wb[Tile::kWords];
         load_rows8<R>(prof_s + oA, wa);
         load_rows8<R>(prof_s + oB, wb);
+        if constexpr (MODE == kSw16RevEnd) {
+#pragma unroll
+          for (int v = 0; v < Tile::kWords; ++v) {
+            wa[v] &= maskA[v];
+            wb[v] &= maskB[v];
+          }
+        }
         uint32_t hd = j == 0 ? hup_prev : h_in[j - 1];
         uint32_t F = f_in[j];
         uint32_t t_odd = 0;
+        if constexpr (kEnds) best = 0;  // the column's
 #pragma unroll
         for (int k = 0; k < R; ++k) {
           const uint32_t S = prmt(wa[k >> 2], wb[k >> 2], sel_pair(k & 3));
@@ -440,9 +574,71 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 4 || R == 8 ? 3 : 2) sw16
         }
         my_h[j] = Hp[R - 1];
         my_f[j] = F;
+        if constexpr (kEnds) {
+          if (pk_max(best, thr) != thr) {  // rare: a cell of this column may be the optimum
+            const uint32_t at = (my_col + j) << 16;
+            if (pk_lo(best) > pk_lo(thr)) {
+              const uint32_t v = best & 0xFFFFu;
+              uint32_t row = 0;
+#pragma unroll
+              for (int k = R - 1; k >= 0; --k)
+                if ((Hp[k] & 0xFFFFu) == v) row = k;
+              const uint32_t key = at | (row0 + row);
+              if (static_cast<int32_t>(v) > endsA || key < endA) {
+                endsA = static_cast<int32_t>(v);
+                endA = key;
+              }
+              thr = (thr & 0xFFFF0000u) | v;
+            }
+            if (pk_hi(best) > pk_hi(thr)) {
+              const uint32_t v = best >> 16;
+              uint32_t row = 0;
+#pragma unroll
+              for (int k = R - 1; k >= 0; --k)
+                if ((Hp[k] >> 16) == v) row = k;
+              const uint32_t key = at | (row0 + row);
+              if (static_cast<int32_t>(v) > endsB || key < endB) {
+                endsB = static_cast<int32_t>(v);
+                endB = key;
+              }
+              thr = (thr & 0xFFFFu) | (v << 16);
+            }
+            if constexpr (MODE == kSw16End) g = pk_max(g, best);
+          }
+        }
       }
       hup_prev = h_in[C - 1];
-      if (ctl & kCtlLast) {  // this lane's part of the task is done: fold its maximum into the task slot
+      if constexpr (kEnds) {
+        if (ctl & kCtlLast) {  // this lane's part of the task is done: fold its optimum into the task slot
+          const int slot = static_cast<int>((ctl >> 24) & 7u);
+          unsigned long long* e = s_end[warp][grp][slot];
+          if (endsA > 0) atomicMax(e, (static_cast<unsigned long long>(endsA) << 32) | (0xFFFFFFFFu - endA));
+          if (endsB > 0) atomicMax(e + 1, (static_cast<unsigned long long>(endsB) << 32) | (0xFFFFFFFFu - endB));
+          if (feeder) {  // the group's last lane finishes the task last
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+              const uint32_t p = s_pair[warp][grp][slot][h];
+              if (p == kNoPair) continue;
+              const unsigned long long x = e[h];
+              const int32_t sc = static_cast<int32_t>(x >> 32);
+              const uint32_t key = 0xFFFFFFFFu - static_cast<uint32_t>(x);
+              if constexpr (MODE == kSw16End) {
+                if (sc > thresh) {
+                  prm.ovf_pairs[atomicAdd(prm.ovf_count, 1u)] = p;
+                } else if (sc > 0) {  // a zero score keeps its cleared outputs
+                  prm.scores[p] = sc;
+                  prm.end_q[p] = static_cast<int32_t>(key & 0xFFFFu);
+                  prm.end_t[p] = static_cast<int32_t>(key >> 16);
+                }
+              } else if (sc > 0) {
+                prm.scores[p] = sc;
+                prm.end_q[p] = static_cast<int32_t>(key & 0xFFFFu) - s_rev[warp][grp][slot][h].y;
+                prm.end_t[p] = static_cast<int32_t>(key >> 16);
+              }
+            }
+          }
+        }
+      } else if (ctl & kCtlLast) {  // this lane's part of the task is done: fold its maximum into the task slot
         const int slot = static_cast<int>((ctl >> 24) & 7u);
         atomicMax(&s_best[warp][grp][slot][0], pk_lo(best));
         atomicMax(&s_best[warp][grp][slot][1], pk_hi(best));

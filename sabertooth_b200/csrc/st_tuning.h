@@ -134,11 +134,12 @@ TUNE_HD inline uint32_t tune_cta_unit(uint64_t wt_total, uint32_t sms, uint32_t 
 
 // est[c] = the chip's time (ps) for the query in class c: streamed cells over the rate; a class without a rate
 // counts 1e150 times its cells (taken only when no class with a rate stages the query), one that cannot stage it
-// 1e300.  Returns the least time over the classes with a rate (0: none).
-inline double tuning_estimate(const Tuning* t, uint32_t m, const uint32_t* tlen_desc, size_t n, double* est) {
+// or is not in `allowed` 1e300.  Returns the least time over the classes with a rate (0: none).
+inline double tuning_estimate(const Tuning* t, uint32_t m, const uint32_t* tlen_desc, size_t n, double* est,
+                              uint32_t allowed) {
   double best = 0.0;
   for (int c = 0; c < st_tuning_num_classes(); ++c) {
-    const double v = tune_streamed(c, m, tlen_desc, n);
+    const double v = (allowed >> c & 1u) ? tune_streamed(c, m, tlen_desc, n) : 1e300;
     est[c] = v >= 1e300 ? 1e300 : (t->rate[c] > 0.0f ? v / t->rate[c] : v * 1e150);
     if (est[c] < 1e140 && (best == 0.0 || est[c] < best)) best = est[c];
   }
