@@ -127,7 +127,7 @@ template <int G, int R, int C>
 struct Sw16Tile {
   static_assert(G == 4 || G == 8 || G == 16 || G == 32, "group size");
   static_assert(R % 4 == 0 && R >= 8 && R <= 32, "rows per lane");
-  static_assert(C == 1 || C == 2 || C == 4, "columns per step");
+  static_assert(C == 2 || C == 4, "columns per step");
   static constexpr int kGroups = 32 / G;
   static constexpr int kSlots = 2 * kGroups;
   static constexpr int kWords = R / 4;
@@ -159,14 +159,19 @@ __device__ __forceinline__ void load_rows8(const int8_t* p, uint32_t (&w)[R / 4]
   }
 }
 
-// C residue codes of a target starting at column c (c is a multiple of C), or sentinels past its end.
+// C residue codes of a target starting at column c (c is a multiple of C), or sentinels past its end or without
+// `on`.  A predicated load: the lanes that do not feed the stream pass it without a branch.
 template <int C>
-__device__ __forceinline__ uint32_t load_codes(const uint8_t* t, uint32_t len16, int c) {
-  constexpr uint32_t sent = 0x15151515u & (C == 4 ? 0xFFFFFFFFu : (C == 2 ? 0xFFFFu : 0xFFu));
-  if (static_cast<uint32_t>(c) >= len16) return sent;
-  if constexpr (C == 4) return __ldg(reinterpret_cast<const uint32_t*>(t + c));
-  else if constexpr (C == 2) return __ldg(reinterpret_cast<const uint16_t*>(t + c));
-  else return __ldg(t + c);
+__device__ __forceinline__ uint32_t load_codes(bool on, const uint8_t* t, uint32_t len16, int c) {
+  uint32_t v = 0x15151515u & (C == 4 ? 0xFFFFFFFFu : (C == 2 ? 0xFFFFu : 0xFFu));
+  const uint32_t p = on && static_cast<uint32_t>(c) < len16;
+  if constexpr (C == 4)
+    asm volatile("{ .reg .pred q; setp.ne.u32 q, %2, 0; @q ld.global.nc.u32 %0, [%1]; }" : "+r"(v) : "l"(t + c), "r"(p));
+  else if constexpr (C == 2)
+    asm volatile("{ .reg .pred q; setp.ne.u32 q, %2, 0; @q ld.global.nc.u16 %0, [%1]; }" : "+r"(v) : "l"(t + c), "r"(p));
+  else
+    asm volatile("{ .reg .pred q; setp.ne.u32 q, %2, 0; @q ld.global.nc.u8 %0, [%1]; }" : "+r"(v) : "l"(t + c), "r"(p));
+  return v;
 }
 
 // Four residues of a target read backwards from position last: positions last - c .. last - c - 3 (sentinels
@@ -191,32 +196,26 @@ __device__ __forceinline__ uint32_t dot_byte(int j, uint32_t mul, uint32_t bytes
   return d;
 }
 
+// (H, F) of C columns of the boundary line, loaded or stored when `on` (predicated, as load_codes).
 template <int C>
-__device__ __forceinline__ void load_bnd(const uint2* b, uint32_t (&h)[C], uint32_t (&f)[C]) {
-  if constexpr (C == 4) {
-    const uint4 x = *reinterpret_cast<const uint4*>(b);
-    const uint4 y = *reinterpret_cast<const uint4*>(b + 2);
-    h[0] = x.x; f[0] = x.y; h[1] = x.z; f[1] = x.w;
-    h[2] = y.x; f[2] = y.y; h[3] = y.z; f[3] = y.w;
-  } else if constexpr (C == 2) {
-    const uint4 x = *reinterpret_cast<const uint4*>(b);
-    h[0] = x.x; f[0] = x.y; h[1] = x.z; f[1] = x.w;
-  } else {
-    const uint2 x = *b;
-    h[0] = x.x; f[0] = x.y;
-  }
+__device__ __forceinline__ void load_bnd(bool on, const uint2* b, uint32_t (&h)[C], uint32_t (&f)[C]) {
+  static_assert(C % 2 == 0, "whole vectors");
+  const uint32_t p = on;
+#pragma unroll
+  for (int j = 0; j < C; j += 2)
+    asm volatile("{ .reg .pred q; setp.ne.u32 q, %5, 0; @q ld.global.v4.u32 {%0, %1, %2, %3}, [%4]; }"
+                 : "+r"(h[j]), "+r"(f[j]), "+r"(h[j + 1]), "+r"(f[j + 1])
+                 : "l"(b + j), "r"(p)
+                 : "memory");
 }
-
 template <int C>
-__device__ __forceinline__ void store_bnd(uint2* b, const uint32_t (&h)[C], const uint32_t (&f)[C]) {
-  if constexpr (C == 4) {
-    *reinterpret_cast<uint4*>(b) = make_uint4(h[0], f[0], h[1], f[1]);
-    *reinterpret_cast<uint4*>(b + 2) = make_uint4(h[2], f[2], h[3], f[3]);
-  } else if constexpr (C == 2) {
-    *reinterpret_cast<uint4*>(b) = make_uint4(h[0], f[0], h[1], f[1]);
-  } else {
-    *b = make_uint2(h[0], f[0]);
-  }
+__device__ __forceinline__ void store_bnd(bool on, uint2* b, const uint32_t (&h)[C], const uint32_t (&f)[C]) {
+  const uint32_t p = on;
+#pragma unroll
+  for (int j = 0; j < C; j += 2)
+    asm volatile("{ .reg .pred q; setp.ne.u32 q, %5, 0; @q st.global.v4.u32 [%4], {%0, %1, %2, %3}; }" ::"r"(h[j]),
+                 "r"(f[j]), "r"(h[j + 1]), "r"(f[j + 1]), "l"(b + j), "r"(p)
+                 : "memory");
 }
 
 // Per-group view of a warp task's two targets (meaningful in the group's lane 0).
@@ -268,14 +267,16 @@ __device__ __forceinline__ uint32_t rows_from(int nz, int v) {
 // streams the CTA task's warp tasks, claimed from a shared counter.
 //
 // Beside the cells a step costs its 3 + 2C shuffles, the residues' row offsets
-// (one dot product each, dot_byte) and the feeder's loads; the decisions of the
-// stream (pass, task, idle) are taken only at the end of a pass, and the first
-// pass reads no boundary line.  Registers are the other lever: asking for three
-// CTAs of four warps (R >= 28, up to 168 registers) or three of eight (R = 8)
-// and two of eight otherwise lets the profile loads of a column be issued ahead
-// of its rows.  Streamed cells/s of single classes on the 1.2 M-pair PSSM batch,
-// before -> after: <8,32> 5.23 -> 5.79 T, <16,32> 5.13 -> 5.77, <16,24> 5.40 -> 5.67,
-// <8,24> 5.41 -> 5.60, <16,20> 5.20 -> 5.54, <8,8> 4.57 -> 4.68 (4.25 with two CTAs).
+// (one dot product each, dot_byte) and the feeder's loads and stores, which are
+// predicated; one vote decides whether any lane is at an event or lane 0 near
+// the end of its pass, and only then the stream is looked at (a lone warp's
+// step spent 160 of 1,140 cycles on resolving 15 branches, now 4).  Registers are
+// the other lever: asking for three CTAs of four warps (R >= 28, up to 168
+// registers) or three of eight (R = 8) and two of eight otherwise lets the
+// profile loads of a column be issued ahead of its rows.  Streamed cells/s of
+// single classes on the 1.2 M-pair PSSM batch, before -> after: <8,24> 5.41 -> 5.77 T,
+// <16,24> 5.40 -> 5.76, <16,32> 5.13 -> 5.62, <8,16> 4.96 -> 5.33, <8,12> 4.82 -> 5.17; a lone
+// warp's step <8,24> 1,756 -> 1,541 cycles, <8,8> 1,050 -> 771.
 template <int G, int R, int C, int WARPS, int MODE = kSw16Score>
 __global__ void __launch_bounds__(WARPS * 32, WARPS == 4 || (R == 8 && MODE == kSw16Score) ? 3 : 2)
     sw16_kernel(const Sw16Params prm) {
@@ -364,8 +365,8 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 4 || (R == 8 && MODE == k
       return r;
     };
     auto load_step = [&](const uint8_t* t, uint32_t len, int c) -> uint32_t {
-      if constexpr (MODE == kSw16RevEnd) return load_codes_rev(t, static_cast<int>(len) - 1, c);
-      else return load_codes<C>(t, len, c);
+      if constexpr (MODE == kSw16RevEnd) return feeder ? load_codes_rev(t, static_cast<int>(len) - 1, c) : SENTW;
+      else return load_codes<C>(feeder, t, len, c);
     };
     // a task enters the ring (the group's feeder)
     auto open_slot = [&](int slot, const Sw16Pair2& r) {
@@ -394,9 +395,10 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 4 || (R == 8 && MODE == k
     if (feeder) open_slot(0, cur);
     // Lane 0's position: column u_col of pass u_pass of task u_seq.  The control word of an ordinary step is
     // u_ctl; the first and the last step of a pass add their events, so an ordinary step takes no decisions
-    // beyond comparing its column with the pass's end.
-    int u_col = 0, u_pass = 0, u_seq = 0, drain = 0;
-    int u_end = static_cast<int>(wt_cur.ncols);  // columns of the pass
+    // beyond one vote (is any lane at an event, or lane 0 within a step of its pass's end).
+    int u_col = 0, u_pass = 0, u_seq = 0;
+    bool done = false;
+    int u_end = static_cast<int>(wt_cur.ncols);  // columns of the pass; of the idle steps at the end of the stream
     uint32_t u_ctl = P > 1 ? kCtlMore : 0u;
     uint32_t u_last = P > 1 ? 0u : kCtlLast;     // the event of the pass's last step
 
@@ -428,11 +430,10 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 4 || (R == 8 && MODE == k
       my_h[j] = 0;
       my_f[j] = F0;
     }
-    if (feeder) {  // lane 0's first step: column 0, pass 0 of the first task
-      my_ctl = kCtlFirst | u_ctl;
-      my_rA = load_step(cur.tA, cur.lenA, 0);
-      my_rB = load_step(cur.tB, cur.lenB, 0);
-    }
+    // lane 0's first step: column 0, pass 0 of the first task
+    if (feeder) my_ctl = kCtlFirst | u_ctl;
+    my_rA = load_step(cur.tA, cur.lenA, 0);
+    my_rB = load_step(cur.tB, cur.lenB, 0);
     __syncwarp();
 
     for (;;) {
@@ -454,10 +455,13 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 4 || (R == 8 && MODE == k
       // lane 0's next step (uniform across the warp)
       uint32_t n_ctl = u_ctl;
       u_col += C;
-      if (u_col == u_end) {
-        if (have) {
+      const bool event = __any_sync(FULL, (ctl & (kCtlFirst | kCtlLast)) != 0 || u_col + C >= u_end);
+      if (event) {
+        if (u_col == u_end) {
           n_ctl = kCtlFirst;
-          if (++u_pass == P) {  // task done: the pre-claimed task becomes current, claim the one after
+          if (!have) {  // the idle steps are over
+            done = true;
+          } else if (++u_pass == P) {  // task done: the pre-claimed task becomes current, claim the one after
             u_pass = 0;
             ++u_seq;
             have = have_nxt;
@@ -474,33 +478,22 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 4 || (R == 8 && MODE == k
               u_end = static_cast<int>(wt_cur.ncols);
             }
           }
+          u_col = 0;
           if (have) {
             const uint32_t at = (static_cast<uint32_t>(u_pass) << 16) |
                                 (static_cast<uint32_t>(u_seq & (kSlotRing - 1)) << 24);
             u_ctl = u_pass + 1 < P ? kCtlMore : 0u;
             u_last = u_pass + 1 < P ? 0u : kCtlLast | at;
             n_ctl |= u_ctl | at;
-            u_col = 0;
           } else {  // idle steps until the last lane has finished
             cur.lenA = cur.lenB = 0;
             u_ctl = u_last = n_ctl = 0u;
-            u_col = 0;
-            u_end = -C;
+            u_end = (G - 1) * C;
           }
+        } else if (u_col + C == u_end) {
+          n_ctl |= u_last;
         }
-      } else if (u_col + C == u_end) {
-        n_ctl |= u_last;
-      }
-      if (!have) ++drain;
-      uint32_t nA = SENTW, nB = SENTW;
-      if (feeder) {  // its residues, on their way while this step is computed
-        nA = load_step(cur.tA, cur.lenA, u_col);
-        nB = load_step(cur.tB, cur.lenB, u_col);
-      }
-      // first column of a pass: left border H = 0, first-column E. The groups of a
-      // warp move in step, so lane l of every group resets on the same steps: the
-      // branch is skipped on the other steps of a pass.
-      if (__any_sync(FULL, (ctl & kCtlFirst) != 0)) {
+        // first column of a pass: left border H = 0, first-column E
         if (ctl & kCtlFirst) {
 #pragma unroll
           for (int k = 0; k < R; ++k) {
@@ -534,7 +527,11 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 4 || (R == 8 && MODE == k
             }
           }
         }
+        __syncwarp();
       }
+      // the feeder's residues, on their way while this step is computed
+      const uint32_t nA = load_step(cur.tA, cur.lenA, u_col);
+      const uint32_t nB = load_step(cur.tB, cur.lenB, u_col);
       if constexpr (MODE == kSw16End) {
         if (gl != 0) g = pk_max(g, g_in);
         thr = pk_max(thr, pk_add(g, 0xFFFFFFFFu));  // g - 1: an equal score may come first by its column
@@ -609,7 +606,7 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 4 || (R == 8 && MODE == k
       }
       hup_prev = h_in[C - 1];
       if constexpr (kEnds) {
-        if (ctl & kCtlLast) {  // this lane's part of the task is done: fold its optimum into the task slot
+        if (event && (ctl & kCtlLast)) {  // this lane's part of the task is done: fold its optimum into the task slot
           const int slot = static_cast<int>((ctl >> 24) & 7u);
           unsigned long long* e = s_end[warp][grp][slot];
           if (endsA > 0) atomicMax(e, (static_cast<unsigned long long>(endsA) << 32) | (0xFFFFFFFFu - endA));
@@ -638,7 +635,7 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 4 || (R == 8 && MODE == k
             }
           }
         }
-      } else if (ctl & kCtlLast) {  // this lane's part of the task is done: fold its maximum into the task slot
+      } else if (event && (ctl & kCtlLast)) {  // this lane's part of the task is done: fold its maximum into the task slot
         const int slot = static_cast<int>((ctl >> 24) & 7u);
         atomicMax(&s_best[warp][grp][slot][0], pk_lo(best));
         atomicMax(&s_best[warp][grp][slot][1], pk_hi(best));
@@ -665,25 +662,22 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 4 || (R == 8 && MODE == k
         }
       }
       // the bottom row of a pass that is not the last goes to the scratch line
-      if (feeder && (ctl & kCtlMore)) store_bnd<C>(bnd + my_col, my_h, my_f);
+      store_bnd<C>(feeder && (ctl & kCtlMore) != 0, bnd + my_col, my_h, my_f);
       my_col += C;
-      __syncwarp();
-      if (drain >= G) break;  // the last lane has done the last step
-      // the feeder's outgoing registers become lane 0's inputs for the next step
+      if (done) break;
+      // the feeder's outgoing registers become lane 0's inputs for the next step; above the query's first row
+      // H = 0 and the first-row F, else the previous pass's bottom row (which this lane stored)
       if (feeder) {
         my_ctl = n_ctl;
         my_rA = nA;
         my_rB = nB;
-        if (u_pass > 0) {
-          load_bnd<C>(bnd + u_col, my_h, my_f);
-        } else {  // above the query's first row: H = 0, first-row F
 #pragma unroll
-          for (int j = 0; j < C; ++j) {
-            my_h[j] = 0;
-            my_f[j] = F0;
-          }
+        for (int j = 0; j < C; ++j) {
+          my_h[j] = 0;
+          my_f[j] = F0;
         }
       }
+      load_bnd<C>(feeder && u_pass > 0, bnd + u_col, my_h, my_f);
     }
     __syncthreads();
   }

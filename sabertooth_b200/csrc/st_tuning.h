@@ -63,13 +63,13 @@ inline float tuning_default_rate(int G, int R, int C) {
     int G, R;
     float rate;
   } kRates[] = {
-      {4, 8, 3.737f}, {8, 8, 4.675f}, {16, 8, 4.779f}, {32, 8, 4.641f},
-      {4, 12, 3.677f}, {8, 12, 4.824f}, {16, 12, 4.983f}, {32, 12, 4.887f},
-      {4, 16, 4.073f}, {8, 16, 5.130f}, {16, 16, 5.240f}, {32, 16, 5.070f},
-      {4, 20, 4.443f}, {8, 20, 5.446f}, {16, 20, 5.541f}, {32, 20, 5.424f},
-      {4, 24, 4.677f}, {8, 24, 5.595f}, {16, 24, 5.670f}, {32, 24, 5.477f},
-      {4, 28, 5.082f}, {8, 28, 5.273f}, {16, 28, 5.294f}, {4, 32, 5.581f},
-      {8, 32, 5.792f}, {16, 32, 5.771f}, {32, 32, 5.663f},
+      {4, 8, 4.095f}, {8, 8, 4.718f}, {16, 8, 4.677f}, {32, 8, 4.762f},
+      {4, 12, 3.985f}, {8, 12, 5.166f}, {16, 12, 5.248f}, {32, 12, 5.037f},
+      {4, 16, 4.356f}, {8, 16, 5.331f}, {16, 16, 5.360f}, {32, 16, 5.190f},
+      {4, 20, 4.543f}, {8, 20, 5.438f}, {16, 20, 5.442f}, {32, 20, 5.421f},
+      {4, 24, 4.926f}, {8, 24, 5.766f}, {16, 24, 5.762f}, {32, 24, 5.444f},
+      {4, 28, 5.305f}, {8, 28, 5.452f}, {16, 28, 5.471f}, {4, 32, 5.464f},
+      {8, 32, 5.600f}, {16, 32, 5.615f}, {32, 32, 5.578f},
   };
   for (const auto& r : kRates)
     if (r.G == G && r.R == R) return r.rate;
@@ -107,11 +107,12 @@ inline double tune_streamed(int c, uint32_t m, const uint32_t* tlen_desc, size_t
 }
 
 // Critical path: the time of the wavefront that streams a query's longest target, alone on its scheduler, in
-// picoseconds.  A step of a lone warp takes about 700 cycles (the shuffles, the profile loads, the dependent
-// rows) plus 11.5 for each of its R*C cell pairs; measured at 1,965 MHz on 4,000-column targets: 1,090 cycles for
-// R = 8, 1,380 for 16, 1,780 for 24, 2,200 for 32 (C = 4), 990 for R = 16, C = 2.
+// picoseconds.  A step of a lone warp takes about 400 cycles (the shuffles, the profile loads, the dependent
+// rows; 560 with 4 or 32 lanes) plus 11.8 for each of its R*C cell pairs; measured at 1,965 MHz on 4,000-column
+// targets: <8,8> 771 cycles, <32,8> 938, <16,16> 1,182, <8,24> 1,541, <32,24> 1,570, <32,32> 1,932.
 TUNE_HD inline double tune_crit_ps(uint32_t G, uint32_t R, uint32_t C, uint32_t P, uint32_t ncols) {
-  return (static_cast<double>(P) * (ncols / C) + G) * (700.0 + 11.5 * (R * C)) * (1e6 / 1965.0);
+  const double fixed = G == 8 || G == 16 || C == 2 ? 400.0 : 560.0;
+  return (static_cast<double>(P) * (ncols / C) + G) * (fixed + 11.8 * (R * C)) * (1e6 / 1965.0);
 }
 
 // What a query costs the batch in a class: the chip's time for its cells, plus what its critical path adds when
