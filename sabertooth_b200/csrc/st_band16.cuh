@@ -5,8 +5,8 @@
 // infinity) leaves a band of 2*radius + 1 cells per row; pairs carrying it
 // have their own query each in the long/overflow mix, so the 16-bit tile
 // classes (which share one query's staged profile among many targets) do not
-// fit them.  Here one warp scores two banded pairs at once, one per 16-bit
-// half of every register, with the geometry of the exact 32-bit kernel: lane l
+// fit them.  Here two banded pairs are scored at once, one per 16-bit half of
+// every register.  band16_couple has the geometry of the exact 32-bit kernel: lane l
 // owns query rows [pass*256 + 8l, +8), the columns of both pairs' band windows
 // stream through the warp as a wavefront, and a query of more than 256 rows
 // is scored in passes whose bottom row goes through the warp's scratch line.
@@ -23,9 +23,11 @@
 // past a window's columns or on a half's idle passes score 0 and cannot raise
 // the maximum (open, extend >= 0).
 //
-// Work: warps claim two entries of the 32-bit list's static part at a time;
+// Work: warps claim four entries of the 32-bit list's static part at a time;
 // entries that are not banded pairs with int8 rows are left to the 32-bit
-// kernel, which skips exactly the entries taken here (band16_takes).
+// kernel, which skips exactly the entries taken here (band16_takes).  Bands of
+// radius up to 140 take band16_ring, wider ones the whole-warp passes of
+// band16_couple (which then stream mostly band cells).
 #pragma once
 #include "st_common.cuh"
 #include "st_sw32.cuh"
@@ -347,6 +349,173 @@ __device__ __forceinline__ void band16_couple(const Sw32Params& prm, uint32_t pA
   }
 }
 
+// ---- narrow bands: row blocks chase each other along the diagonal ----
+// With radius r only 2r + 8 columns of a lane's eight rows hold band cells, a third
+// of the 256 + 2r columns that a whole-warp pass streams at r = 64.  Here a lane
+// streams just its own window.  Row block k (rows 8k .. 8k + 7) processes column
+// 8k + center - r + u at step 9k + u, 0 <= u < 2r + 8: block k - 1 left the bottom row's
+// cell above it one step before, so the blocks form a ring over G lanes (block k on
+// lane k mod G) as long as a lane is done with one block before its next begins,
+// 2r + 8 <= 9G: G = 16 up to radius 68 (two couples of pairs in a warp), G = 32 up to
+// 140.  No pass boundary goes through memory, a pair takes 9 m / 8 + 2r steps and
+// nothing waits for the end of a pass.  Outside its window a lane's masks are
+// empty, so its outputs are the out-of-band ones (H = 0, F = -infinity), which is
+// also what the first block sees above it.  A lane's own byte and profile loads run
+// two steps and one step ahead.  The recurrence is the literal one: opening both
+// gaps from the match state (as the tile classes do) would move a gap pair across
+// the band's edge.
+//
+// What bounds it is a step's latency (about 160 instructions on one or two warps a
+// scheduler).  5,000 pairs of the long mix (4,600 of them banded, radius 64):
+// 1.80 ms with whole-warp passes, 0.66 ms so (both alone, cold).
+constexpr int kRingLag = 9;  // steps between a row block and the next
+__host__ __device__ constexpr int band_ring_radius(int G) { return (kRingLag * G - 8) / 2; }
+
+// Byte masks of a lane's eight rows at local column u of a half: rows u - 2r .. u, none outside the target or past
+// the query's row blocks.
+__device__ __forceinline__ uint2 ring_mask(int u, int col, int row0, int r2, int m, int n) {
+  const int lo = max(u - r2, 0), hi = min(u, 7);
+  const bool any = lo <= hi && static_cast<uint32_t>(col) < static_cast<uint32_t>(n) && row0 < m;
+  const uint32_t bits = any ? (0xFFu >> (7 - hi)) & (0xFFu << lo) : 0u;
+  return make_uint2(band16_bytes(bits & 0xFu), band16_bytes(bits >> 4));
+}
+
+template <int G>
+__device__ __forceinline__ void band16_ring(const Sw32Params& prm, uint32_t pA, uint32_t pB, int2* bnd) {
+  constexpr int R = kSw32R;
+  constexpr int T = kRingLag * G;  // steps between a lane's row blocks
+  const int lane = threadIdx.x & 31;
+  const int gl = lane % G;
+  const uint32_t FULL = 0xFFFFFFFFu;
+  bool emptyA, emptyB;
+  const Band16Half A = band16_half(prm, pA, &emptyA);
+  const Band16Half B = band16_half(prm, pB, &emptyB);
+  if (gl == 0) {  // a pair without band cells scores 0
+    if (emptyA) {
+      prm.scores[pA] = 0;
+      if (prm.kernels) prm.kernels[pA] = 1u;
+    }
+    if (emptyB) {
+      prm.scores[pB] = 0;
+      if (prm.kernels) prm.kernels[pB] = 1u;
+    }
+  }
+  // a band with cells has its center within the query's and target's lengths plus the radius
+  const int mA = A.on ? A.m : 0, mB = B.on ? B.m : 0;
+  const int r2A = A.on ? 2 * static_cast<int>(A.radius) : 0, r2B = B.on ? 2 * static_cast<int>(B.radius) : 0;
+  const int c0A = A.on ? static_cast<int>(A.center - A.radius) : 0;
+  const int c0B = B.on ? static_cast<int>(B.center - B.radius) : 0;
+  int steps = 0;
+  if (mA) steps = kRingLag * ((mA - 1) / R) + r2A + R;
+  if (mB) steps = max(steps, kRingLag * ((mB - 1) / R) + r2B + R);
+  steps = __reduce_max_sync(FULL, steps);
+  const uint32_t MOPEN = pk_splat(-prm.open);
+  const uint32_t MEXT = pk_splat(-prm.ext);
+  const uint32_t E0 = MOPEN, F0 = MOPEN;
+
+  uint32_t Hp[R], E[R];
+#pragma unroll
+  for (int k = 0; k < R; ++k) {
+    Hp[k] = 0;
+    E[k] = E0;
+  }
+  uint32_t best = 0, hup_prev = 0, h_bot = 0, f_out = F0;
+  const int src_lane = (lane & ~(G - 1)) | ((lane - 1) & (G - 1));
+  // this lane's position now, one and two steps ahead: local column and first row
+  int u0 = -kRingLag * gl, row0 = gl * R;
+  auto next = [&](int& u, int& row) {
+    if (++u == T) {
+      u = 0;
+      row += G * R;
+    }
+  };
+  auto byte_at = [&](const Band16Half& h, int c0, int u, int row) -> uint32_t {
+    const int col = row + c0 + u;
+    uint32_t v = kSentinel;
+    if (u >= 0 && row < h.m && static_cast<uint32_t>(col) < static_cast<uint32_t>(h.n)) v = __ldg(h.t + col);
+    return v;
+  };
+  int u1 = u0, row1 = row0;
+  next(u1, row1);
+  int u2 = u1, row2 = row1;
+  next(u2, row2);
+  uint32_t ra = byte_at(A, c0A, u0, row0), rb = byte_at(B, c0B, u0, row0);
+  uint2 sa = band16_scores(A, ra, row0), sb = band16_scores(B, rb, row0);
+  ra = byte_at(A, c0A, u1, row1);  // the residues of the next step
+  rb = byte_at(B, c0B, u1, row1);
+
+  for (int s = 0; s < steps; ++s) {
+    const uint32_t hin = __shfl_sync(FULL, h_bot, src_lane);
+    const uint32_t fin = __shfl_sync(FULL, f_out, src_lane);
+    const uint2 san = band16_scores(A, ra, row1);
+    const uint2 sbn = band16_scores(B, rb, row1);
+    ra = byte_at(A, c0A, u2, row2);
+    rb = byte_at(B, c0B, u2, row2);
+    if (u0 == 0) {  // left of the band: H = 0, E = -infinity
+#pragma unroll
+      for (int k = 0; k < R; ++k) {
+        Hp[k] = 0;
+        E[k] = E0;
+      }
+    }
+    const uint2 ma = ring_mask(u0, row0 + c0A + u0, row0, r2A, mA, A.n);
+    const uint2 mb = ring_mask(u0, row0 + c0B + u0, row0, r2B, mB, B.n);
+    const uint32_t wa[2] = {sa.x, sa.y}, wb[2] = {sb.x, sb.y};
+    uint32_t hd = hup_prev;
+    uint32_t F = fin;
+#pragma unroll
+    for (int k = 0; k < R; ++k) {
+      const uint32_t S = prmt(wa[k >> 2], wb[k >> 2], sel_pair(k & 3));
+      const uint32_t M = prmt(k < 4 ? ma.x : ma.y, k < 4 ? mb.x : mb.y,
+                              static_cast<uint32_t>((k & 3) | ((k & 3) << 4) | ((4 + (k & 3)) << 8) |
+                                                    ((4 + (k & 3)) << 12)));
+      const uint32_t t = pk_addmax(hd, S, E[k]);
+      const uint32_t H = pk_max_relu(t, F) & M;  // out of the band: H = 0
+      best = pk_max(best, H);
+      const uint32_t Ho = pk_add(H, MOPEN);
+      E[k] = (pk_addmax(E[k], MEXT, Ho) & M) | (E0 & ~M);
+      F = (pk_addmax(F, MEXT, Ho) & M) | (F0 & ~M);
+      hd = Hp[k];
+      Hp[k] = H;
+    }
+    hup_prev = hin;
+    h_bot = Hp[R - 1];
+    f_out = F;
+    u0 = u1;
+    row0 = row1;
+    u1 = u2;
+    row1 = row2;
+    next(u2, row2);
+    sa = san;
+    sb = sbn;
+  }
+#pragma unroll
+  for (int o = G / 2; o > 0; o >>= 1) best = pk_max(best, __shfl_xor_sync(FULL, best, o));
+  const int32_t bA = pk_lo(best), bB = pk_hi(best);
+  const bool overA = A.on && bA > A.thresh, overB = B.on && bB > B.thresh;
+  if (gl == 0) {
+    if (A.on && !overA) {
+      prm.scores[pA] = bA;
+      if (prm.kernels) prm.kernels[pA] = 1u;
+    }
+    if (B.on && !overB) {
+      prm.scores[pB] = bB;
+      if (prm.kernels) prm.kernels[pB] = 1u;
+    }
+  }
+  // past the headroom: rescored exactly by the 32-bit code, the whole warp on one pair after the other
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    uint32_t over = __ballot_sync(FULL, gl == 0 && (h ? overB : overA));
+    while (over) {
+      const int src = __ffs(over) - 1;
+      over &= over - 1;
+      sw32_pair<kSw32Score>(prm, __shfl_sync(FULL, h ? pB : pA, src), bnd);
+    }
+  }
+}
+
+// Warps claim four entries of the list at a time; the widest band among them says how they are scored.
 template <int WARPS>
 __global__ void __launch_bounds__(WARPS * 32) sw16_band_kernel(const Sw32Params prm) {
   const int warp = threadIdx.x >> 5;
@@ -355,15 +524,37 @@ __global__ void __launch_bounds__(WARPS * 32) sw16_band_kernel(const Sw32Params 
   const uint32_t n = prm.n_static;
   for (;;) {
     uint32_t w = 0;
-    if (lane == 0) w = atomicAdd(prm.work_counter, 2u);
+    if (lane == 0) w = atomicAdd(prm.work_counter, 4u);
     w = __shfl_sync(0xFFFFFFFFu, w, 0);
     if (w >= n) break;
-    const uint32_t a = prm.list[w];
-    const uint32_t b = w + 1 < n ? prm.list[w + 1] : kBandNone;
-    const uint32_t pA = band16_takes(prm, a) ? a : kBandNone;
-    const uint32_t pB = (b != kBandNone && band16_takes(prm, b)) ? b : kBandNone;
-    if (pA == kBandNone && pB == kBandNone) continue;
-    band16_couple(prm, pA, pB, bnd);
+    uint32_t p[4];
+    int32_t widest = -1;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      p[k] = kBandNone;
+      if (w + k < n) {
+        const uint32_t e = prm.list[w + k];
+        if (band16_takes(prm, e)) {
+          p[k] = e;
+          widest = max(widest, prm.pair_radius[e]);
+        }
+      }
+    }
+    if (widest < 0) continue;
+    if (widest <= band_ring_radius(16)) {
+      const bool upper = lane >= 16;
+      band16_ring<16>(prm, upper ? p[2] : p[0], upper ? p[3] : p[1], bnd);
+    } else {
+#pragma unroll 1
+      for (int k = 0; k < 4; k += 2) {
+        const uint32_t a = k ? p[2] : p[0], b = k ? p[3] : p[1];
+        if (a == kBandNone && b == kBandNone) continue;
+        if (widest <= band_ring_radius(32))
+          band16_ring<32>(prm, a, b, bnd);
+        else
+          band16_couple(prm, a, b, bnd);
+      }
+    }
   }
 }
 

@@ -23,6 +23,7 @@
 #include <cstdint>
 
 #include "../../include/sabertooth_b200.h"
+#include "st_band16.cuh"
 #include "st_common.cuh"
 #include "st_sw16.cuh"
 #include "st_tuning.h"
@@ -178,17 +179,21 @@ __global__ void __launch_bounds__(256) dp_classify_kernel(const DpIn in, const D
 }
 
 // ---- 32-bit list order: longest first by the steps a warp spends on a pair ----
-// passes x (streamed columns + ramp); a banded pair streams one 256-row pass's band window per pass.  The
-// key is inverted so that an ascending sort puts the costliest first.
+// passes x (streamed columns + ramp); a wide band streams one 256-row pass's window per pass, a narrow one follows
+// its diagonal.  The key is inverted so that an ascending sort puts the costliest first.
 __global__ void __launch_bounds__(256) dp_list_keys_kernel(const DpIn in, const DpWork w, uint32_t n_list,
                                                             unsigned long long* keys, uint32_t* vals) {
   for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < n_list; k += gridDim.x * blockDim.x) {
     const uint32_t i = w.list32[k];
     const unsigned long long m = in.prof.qlen[w.pq[i]], tl = in.db.length[w.pt[i]];
     const unsigned long long P = (m + 255) / 256;
-    unsigned long long wc = tl;
-    if (w.pr[i] >= 0) wc = min(tl, 256ull + 2ull * static_cast<unsigned long long>(w.pr[i]));
-    const unsigned long long cost = min(P * (wc + 31), (1ull << 48) - 1);
+    const int32_t r = w.pr[i];
+    unsigned long long cost = P * (tl + 31);
+    if (r >= 0 && r <= band_ring_radius(32))
+      cost = kRingLag * (m / kSw32R) + 2ull * r;
+    else if (r >= 0)
+      cost = P * (min(tl, 256ull + 2ull * static_cast<unsigned long long>(r)) + 31);
+    cost = min(cost, (1ull << 48) - 1);
     keys[k] = ((1ull << 48) - 1) - cost;
     vals[k] = i;
   }

@@ -1487,7 +1487,8 @@ static int plan_build(st_ctx* c, const st_pair* pairs, uint64_t n, int32_t open,
     }
   }
   // The 32-bit list longest first (its kernels pull entries in order), by the steps a warp spends on a pair:
-  // passes x (streamed columns + ramp), a banded pair streaming one 256-row pass's band window per pass.
+  // passes x (streamed columns + ramp), a wide band streaming one 256-row pass's window per pass, a narrow one
+  // following its diagonal.
   // The packed band kernel scores neighbouring entries together, so similar pairs share a warp.
   if (list32.size() > 1) {
     std::vector<std::pair<uint64_t, uint32_t>> ord(list32.size());
@@ -1496,9 +1497,12 @@ static int plan_build(st_ctx* c, const st_pair* pairs, uint64_t n, int32_t open,
       const uint32_t i = list32[k];
       const uint64_t m = c->profs[pq[i]].m, tl = tlen[i];
       const uint64_t P = (m + kSw32Rows - 1) / kSw32Rows;
-      uint64_t w = tl;
-      if (pr[i] >= 0) w = std::min<uint64_t>(tl, static_cast<uint64_t>(kSw32Rows) + 2 * static_cast<uint64_t>(pr[i]));
-      ord[k] = {P * (w + 31), i};
+      uint64_t cost = P * (tl + 31);
+      if (pr[i] >= 0 && pr[i] <= band_ring_radius(32))
+        cost = kRingLag * (m / kSw32R) + 2 * static_cast<uint64_t>(pr[i]);
+      else if (pr[i] >= 0)
+        cost = P * (std::min<uint64_t>(tl, static_cast<uint64_t>(kSw32Rows) + 2 * static_cast<uint64_t>(pr[i])) + 31);
+      ord[k] = {cost, i};
     }
     std::stable_sort(ord.begin(), ord.end(), [](const std::pair<uint64_t, uint32_t>& a,
                                                  const std::pair<uint64_t, uint32_t>& b) { return a.first > b.first; });
