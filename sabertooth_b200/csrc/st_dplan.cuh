@@ -35,6 +35,7 @@ constexpr uint32_t kDpNoClass = 63;  // sort key of a query with no 16-bit pairs
 
 struct DpClass {
   uint32_t G, R, C, W;
+  uint32_t team;      // a CTA's warps share each warp task's passes
   uint32_t rows;      // G * R
   uint32_t S;         // targets per warp task, 64 / G
   uint32_t max_mpad;  // the largest staged row count that fits the class's shared memory
@@ -230,6 +231,7 @@ __global__ void __launch_bounds__(256) dp_estimate_kernel(const DpIn in, const D
       unsigned long long cols = 0;
       for (uint32_t x = lane; x < nw; x += 32) cols += max(sh.minc, dp_up4(tl(x * c.S)));
       cols = dp_warp_sum(cols);
+      if (c.team) cols += static_cast<unsigned long long>(nw) * tune_team_cols(c.G, c.C, sh.P, c.W);
       v = static_cast<double>(cols) * c.S * sh.mpad;
       v = c.rate > 0.0f ? v / c.rate : v * 1e150;
     }
@@ -273,7 +275,7 @@ __global__ void __launch_bounds__(256) dp_pick_kernel(const DpIn in, const DpWor
     if (lane < cls.n && est[lane] < 1e300) {
       const DpClass& c = cls.c[lane];
       const DpShape sh = dp_shape(c, m);
-      v = tune_objective(est[lane], tune_crit_ps(c.G, c.R, c.C, sh.P, max(sh.minc, dp_up4(tl(0)))),
+      v = tune_objective(est[lane], tune_crit_ps(c.G, c.R, c.C, sh.P, max(sh.minc, dp_up4(tl(0))), c.team ? c.W : 1u),
                          static_cast<double>(w.totals->batch_ps));
     }
     int k = lane;
@@ -309,8 +311,8 @@ __global__ void __launch_bounds__(256) dp_pick_kernel(const DpIn in, const DpWor
   }
 }
 
-// CTA tasks of one query, by one warp: consecutive warp tasks in units of tune_cta_unit; a task ends at 128 warp
-// tasks or where the query's running cost passes a multiple of the class's cap (its cost over two CTAs on every
+// CTA tasks of one query, by one warp: consecutive warp tasks in units of tune_cta_unit (a team class: one each); a
+// task ends at 128 warp tasks or where the query's running cost passes a multiple of the class's cap (its cost over two CTAs on every
 // SM).  f(t, w0, w1, cost) is called once for each task t by some lane; returns the number of tasks.
 template <class F>
 __device__ __forceinline__ uint32_t dp_for_each_cta(const DpClasses& cls, const DpTotals* tot, uint32_t k,
@@ -319,7 +321,7 @@ __device__ __forceinline__ uint32_t dp_for_each_cta(const DpClasses& cls, const 
   const int lane = threadIdx.x & 31;
   unsigned long long wt_total = lane < cls.n ? tot->n_wt[lane] : 0u;
   wt_total = dp_warp_sum(wt_total);
-  const uint32_t unit = tune_cta_unit(wt_total, cls.sms, c.W);
+  const uint32_t unit = c.team ? 1u : tune_cta_unit(wt_total, cls.sms, c.W);
   const unsigned long long cap = max(1ull, tot->cost[k] / (2ull * cls.sms));
   unsigned long long base = 0;         // cost of the warp tasks before this round's
   unsigned long long last_bucket = 0;  // of the last unit of the round before
@@ -338,7 +340,7 @@ __device__ __forceinline__ uint32_t dp_for_each_cta(const DpClasses& cls, const 
     const unsigned long long bucket = excl / cap;
     unsigned long long before = __shfl_up_sync(0xFFFFFFFFu, bucket, unit);
     if (lane < static_cast<int>(unit)) before = last_bucket;
-    const bool begin = x < nw && x % unit == 0 && (x == 0 || bucket != before || x % 128u == 0);
+    const bool begin = x < nw && x % unit == 0 && (x == 0 || bucket != before || x % 128u == 0 || c.team);
     const uint32_t mask = __ballot_sync(0xFFFFFFFFu, begin);
     const uint32_t lower = mask & ((1u << lane) - 1u);
     // the task before mine: begun by the next lower lane of the ballot, or the open one

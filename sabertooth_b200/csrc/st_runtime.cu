@@ -239,10 +239,12 @@ using Sw16Fn = void (*)(const Sw16Params);
 struct Sw16Class {
   int G, R, C, W;  // lanes per alignment, rows per lane, columns per step, warps per CTA
   Sw16Fn fn;
+  bool team = false;  // a CTA's warps share each warp task's passes
 };
 
 #define ST_CLASS(g, r, c) {g, r, c, kWarps16, sw16_kernel<g, r, c, kWarps16>}
 #define ST_CLASS_W(g, r, c, w) {g, r, c, w, sw16_kernel<g, r, c, w>}
+#define ST_TEAM(g, r, c) {g, r, c, kWarps16, sw16_kernel<g, r, c, kWarps16, kSw16Score, true>, true}
 static const Sw16Class kClasses[] = {
     ST_CLASS(4, 8, 4),   ST_CLASS(8, 8, 4),   ST_CLASS(16, 8, 4),  ST_CLASS(32, 8, 4),
     ST_CLASS(4, 12, 4),  ST_CLASS(8, 12, 4),  ST_CLASS(16, 12, 4), ST_CLASS(32, 12, 4),
@@ -251,10 +253,11 @@ static const Sw16Class kClasses[] = {
     ST_CLASS(4, 24, 4),  ST_CLASS(8, 24, 4),  ST_CLASS(16, 24, 4), ST_CLASS(32, 24, 4),
     ST_CLASS_W(4, 28, 4, 4), ST_CLASS_W(8, 28, 4, 4), ST_CLASS_W(16, 28, 4, 4),
     ST_CLASS_W(4, 32, 4, 4), ST_CLASS_W(8, 32, 4, 4), ST_CLASS_W(16, 32, 4, 4),
-    ST_CLASS(32, 16, 2), ST_CLASS_W(32, 32, 4, 4),
+    ST_CLASS(32, 16, 2), ST_CLASS_W(32, 32, 4, 4), ST_TEAM(32, 8, 4),
 };
 #undef ST_CLASS
 #undef ST_CLASS_W
+#undef ST_TEAM
 constexpr int kNumClasses = sizeof(kClasses) / sizeof(kClasses[0]);
 
 // The tile classes built for end cells too: 64 to 512 rows a pass, so that every query length has a class that
@@ -267,7 +270,7 @@ struct Sw16EndFns {
 static const Sw16EndFns kEndFns[] = {ST_END(8, 8), ST_END(32, 8), ST_END(8, 16), ST_END(16, 16), ST_END(32, 16)};
 #undef ST_END
 static const Sw16EndFns* end_fns(int cls) {
-  if (kClasses[cls].C != 4) return nullptr;
+  if (kClasses[cls].C != 4 || kClasses[cls].team) return nullptr;
   for (const auto& f : kEndFns)
     if (f.G == kClasses[cls].G && f.R == kClasses[cls].R) return &f;
   return nullptr;
@@ -277,6 +280,8 @@ constexpr uint32_t kEndMaxLen = 65535;  // an end cell's column travels in 16 bi
 static_assert(kNumClasses <= kMaxTileClasses, "tile classes exceed the tuning arrays");
 
 int st_tuning_num_classes() { return kNumClasses; }
+bool st_tuning_class_team(int c) { return kClasses[c].team; }
+int st_tuning_class_warps(int c) { return kClasses[c].W; }
 void st_tuning_class_shape(int c, int* G, int* R, int* C) {
   *G = kClasses[c].G;
   *R = kClasses[c].R;
@@ -1608,7 +1613,9 @@ static int plan_build(st_ctx* c, const st_pair* pairs, uint64_t n, int32_t open,
     for (uint32_t w = 0; w < e.n_wt; ++w) {
       const uint32_t nc = wt_cols(k, sh, w);
       e.cost += wt_cost(sh, nc);
-      e.streamed += static_cast<uint64_t>(sh.P) * sh.rows * nc * sh.S;
+      const Sw16Class& kc = kClasses[qclass[k]];
+      e.streamed += static_cast<uint64_t>(sh.P) * sh.rows * sh.S *
+                    (nc + (kc.team ? tune_team_cols(kc.G, kc.C, sh.P, kc.W) : 0u));
     }
   }
   std::vector<uint64_t> cap(kNumClasses, 0);
@@ -1620,13 +1627,14 @@ static int plan_build(st_ctx* c, const st_pair* pairs, uint64_t n, int32_t open,
   auto for_each_cta = [&](int64_t k, const QShape& sh, auto&& f) {
     const uint32_t n_wt = qe[k].n_wt;
     const uint64_t cp = cap[qclass[k]];
-    const uint32_t unit = tune_cta_unit(wt_total, c->sms, kClasses[qclass[k]].W);
+    const Sw16Class& kc = kClasses[qclass[k]];
+    const uint32_t unit = kc.team ? 1u : tune_cta_unit(wt_total, c->sms, kc.W);
     uint32_t w0 = 0;
     uint64_t acc = 0, start = 0, bucket = 0;
     for (uint32_t w = 0; w < n_wt; ++w) {
       if (w % unit == 0) {
         const uint64_t bk = acc / cp;
-        if (w > 0 && (bk != bucket || w % kMaxWtPerCta == 0)) {
+        if (w > 0 && (bk != bucket || w % kMaxWtPerCta == 0 || kc.team)) {
           f(w0, w, acc - start);
           w0 = w;
           start = acc;
@@ -2106,6 +2114,7 @@ static int dplan_build(st_ctx* c, const st_pair* pairs, uint64_t n, int32_t open
     d.R = kClasses[k].R;
     d.C = kClasses[k].C;
     d.W = kClasses[k].W;
+    d.team = kClasses[k].team ? 1u : 0u;
     d.rows = d.G * d.R;
     d.S = 64 / d.G;
     const uint32_t smem = static_cast<uint32_t>(std::min<int>(g_class_smem[k], 216 * 1024));

@@ -43,6 +43,13 @@
 // pipe instead of prmt measured no faster (6.3 against 6.4 T cells/s in a bare cell
 // loop: the third register operand of both pipes' instructions is what limits then).
 //
+// Teams.  In the team form a CTA's warps share one warp task and run its passes
+// side by side: warp w takes passes w, w + 8, ..., each some 36 steps behind the pass
+// above it, whose feeder publishes the columns of its boundary line in a counter.
+// It is for batches that a query of many rows would otherwise keep waiting: the
+// wavefront of 2,000 rows x 900 columns is 510 steps of 32 x 8 rows instead of 480 of
+// 32 x 32 (938 against 1,932 cycles each) or 1,830 of 32 x 8.
+//
 // End cells.  In the end modes a column's maximum is compared with a threshold
 // before anything else is done: the best score seen by this lane or by the lanes
 // above it (their g travels with the columns), less one, as an equal score may
@@ -122,6 +129,7 @@ constexpr uint32_t kCtlLast = 1u << 27;   // last step of the task
 constexpr uint32_t kCtlFirst = 1u << 28;  // first step of a pass
 constexpr uint32_t kCtlMore = 1u << 29;   // a pass that is not the last: its bottom row is kept
 constexpr int kSlotRing = 8;
+constexpr uint32_t kTeamSpins = 1u << 22;  // polls of a producer's count before a team gives its pair up
 
 template <int G, int R, int C>
 struct Sw16Tile {
@@ -277,7 +285,7 @@ __device__ __forceinline__ uint32_t rows_from(int nz, int v) {
 // single classes on the 1.2 M-pair PSSM batch, before -> after: <8,24> 5.41 -> 5.77 T,
 // <16,24> 5.40 -> 5.76, <16,32> 5.13 -> 5.62, <8,16> 4.96 -> 5.33, <8,12> 4.82 -> 5.17; a lone
 // warp's step <8,24> 1,756 -> 1,541 cycles, <8,8> 1,050 -> 771.
-template <int G, int R, int C, int WARPS, int MODE = kSw16Score>
+template <int G, int R, int C, int WARPS, int MODE = kSw16Score, bool TEAM = false>
 __global__ void __launch_bounds__(WARPS * 32, WARPS == 4 || (R == 8 && MODE == kSw16Score) ? 3 : 2)
     sw16_kernel(const Sw16Params prm) {
   using Tile = Sw16Tile<G, R, C>;
@@ -293,10 +301,16 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 4 || (R == 8 && MODE == k
   __shared__ unsigned long long s_end[kEnds ? WARPS : 1][kEnds ? NG : 1][kSlotRing][2];
   __shared__ int2 s_rev[MODE == kSw16RevEnd ? WARPS : 1][MODE == kSw16RevEnd ? NG : 1][kSlotRing][2];
 
+  // team form: a column count per warp, that of the boundary columns it has published; and whether a wait ran out
+  __shared__ volatile uint32_t s_prog[TEAM ? WARPS : 1];
+  __shared__ volatile uint32_t s_fail;
+  static_assert(!TEAM || (G == 32 && MODE == kSw16Score), "a team's warps are whole groups");
+
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
   const int gl = lane % G;
   const int grp = lane / G;
+  const int own = TEAM ? 0 : warp;  // whose slots this warp's tasks use
   uint2* bnd = prm.scratch + static_cast<size_t>((blockIdx.x * WARPS + warp) * NG + grp) * prm.scratch_stride;
   const uint32_t MOPEN = pk_splat(-prm.open);
   const uint32_t MEXT = pk_splat(-min(prm.ext, prm.open));
@@ -334,6 +348,14 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 4 || (R == 8 && MODE == k
       }
     }
     if (threadIdx.x == 0) s_next = task.wt_begin;
+    if constexpr (TEAM) {
+      if (threadIdx.x < WARPS) s_prog[threadIdx.x] = 0;
+      if (threadIdx.x == 0) {
+        s_fail = 0;
+        s_best[0][0][0][0] = 0;
+        s_best[0][0][0][1] = 0;
+      }
+    }
     const int32_t thresh = 32767 - prm.prof.max_score[q];
     __syncthreads();
 
@@ -350,12 +372,10 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 4 || (R == 8 && MODE == k
       if (lane == 0) w = atomicAdd(&s_next, 1u);
       return __shfl_sync(FULL, w, 0);
     };
-    uint32_t w_cur = claim();
-    bool have = w_cur < task.wt_end;
-    if (!have) {
-      __syncthreads();
-      continue;
-    }
+    // a team's warps share the CTA task's one warp task: warp w takes its passes w, w + WARPS, ...
+    uint32_t w_cur = TEAM ? task.wt_begin : claim();
+    bool have = TEAM ? warp < P : w_cur < task.wt_end;
+    if (have) {
     auto load_pairs = [&](uint32_t slot_begin) {
       Sw16Pair2 r = load_pair2(prm, slot_begin, grp);
       if constexpr (MODE == kSw16RevEnd) {
@@ -370,8 +390,8 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 4 || (R == 8 && MODE == k
     };
     // a task enters the ring (the group's feeder)
     auto open_slot = [&](int slot, const Sw16Pair2& r) {
-      s_pair[warp][grp][slot][0] = r.pA;
-      s_pair[warp][grp][slot][1] = r.pB;
+      s_pair[own][grp][slot][0] = r.pA;
+      s_pair[own][grp][slot][1] = r.pB;
       if constexpr (kEnds) {
         s_end[warp][grp][slot][0] = 0;
         s_end[warp][grp][slot][1] = 0;
@@ -380,27 +400,28 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 4 || (R == 8 && MODE == k
           s_rev[warp][grp][slot][1] = make_int2(r.sB, static_cast<int>(r.offB));
         }
       } else {
-        s_best[warp][grp][slot][0] = 0;
-        s_best[warp][grp][slot][1] = 0;
+        s_best[own][grp][slot][0] = 0;
+        s_best[own][grp][slot][1] = 0;
       }
     };
     Sw16WarpTask wt_cur = prm.warp_tasks[w_cur];
     Sw16Pair2 cur{};
     if (feeder) cur = load_pairs(wt_cur.slot_begin);
-    uint32_t w_nxt = claim();
+    uint32_t w_nxt = TEAM ? task.wt_end : claim();
     bool have_nxt = w_nxt < task.wt_end;
     Sw16WarpTask wt_nxt = have_nxt ? prm.warp_tasks[w_nxt] : Sw16WarpTask{0, 0};
     Sw16Pair2 nxt{};
     if (have_nxt && feeder) nxt = load_pairs(wt_nxt.slot_begin);
-    if (feeder) open_slot(0, cur);
+    if (!TEAM && feeder) open_slot(0, cur);
     // Lane 0's position: column u_col of pass u_pass of task u_seq.  The control word of an ordinary step is
     // u_ctl; the first and the last step of a pass add their events, so an ordinary step takes no decisions
     // beyond one vote (is any lane at an event, or lane 0 within a step of its pass's end).
-    int u_col = 0, u_pass = 0, u_seq = 0;
-    bool done = false;
+    constexpr int kPassStep = TEAM ? WARPS : 1;
+    int u_col = 0, u_pass = TEAM ? warp : 0, u_seq = 0;
+    bool done = false, gap = false;
     int u_end = static_cast<int>(wt_cur.ncols);  // columns of the pass; of the idle steps at the end of the stream
-    uint32_t u_ctl = P > 1 ? kCtlMore : 0u;
-    uint32_t u_last = P > 1 ? 0u : kCtlLast;     // the event of the pass's last step
+    uint32_t u_ctl = u_pass + 1 < P ? kCtlMore : 0u;
+    uint32_t u_last = u_pass + kPassStep < P ? 0u : kCtlLast;  // the event of the pass's last step
 
     // per-lane wavefront state
     uint32_t Hp[R], E[R];
@@ -431,9 +452,27 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 4 || (R == 8 && MODE == k
       my_f[j] = F0;
     }
     // lane 0's first step: column 0, pass 0 of the first task
-    if (feeder) my_ctl = kCtlFirst | u_ctl;
+    if (feeder) my_ctl = kCtlFirst | u_ctl | (static_cast<uint32_t>(u_pass) << 16);
     my_rA = load_step(cur.tA, cur.lenA, 0);
     my_rB = load_step(cur.tB, cur.lenB, 0);
+    // Team form: the boundary of the next step comes from the warp that runs the pass above, once it has published
+    // the columns.  The wait is bounded; when it runs out the pair goes to the exact 32-bit kernel instead.
+    const uint32_t team_cols = wt_cur.ncols;
+    uint32_t seen = 0;     // columns of the producer known to be published
+    uint32_t my_base = 0;  // this lane's columns published in earlier passes
+    auto team_load = [&]() {
+      const int from = (u_pass - 1) % WARPS;
+      const uint32_t need = static_cast<uint32_t>((u_pass - 1) / WARPS) * team_cols + u_col + C;
+      if (seen < need) {
+        for (uint32_t spin = 0; (seen = s_prog[from]) < need && s_fail == 0; ++spin)
+          if (spin >= kTeamSpins) s_fail = 1;
+        __threadfence_block();
+      }
+      load_bnd<C>(true, prm.scratch + static_cast<size_t>(blockIdx.x * WARPS + from) * prm.scratch_stride + u_col,
+                  my_h, my_f);
+    };
+    if constexpr (TEAM)
+      if (feeder && u_pass > 0) team_load();
     __syncwarp();
 
     for (;;) {
@@ -461,32 +500,39 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 4 || (R == 8 && MODE == k
           n_ctl = kCtlFirst;
           if (!have) {  // the idle steps are over
             done = true;
-          } else if (++u_pass == P) {  // task done: the pre-claimed task becomes current, claim the one after
-            u_pass = 0;
-            ++u_seq;
-            have = have_nxt;
-            wt_cur = wt_nxt;
-            cur = nxt;
-            if (have) {
-              if (feeder) open_slot(u_seq & (kSlotRing - 1), cur);
-              w_nxt = claim();
-              have_nxt = w_nxt < task.wt_end;
-              if (have_nxt) {
-                wt_nxt = prm.warp_tasks[w_nxt];
-                if (feeder) nxt = load_pairs(wt_nxt.slot_begin);
+          } else if (TEAM && !gap && u_pass + kPassStep < P) {
+            gap = true;  // a team's warp finishes and publishes a pass before it may have to wait for its next one
+          } else {
+            gap = false;
+            u_pass += kPassStep;
+            if (u_pass >= P) {  // task done: the pre-claimed task becomes current, claim the one after
+              u_pass = 0;
+              ++u_seq;
+              have = have_nxt;
+              wt_cur = wt_nxt;
+              cur = nxt;
+              if (have) {
+                if (feeder) open_slot(u_seq & (kSlotRing - 1), cur);
+                w_nxt = claim();
+                have_nxt = w_nxt < task.wt_end;
+                if (have_nxt) {
+                  wt_nxt = prm.warp_tasks[w_nxt];
+                  if (feeder) nxt = load_pairs(wt_nxt.slot_begin);
+                }
+                u_end = static_cast<int>(wt_cur.ncols);
               }
-              u_end = static_cast<int>(wt_cur.ncols);
             }
           }
           u_col = 0;
-          if (have) {
+          if (have && !gap) {
+            if constexpr (TEAM) u_end = static_cast<int>(team_cols);
             const uint32_t at = (static_cast<uint32_t>(u_pass) << 16) |
                                 (static_cast<uint32_t>(u_seq & (kSlotRing - 1)) << 24);
             u_ctl = u_pass + 1 < P ? kCtlMore : 0u;
-            u_last = u_pass + 1 < P ? 0u : kCtlLast | at;
+            u_last = u_pass + kPassStep < P ? 0u : kCtlLast | at;
             n_ctl |= u_ctl | at;
           } else {  // idle steps until the last lane has finished
-            cur.lenA = cur.lenB = 0;
+            if (!TEAM) cur.lenA = cur.lenB = 0;
             u_ctl = u_last = n_ctl = 0u;
             u_end = (G - 1) * C;
           }
@@ -503,6 +549,7 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 4 || (R == 8 && MODE == k
           hup_prev = 0;
           my_col = 0;
           row0 = ((ctl >> 16) & 0xFFu) * (G * R) + gl * R;
+          if constexpr (TEAM) my_base = ((ctl >> 16) & 0xFFu) / WARPS * team_cols;
           if constexpr (kEnds) {
             const bool begin = (ctl & 0x00FF0000u) == 0;  // the task's first pass
             if (begin) {
@@ -530,8 +577,9 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 4 || (R == 8 && MODE == k
         __syncwarp();
       }
       // the feeder's residues, on their way while this step is computed
-      const uint32_t nA = load_step(cur.tA, cur.lenA, u_col);
-      const uint32_t nB = load_step(cur.tB, cur.lenB, u_col);
+      const bool idle = TEAM && (gap || !have);
+      const uint32_t nA = load_step(cur.tA, idle ? 0u : cur.lenA, u_col);
+      const uint32_t nB = load_step(cur.tB, idle ? 0u : cur.lenB, u_col);
       if constexpr (MODE == kSw16End) {
         if (gl != 0) g = pk_max(g, g_in);
         thr = pk_max(thr, pk_add(g, 0xFFFFFFFFu));  // g - 1: an equal score may come first by its column
@@ -614,7 +662,7 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 4 || (R == 8 && MODE == k
           if (feeder) {  // the group's last lane finishes the task last
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
-              const uint32_t p = s_pair[warp][grp][slot][h];
+              const uint32_t p = s_pair[own][grp][slot][h];
               if (p == kNoPair) continue;
               const unsigned long long x = e[h];
               const int32_t sc = static_cast<int32_t>(x >> 32);
@@ -637,12 +685,12 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 4 || (R == 8 && MODE == k
         }
       } else if (event && (ctl & kCtlLast)) {  // this lane's part of the task is done: fold its maximum into the task slot
         const int slot = static_cast<int>((ctl >> 24) & 7u);
-        atomicMax(&s_best[warp][grp][slot][0], pk_lo(best));
-        atomicMax(&s_best[warp][grp][slot][1], pk_hi(best));
+        atomicMax(&s_best[own][grp][slot][0], pk_lo(best));
+        atomicMax(&s_best[own][grp][slot][1], pk_hi(best));
         best = 0;
-        if (feeder) {  // the group's last lane finishes the task last: report both scores
-          const int32_t bA = s_best[warp][grp][slot][0], bB = s_best[warp][grp][slot][1];
-          const uint32_t pA = s_pair[warp][grp][slot][0], pB = s_pair[warp][grp][slot][1];
+        if (!TEAM && feeder) {  // the group's last lane finishes the task last: report both scores
+          const int32_t bA = s_best[own][grp][slot][0], bB = s_best[own][grp][slot][1];
+          const uint32_t pA = s_pair[own][grp][slot][0], pB = s_pair[own][grp][slot][1];
           if (pA != kNoPair) {
             if (bA > thresh) {
               prm.ovf_pairs[atomicAdd(prm.ovf_count, 1u)] = pA;
@@ -664,6 +712,12 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 4 || (R == 8 && MODE == k
       // the bottom row of a pass that is not the last goes to the scratch line
       store_bnd<C>(feeder && (ctl & kCtlMore) != 0, bnd + my_col, my_h, my_f);
       my_col += C;
+      if constexpr (TEAM) {
+        if (feeder && (ctl & kCtlMore) && ((my_col & 15) == 0 || my_col == team_cols)) {
+          __threadfence_block();  // the columns before their count
+          s_prog[warp] = my_base + my_col;
+        }
+      }
       if (done) break;
       // the feeder's outgoing registers become lane 0's inputs for the next step; above the query's first row
       // H = 0 and the first-row F, else the previous pass's bottom row (which this lane stored)
@@ -677,9 +731,29 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 4 || (R == 8 && MODE == k
           my_f[j] = F0;
         }
       }
-      load_bnd<C>(feeder && u_pass > 0, bnd + u_col, my_h, my_f);
+      if constexpr (TEAM) {
+        if (feeder && have && !gap && u_pass > 0) team_load();
+      } else {
+        load_bnd<C>(feeder && u_pass > 0, bnd + u_col, my_h, my_f);
+      }
     }
+    }  // have
     __syncthreads();
+    if constexpr (TEAM) {
+      if (threadIdx.x < 2) {  // both targets of the team's task
+        const Sw16Slot sl = prm.slots[prm.warp_tasks[task.wt_begin].slot_begin + threadIdx.x];
+        const int32_t b = s_best[0][0][0][threadIdx.x];
+        if (sl.pair != kNoPair) {
+          if (b > thresh || s_fail != 0) {
+            prm.ovf_pairs[atomicAdd(prm.ovf_count, 1u)] = sl.pair;
+          } else {
+            prm.scores[sl.pair] = b;
+            if (prm.kernels) prm.kernels[sl.pair] = 1u;
+          }
+        }
+      }
+      __syncthreads();  // before the next task's state is set up
+    }
   }
 }
 

@@ -8,9 +8,8 @@
 // critical path exceeds the whole batch by.  A table entry per (query length,
 // mean target length) bin, set by the caller, forces a class for that bin.
 //
-// Single alignments (the per-call path) use a model of the wavefront: a task
-// streams P * ncols / C + G - 1 steps, each costing about R * C row updates
-// plus a fixed per-step overhead.
+// Single alignments (the per-call path) take the class of the shortest
+// critical path.
 #pragma once
 #include <algorithm>
 #include <cstdint>
@@ -27,12 +26,13 @@ constexpr int kMaxTileClasses = 32;
 
 struct Tuning {
   int table[kTuneMBins][kTuneNBins];  // class index, -1 = rate model
-  double step_overhead;               // per-step overhead in row-update units (single alignments)
   float rate[kMaxTileClasses];        // streamed cells per second / 1e12, per class; 0 = not used
 };
 
 int st_tuning_num_classes();
 void st_tuning_class_shape(int c, int* G, int* R, int* C);
+bool st_tuning_class_team(int c);
+int st_tuning_class_warps(int c);
 
 inline int tune_mbin(uint32_t m) {
   int b = 0;
@@ -57,7 +57,7 @@ inline int tune_nbin(uint32_t n) {
 // Rates measured on B200 (148 SMs, 1965 MHz), streamed cells per second / 1e12,
 // with every query of the PSSM workload (4,000 queries of 50-2,000 rows, 1.2 M
 // pairs, targets of 160 residues on average) forced into one class.
-inline float tuning_default_rate(int G, int R, int C) {
+inline float tuning_default_rate(int G, int R, int C, bool team) {
   if (C != 4) return 0.0f;
   static const struct {
     int G, R;
@@ -71,6 +71,7 @@ inline float tuning_default_rate(int G, int R, int C) {
       {4, 28, 5.305f}, {8, 28, 5.452f}, {16, 28, 5.471f}, {4, 32, 5.464f},
       {8, 32, 5.600f}, {16, 32, 5.615f}, {32, 32, 5.578f},
   };
+  if (team) return 4.334f;
   for (const auto& r : kRates)
     if (r.G == G && r.R == R) return r.rate;
   return 0.0f;
@@ -79,13 +80,19 @@ inline float tuning_default_rate(int G, int R, int C) {
 inline void tuning_defaults(Tuning* t) {
   for (int i = 0; i < kTuneMBins; ++i)
     for (int j = 0; j < kTuneNBins; ++j) t->table[i][j] = -1;
-  t->step_overhead = 8.0;
   for (int c = 0; c < kMaxTileClasses; ++c) t->rate[c] = 0.0f;
   for (int c = 0; c < st_tuning_num_classes() && c < kMaxTileClasses; ++c) {
     int G, R, C;
     st_tuning_class_shape(c, &G, &R, &C);
-    t->rate[c] = tuning_default_rate(G, R, C);
+    t->rate[c] = tuning_default_rate(G, R, C, st_tuning_class_team(c));
   }
+}
+
+// Columns that a team's task costs beside its longest target's: the lag of each further pass of a round, during
+// which the CTA waits in part (a pass starts G + 5 steps after the one above it).
+constexpr uint32_t kTeamLag = 5;
+TUNE_HD inline uint32_t tune_team_cols(uint32_t G, uint32_t C, uint32_t P, uint32_t W) {
+  return ((P < W ? P : W) - 1) * (G + kTeamLag) * C;
 }
 
 // Streamed cells of one query (m rows) in class c over its targets' lengths,
@@ -103,26 +110,36 @@ inline double tune_streamed(int c, uint32_t m, const uint32_t* tlen_desc, size_t
   if (P > 1) minc = std::max<uint32_t>(minc, (static_cast<uint32_t>(C * G) + 15) & ~15u);
   double cols = 0;
   for (size_t w = 0; w < n; w += S) cols += std::max<uint32_t>(minc, (tlen_desc[w] + 3) & ~3u);
+  if (st_tuning_class_team(c)) cols += static_cast<double>((n + S - 1) / S) * tune_team_cols(G, C, P, st_tuning_class_warps(c));
   return cols * S * P * rows;
 }
 
 // Critical path: the time of the wavefront that streams a query's longest target, alone on its scheduler, in
 // picoseconds.  A step of a lone warp takes about 400 cycles (the shuffles, the profile loads, the dependent
 // rows; 560 with 4 or 32 lanes) plus 11.8 for each of its R*C cell pairs; measured at 1,965 MHz on 4,000-column
-// targets: <8,8> 771 cycles, <32,8> 938, <16,16> 1,182, <8,24> 1,541, <32,24> 1,570, <32,32> 1,932.
-TUNE_HD inline double tune_crit_ps(uint32_t G, uint32_t R, uint32_t C, uint32_t P, uint32_t ncols) {
+// targets: <8,8> 771 cycles, <32,8> 938, <16,16> 1,182, <8,24> 1,541, <32,24> 1,570, <32,32> 1,932.  With a team of
+// warps a pass starts G + 5 steps after the one above it, in rounds of `team` passes.
+TUNE_HD inline double tune_crit_ps(uint32_t G, uint32_t R, uint32_t C, uint32_t P, uint32_t ncols, uint32_t team) {
   const double fixed = G == 8 || G == 16 || C == 2 ? 400.0 : 560.0;
-  return (static_cast<double>(P) * (ncols / C) + G) * (fixed + 11.8 * (R * C)) * (1e6 / 1965.0);
+  double steps = static_cast<double>(P) * (ncols / C);
+  if (team > 1) {
+    const uint32_t lag = G + kTeamLag, pass = ncols / C + G, round = pass > team * lag ? pass : team * lag;
+    steps = static_cast<double>((P - 1) / team) * round + (P - 1) % team * lag + pass;
+  }
+  return (steps + G) * (fixed + 11.8 * (R * C)) * (1e6 / 1965.0);
 }
 
-// What a query costs the batch in a class: the chip's time for its cells, plus what its critical path adds when
-// that is longer than the whole batch (batch_ps: the batch's time with every query in its cheapest class).  Large
-// batches are all cell time and take the classes of few lanes, which pad least; in a small one the chip waits
-// for the longest wavefront, so a query of many rows takes more lanes and fewer passes.  1.5: a warp that shares
-// its scheduler at the start and ends alone runs between once and 2.6 times its lone time.
+// What a query costs the batch in a class: the chip's time for its cells, plus a part of what its critical path
+// exceeds the whole batch by (batch_ps: the batch's time with every query in its cheapest class).  Large batches
+// are all cell time and take the classes of few lanes, which pad least; in a small one the chip waits for the
+// longest wavefront, so a query of many rows takes more lanes and fewer passes, or a team.  A path counts three
+// times its lone length (a warp shares its scheduler with up to three others for most of its run), and its excess
+// a tenth (the queries that exceed do so side by side).  Measured over factors 0-5 and weights 0.03-3: 100 PSSM
+// queries x 300 targets 2.30 ms without the term, 1.44 with (1.5, 1), 1.10 with (3, 0.1); 600 queries 4.92, 4.83,
+// 4.70 ms; 64 profiles x 1,000 samples 3.74, 2.42, 2.42 ms.
 TUNE_HD inline double tune_objective(double est_ps, double crit_ps, double batch_ps) {
-  const double over = 1.5 * crit_ps - batch_ps;
-  return est_ps + (over > 0.0 ? over : 0.0);
+  const double over = 3.0 * crit_ps - batch_ps;
+  return est_ps + (over > 0.0 ? 0.1 * over : 0.0);
 }
 
 // Warp tasks per unit of a CTA task: a CTA's warps, fewer (a power of two) when the batch has not that many for
@@ -160,7 +177,8 @@ inline int tuning_pick_batch(const Tuning* t, uint32_t m, uint32_t longest, uint
     st_tuning_class_shape(c, &G, &R, &C);
     const uint32_t rows = static_cast<uint32_t>(G * R), P = (m + rows - 1) / rows;
     const uint32_t minc = P > 1 ? std::max<uint32_t>(32, (static_cast<uint32_t>(C * G) + 15) & ~15u) : 32u;
-    const double crit = tune_crit_ps(G, R, C, P, std::max<uint32_t>(minc, (longest + 3) & ~3u));
+    const double crit = tune_crit_ps(G, R, C, P, std::max<uint32_t>(minc, (longest + 3) & ~3u),
+                                     st_tuning_class_team(c) ? st_tuning_class_warps(c) : 1);
     const double v = tune_objective(est[c], crit, batch_ps);
     if (v < bt) {
       bt = v;
@@ -170,28 +188,18 @@ inline int tuning_pick_batch(const Tuning* t, uint32_t m, uint32_t longest, uint
   return best;
 }
 
-// Estimated cost of scoring one query (m rows) against targets of mean length n in class c:
-// a warp streams P * ncols / C steps per warp task of 64/G targets, each step costing R*C
-// row updates plus a per-step overhead; a lone alignment also pays the wavefront ramp.
-inline double tune_cost(const Tuning* t, int c, uint32_t m, uint32_t n, bool single) {
-  int G, R, C;
-  st_tuning_class_shape(c, &G, &R, &C);
-  const uint32_t rows = static_cast<uint32_t>(G * R);
-  const uint32_t P = (m + rows - 1) / rows;
-  if (22.0 * P * rows > 216.0 * 1024) return 1e300;  // profile does not fit shared memory
-  double ncols = n < 32 ? 32.0 : static_cast<double>((n + 15) & ~15u);
-  if (P > 1 && ncols < C * G) ncols = ((C * G + 15) / 16) * 16.0;
-  const double steps = P * ncols / C;
-  const double per_step = R * C + t->step_overhead;
-  if (single) return (steps + G - 1) * per_step;
-  return steps * per_step * G / 64.0;
-}
-
-inline int tuning_model_pick(const Tuning* t, uint32_t m, uint32_t n, bool single) {
+// The class in which a lone alignment of m rows and n columns is done first.
+inline int tuning_pick_single(const Tuning*, uint32_t m, uint32_t n) {
   int best = 0;
   double bc = 1e301;
   for (int c = 0; c < st_tuning_num_classes(); ++c) {
-    const double v = tune_cost(t, c, m, n, single);
+    int G, R, C;
+    st_tuning_class_shape(c, &G, &R, &C);
+    const uint32_t rows = static_cast<uint32_t>(G * R), P = (m + rows - 1) / rows;
+    if (22.0 * P * rows > 216.0 * 1024) continue;  // profile does not fit shared memory
+    uint32_t ncols = std::max<uint32_t>(32, (n + 3) & ~3u);
+    if (P > 1) ncols = std::max<uint32_t>(ncols, (static_cast<uint32_t>(C * G) + 15) & ~15u);
+    const double v = tune_crit_ps(G, R, C, P, ncols, st_tuning_class_team(c) ? st_tuning_class_warps(c) : 1);
     if (v < bc) {
       bc = v;
       best = c;
@@ -199,5 +207,3 @@ inline int tuning_model_pick(const Tuning* t, uint32_t m, uint32_t n, bool singl
   }
   return best;
 }
-
-inline int tuning_pick_single(const Tuning* t, uint32_t m, uint32_t n) { return tuning_model_pick(t, m, n, true); }
