@@ -384,6 +384,14 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 4 || (R == 8 && MODE == k
       }
       return r;
     };
+    // the reverse mode streams the longest prefix of the task, not its longest target (all lanes call it)
+    auto clip = [&](Sw16WarpTask& wt, const Sw16Pair2& r) {
+      if constexpr (MODE == kSw16RevEnd) {
+        const uint32_t len = __reduce_max_sync(FULL, feeder ? max(r.lenA, r.lenB) : 0u);
+        const uint32_t least = P > 1 ? (C * G + 15u) & ~15u : 32u;
+        wt.ncols = min(wt.ncols, max(least, (len + 3u) & ~3u));
+      }
+    };
     auto load_step = [&](const uint8_t* t, uint32_t len, int c) -> uint32_t {
       if constexpr (MODE == kSw16RevEnd) return feeder ? load_codes_rev(t, static_cast<int>(len) - 1, c) : SENTW;
       else return load_codes<C>(feeder, t, len, c);
@@ -407,11 +415,13 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 4 || (R == 8 && MODE == k
     Sw16WarpTask wt_cur = prm.warp_tasks[w_cur];
     Sw16Pair2 cur{};
     if (feeder) cur = load_pairs(wt_cur.slot_begin);
+    clip(wt_cur, cur);
     uint32_t w_nxt = TEAM ? task.wt_end : claim();
     bool have_nxt = w_nxt < task.wt_end;
     Sw16WarpTask wt_nxt = have_nxt ? prm.warp_tasks[w_nxt] : Sw16WarpTask{0, 0};
     Sw16Pair2 nxt{};
     if (have_nxt && feeder) nxt = load_pairs(wt_nxt.slot_begin);
+    if (have_nxt) clip(wt_nxt, nxt);
     if (!TEAM && feeder) open_slot(0, cur);
     // Lane 0's position: column u_col of pass u_pass of task u_seq.  The control word of an ordinary step is
     // u_ctl; the first and the last step of a pass add their events, so an ordinary step takes no decisions
@@ -518,6 +528,7 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 4 || (R == 8 && MODE == k
                 if (have_nxt) {
                   wt_nxt = prm.warp_tasks[w_nxt];
                   if (feeder) nxt = load_pairs(wt_nxt.slot_begin);
+                  clip(wt_nxt, nxt);
                 }
                 u_end = static_cast<int>(wt_cur.ncols);
               }

@@ -46,9 +46,10 @@ def check(ctx, rows, targets, gaps):
 @pytest.mark.parametrize("gaps", [(11, 1), (0, 0), (2, 3)])
 def test_every_end_class(ctx, cls, gaps):
     m = blosum62()
-    rng = XorShift(5 + 100 * cls[0] + cls[1])
+    index = tile_classes().index(cls)
+    rng = XorShift(5 + 100 * index)
     rows, targets = [], []
-    for ql in (1, 7, 8, 63, 65, 129, 260, 530, 1100):
+    for ql in (1, 7, 8, 63, 65, 129, 260, 530, 1100, 2100):
         for tl, letters in ((1, 20), (4, 2), (31, 3), (66, 2), (250, 20), (333, 4)):
             q = np.array(rand_seq(rng, ql, letters), dtype=np.uint8)
             t = np.array(rand_seq(rng, tl, letters), dtype=np.uint8)
@@ -59,7 +60,7 @@ def test_every_end_class(ctx, cls, gaps):
             targets.append(t)
     saved = ctx.tuning_table()
     try:
-        ctx.set_tuning_table(np.full((10, 8), tile_classes().index(cls), dtype=np.int32))
+        ctx.set_tuning_table(np.full((10, 8), index, dtype=np.int32))
         check(ctx, rows, targets, GapCosts(*gaps))
     finally:
         ctx.set_tuning_table(saved)
