@@ -663,6 +663,8 @@ static int set_smem_limits(int device) {
   g_ung_split_smem = std::min<int>(kMaxSmem, optin - static_cast<int>(fa_s.sharedSizeBytes));
   ST_CUDA(cudaFuncSetAttribute(ungapped_hits_split_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                g_ung_split_smem));
+  ST_CUDA(cudaFuncSetAttribute(seed_emit_warp_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               2 * kSeedWarpCap * static_cast<int>(sizeof(int2))));
   cudaFuncAttributes fa_g;
   ST_CUDA(cudaFuncGetAttributes(&fa_g, reinterpret_cast<const void*>(gate_score_kernel)));
   g_gate_smem = std::min<int>(kMaxSmem, optin - static_cast<int>(fa_g.sharedSizeBytes));
@@ -3882,8 +3884,13 @@ static int seed_stage(st_ctx* c, const uint32_t* profiles, uint32_t n_q, const u
     const uint64_t cap = static_cast<uint64_t>(c->sms) * (2048 / block) * 4;
     return static_cast<uint32_t>(std::max<uint64_t>(1, std::min<uint64_t>((items + block - 1) / block, cap)));
   };
-  seed_sort_rows_kernel<<<n_q, 128, 0, s>>>(prof_view(c), Q.qids, Q.row0, const_cast<SeedRow*>(Q.rows));
-  seed_count_kernel<<<grid_for(nw + 1, 128), 128, 0, s>>>(Q, P, slots, win, st);
+  // rows of one query over several CTAs when there are few queries
+  const uint32_t row_ctas = std::max<uint32_t>(1, std::min<uint32_t>(64, 8 * c->sms / n_q));
+  seed_sort_rows_kernel<<<dim3(n_q, row_ctas), 128, 0, s>>>(prof_view(c), Q.qids, Q.row0,
+                                                            const_cast<SeedRow*>(Q.rows));
+  // one warp a window: CTAs of a warp, several rounds' worth for balance
+  const uint32_t win_ctas = static_cast<uint32_t>(std::min<uint64_t>(nw + 1, static_cast<uint64_t>(c->sms) * 64));
+  seed_count_kernel<<<win_ctas, 32, 0, s>>>(Q, P, slots, win, st);
   size_t t = t_scan;
   ST_CUDA(cub::DeviceScan::ExclusiveSum(b + o_tmp, t, slots, soff, nw + 1, s));
   c->launches += 3;
@@ -3909,7 +3916,10 @@ static int seed_stage(st_ctx* c, const uint32_t* profiles, uint32_t n_q, const u
   SeedSeed* seeds = reinterpret_cast<SeedSeed*>(b2 + o_seeds);
   uint32_t* cnt = reinterpret_cast<uint32_t*>(b2 + o_cnt);
   uint32_t* hoff = reinterpret_cast<uint32_t*>(b2 + o_hoff);
-  if (ns) seed_emit_kernel<<<grid_for(nw, 128), 128, 0, s>>>(Q, P, soff, win, seeds, st);
+  if (ns && Q.cap <= kSeedWarpCap)
+    seed_emit_warp_kernel<<<win_ctas, 32, 2 * Q.cap * sizeof(int2), s>>>(Q, P, soff, win, seeds, st);
+  else if (ns)
+    seed_emit_kernel<<<grid_for(nw, 128), 128, 0, s>>>(Q, P, soff, win, seeds, st);
   seed_post_count_kernel<<<grid_for(ns + 1, 256), 256, 0, s>>>(seeds, static_cast<uint32_t>(ns),
                                                                c->seed_off.as<uint32_t>(),
                                                                sp->max_seed_occ, cnt, st);

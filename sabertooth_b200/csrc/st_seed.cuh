@@ -8,7 +8,7 @@
 // per sequence with one atomic counter per code (the order inside a code does
 // not matter: hits are grouped by a sort later).
 //
-// Queries, one thread per window (query, start):
+// Queries, one warp per window (query, start):
 //   count  eligibility (no care residue >= 20 for sequence queries), the number
 //          of k-mers over the 20 standard residues scoring >= kmer_score from a
 //          histogram of partial sums pruned at the threshold (the counting pass
@@ -96,6 +96,9 @@ __global__ void __launch_bounds__(256) seed_index_kernel(DeviceDb db, SeedPat p,
   }
 }
 
+// One warp per query row: a residue's place is the number of residues before it (higher score, or the same and a
+// smaller code), counted over the lanes.  (One thread per row with an insertion sort: 26 us for one query, the
+// dependent swaps of 20 entries in local memory.)
 __global__ void __launch_bounds__(128) seed_sort_rows_kernel(DeviceProfiles prof, const uint32_t* qids,
                                                              const uint32_t* row0, SeedRow* rows) {
   const uint32_t qi = blockIdx.x;
@@ -103,22 +106,21 @@ __global__ void __launch_bounds__(128) seed_sort_rows_kernel(DeviceProfiles prof
   const uint32_t m = prof.qlen[q];
   const int32_t* p32 = prof.p32[q];
   const uint32_t s32 = prof.stride32[q];
-  for (uint32_t i = threadIdx.x; i < m; i += blockDim.x) {
-    SeedRow r;
+  const uint32_t lane = threadIdx.x & 31;
+  const uint32_t warps = gridDim.y * (blockDim.x / 32);
+  for (uint32_t i = blockIdx.y * (blockDim.x / 32) + threadIdx.x / 32; i < m; i += warps) {
+    const int32_t sc = lane < kSeedAA ? p32[lane * s32 + i] : INT32_MIN;
+    uint32_t place = 0;
+#pragma unroll
     for (int a = 0; a < kSeedAA; ++a) {
-      r.sc[a] = p32[a * s32 + i];
-      r.res[a] = static_cast<uint8_t>(a);
+      const int32_t o = __shfl_sync(0xFFFFFFFFu, sc, a);
+      place += o > sc || (o == sc && a < static_cast<int>(lane)) ? 1u : 0u;
     }
-    for (int a = 1; a < kSeedAA; ++a)  // stable: equal scores keep residue order
-      for (int b = a; b > 0 && r.sc[b] > r.sc[b - 1]; --b) {
-        const int32_t ts = r.sc[b];
-        r.sc[b] = r.sc[b - 1];
-        r.sc[b - 1] = ts;
-        const uint8_t tr = r.res[b];
-        r.res[b] = r.res[b - 1];
-        r.res[b - 1] = tr;
-      }
-    rows[row0[qi] + i] = r;
+    if (lane < kSeedAA) {
+      SeedRow& r = rows[row0[qi] + i];
+      r.sc[place] = sc;
+      r.res[place] = static_cast<uint8_t>(lane);
+    }
   }
 }
 
@@ -162,11 +164,37 @@ __device__ __forceinline__ bool seed_window_rows(const SeedQ& Q, const SeedPat& 
   return true;
 }
 
-__global__ void __launch_bounds__(128) seed_count_kernel(SeedQ Q, SeedPat P, uint32_t* slots, SeedWin* win,
-                                                         SeedStatsDev* st) {
+// A window's sorted rows and its suffix maxima in shared memory, by one warp: smax[i] = the best sum of rows i .. w-1.
+struct SeedWinRows {
+  int32_t sc[kSeedMaxW][kSeedAA];
+  uint8_t res[kSeedMaxW][kSeedAA];
+  int32_t smax[kSeedMaxW + 1];
+};
+__device__ __forceinline__ void seed_load_rows(const SeedPat& P, const SeedRow* const* wr, SeedWinRows& o) {
+  const uint32_t lane = threadIdx.x & 31;
+  for (uint32_t i = 0; i < P.w; ++i)
+    if (lane < kSeedAA) {
+      o.sc[i][lane] = wr[i]->sc[lane];
+      o.res[i][lane] = wr[i]->res[lane];
+    }
+  __syncwarp();
+  if (lane == 0) {
+    o.smax[P.w] = 0;
+    for (int i = static_cast<int>(P.w) - 1; i >= 0; --i) o.smax[i] = o.smax[i + 1] + o.sc[i][0];
+  }
+  __syncwarp();
+}
+
+// One warp (a CTA) per window: the histogram of the partial sums that can still reach the threshold, row by row, its
+// (sum, residue) pairs spread over the lanes with shared-memory atomics.  One thread per window kept both histograms
+// in local memory and took 86 us for a lone query of 257 windows, the latency of one thread's chain.
+__global__ void __launch_bounds__(32) seed_count_kernel(SeedQ Q, SeedPat P, uint32_t* slots, SeedWin* win,
+                                                        SeedStatsDev* st) {
+  __shared__ SeedWinRows W;
+  __shared__ uint32_t hist[2][kSeedMaxBins];
   unsigned long long n_skip = 0, n_cap = 0, n_err = 0;
-  uint32_t dist[kSeedMaxBins], tmp[kSeedMaxBins];
-  for (uint32_t wi = blockIdx.x * blockDim.x + threadIdx.x; wi <= Q.n_win; wi += gridDim.x * blockDim.x) {
+  const uint32_t lane = threadIdx.x;
+  for (uint32_t wi = blockIdx.x; wi <= Q.n_win; wi += gridDim.x) {
     uint32_t n_slots = 0;
     if (wi < Q.n_win) {
       uint32_t qi, start, exact;
@@ -176,68 +204,209 @@ __global__ void __launch_bounds__(128) seed_count_kernel(SeedQ Q, SeedPat P, uin
       if (!seed_window_rows(Q, P, qi, start, wr, exact)) {
         ++n_skip;
       } else {
-        int32_t smax[kSeedMaxW + 1];
-        smax[P.w] = 0;
-        for (int i = static_cast<int>(P.w) - 1; i >= 0; --i) smax[i] = smax[i + 1] + wr[i]->sc[0];
+        seed_load_rows(P, wr, W);
         uint32_t count = 0;
-        if (smax[0] >= Q.thr && Q.cap > 0) {
-          // histogram of the partial sums that can still reach the threshold
+        if (W.smax[0] >= Q.thr && Q.cap > 0) {
           int32_t lo = 0, hi = 0;
-          dist[0] = 1;
+          uint32_t *dist = hist[0], *next = hist[1];
+          if (lane == 0) dist[0] = 1;
+          __syncwarp();
           bool ok = true;
-          for (uint32_t i = 0; i < P.w && ok; ++i) {
-            const int32_t nhi = hi + wr[i]->sc[0];
-            const int32_t nlo = max(lo + wr[i]->sc[kSeedAA - 1], Q.thr - smax[i + 1]);
+          for (uint32_t i = 0; i < P.w; ++i) {
+            const int32_t nhi = hi + W.sc[i][0];
+            const int32_t nlo = max(lo + W.sc[i][kSeedAA - 1], Q.thr - W.smax[i + 1]);
             if (nhi - nlo + 1 > kSeedMaxBins) {
               ok = false;
               break;
             }
-            for (int32_t b = 0; b <= nhi - nlo; ++b) tmp[b] = 0;
-            for (int32_t off = 0; off <= hi - lo; ++off) {
+            for (int32_t b = lane; b <= nhi - nlo; b += 32) next[b] = 0;
+            __syncwarp();
+            const int32_t items = (hi - lo + 1) * kSeedAA;
+            for (int32_t x = lane; x < items; x += 32) {
+              const int32_t off = x / kSeedAA;
               const uint32_t cnt = dist[off];
-              if (!cnt) continue;
-              const int32_t s = lo + off;
-              for (int a = 0; a < kSeedAA; ++a) {
-                const int32_t t = s + wr[i]->sc[a];
-                if (t < nlo) break;
-                tmp[t - nlo] += cnt;
-              }
+              const int32_t t = lo + off + W.sc[i][x - off * kSeedAA];
+              if (cnt && t >= nlo) atomicAdd(&next[t - nlo], cnt);
             }
-            for (int32_t b = 0; b <= nhi - nlo; ++b) dist[b] = tmp[b];
+            __syncwarp();
+            uint32_t* x = dist;
+            dist = next;
+            next = x;
             lo = nlo;
             hi = nhi;
           }
           if (!ok) {
             ++n_err;
           } else {
-            for (int32_t b = 0; b <= hi - lo; ++b) count += dist[b];
-            if (count > Q.cap) {
+            for (int32_t b = lane; b <= hi - lo; b += 32) count += dist[b];
+            count = __reduce_add_sync(0xFFFFFFFFu, count);
+            if (count > Q.cap) {  // the boundary score, 32 bins at a time from the top
               uint32_t above = 0;
-              int32_t t = hi;
-              for (; t > lo; --t) {
-                const uint32_t cnt = dist[t - lo];
-                if (above + cnt >= Q.cap) break;
-                above += cnt;
+              int32_t top = hi;
+              for (;; top -= 32) {
+                const int32_t t = top - static_cast<int32_t>(lane);
+                const uint32_t cnt = t >= lo ? dist[t - lo] : 0u;
+                uint32_t incl = cnt;
+#pragma unroll
+                for (int o = 1; o < 32; o <<= 1) {
+                  const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, incl, o);
+                  if (lane >= o) incl += y;
+                }
+                const uint32_t hit = __ballot_sync(0xFFFFFFFFu, t <= lo || above + incl >= Q.cap);
+                if (hit) {
+                  const int src = __ffs(hit) - 1;
+                  wv.tstar = top - src;
+                  wv.need = Q.cap - (above + __shfl_sync(0xFFFFFFFFu, incl - cnt, src));
+                  break;
+                }
+                above += __shfl_sync(0xFFFFFFFFu, incl, 31);
               }
-              wv.tstar = t;
-              wv.need = Q.cap - above;
               count = Q.cap;
               ++n_cap;
             }
           }
         }
         n_slots = count + (Q.exact ? 1u : 0u);
+        __syncwarp();  // the shared rows and histograms are free for the next window
       }
-      win[wi] = wv;
+      if (lane == 0) win[wi] = wv;
     }
-    slots[wi] = n_slots;
+    if (lane == 0) slots[wi] = n_slots;
   }
-  gate_flush(&st->windows_skipped, n_skip);
-  gate_flush(&st->windows_at_cap, n_cap);
-  gate_flush(&st->errors, n_err);
+  if (lane == 0) {
+    if (n_skip) atomicAdd(&st->windows_skipped, n_skip);
+    if (n_cap) atomicAdd(&st->windows_at_cap, n_cap);
+    if (n_err) atomicAdd(&st->errors, n_err);
+  }
 }
 
-// The kept k-mers of each window in rank-lexicographic depth-first order.
+// The kept k-mers of each window, one warp (a CTA) per window, level by level: the nodes of a level are the prefixes
+// that can still reach the boundary, in rank-lexicographic order, and a node's children are the first ranks of its
+// row.  Those that can exceed the boundary score are all kept (each leads to a k-mer above it, so there are at most
+// as many as such k-mers); of those that can only reach it, the first `need` in order (each leads to a tie, and
+// only the first `need` ties are kept), so a level never holds more than the cap.  Positions come from warp scans,
+// and the children of 32 nodes are written 32 at a time whatever their numbers, so a window costs its k-mers over
+// the lanes.  The set kept is the depth-first walk's (seed_emit_kernel), in its order.  One thread per window took
+// 720 us for a lone query (two CTAs, each thread walking up to 512 k-mers) and 1.38 ms for 150 queries.
+constexpr uint32_t kSeedWarpCap = 4096;  // cap of the warp form: two levels of nodes in shared memory
+
+__global__ void __launch_bounds__(32) seed_emit_warp_kernel(SeedQ Q, SeedPat P, const uint32_t* soff,
+                                                            const SeedWin* win, SeedSeed* seeds, SeedStatsDev* st) {
+  extern __shared__ int2 nodes[];  // [2][cap]: (partial sum, code)
+  __shared__ SeedWinRows W;
+  constexpr uint32_t FULL = 0xFFFFFFFFu;
+  unsigned long long n_gen = 0, n_exact = 0, n_err = 0;
+  const uint32_t lane = threadIdx.x;
+  for (uint32_t wi = blockIdx.x; wi < Q.n_win; wi += gridDim.x) {
+    const uint32_t o0 = soff[wi], o1 = soff[wi + 1];
+    if (o1 == o0) continue;
+    uint32_t qi, start, exact;
+    seed_window_of(Q, wi, qi, start);
+    const SeedRow* wr[kSeedMaxW];
+    seed_window_rows(Q, P, qi, start, wr, exact);
+    const SeedWin wv = win[wi];
+    const uint32_t n_kmers = o1 - o0 - (Q.exact ? 1u : 0u);
+    bool have_exact = false;
+    uint32_t n = 0;
+    if (n_kmers > 0) {
+      seed_load_rows(P, wr, W);
+      const bool capped = wv.tstar != INT32_MIN;
+      const int32_t above_from = capped ? wv.tstar + 1 : Q.thr;  // sums from here on are kept whatever their order
+      const int32_t from = capped && wv.need ? wv.tstar : above_from;
+      int2 *cur = nodes, *nxt = nodes + Q.cap;
+      if (lane == 0) cur[0] = make_int2(0, 0);
+      __syncwarp();
+      uint32_t n_cur = 1;
+      for (uint32_t d = 0; d < P.w; ++d) {
+        const bool leaf = d + 1 == P.w;
+        const int32_t rest = W.smax[d + 1];
+        uint32_t n_out = 0, ties = 0;  // children written, ties met
+        for (uint32_t c0 = 0; c0 < n_cur; c0 += 32) {
+          int2 nd = make_int2(0, 0);
+          uint32_t above = 0, all = 0;  // children that can exceed the boundary, that can reach it
+          if (c0 + lane < n_cur) {
+            nd = cur[c0 + lane];
+            // scores descend: the number of ranks whose sum reaches a bound
+            auto reach = [&](int32_t bound) {
+              uint32_t l = 0, h = kSeedAA;  // ranks below l reach it, ranks from h do not
+              while (l < h) {
+                const uint32_t mid = (l + h) >> 1;
+                if (nd.x + W.sc[d][mid] + rest >= bound) l = mid + 1; else h = mid;
+              }
+              return l;
+            };
+            above = reach(above_from);
+            all = from == above_from ? above : reach(from);
+          }
+          uint32_t tie = all - above, tincl = tie;
+#pragma unroll
+          for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t y = __shfl_up_sync(FULL, tincl, o);
+            if (lane >= o) tincl += y;
+          }
+          const uint32_t tbefore = ties + tincl - tie;
+          tie = tbefore >= wv.need ? 0u : min(tie, wv.need - tbefore);
+          ties += __shfl_sync(FULL, tincl, 31);
+          uint32_t incl = above + tie;
+#pragma unroll
+          for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t y = __shfl_up_sync(FULL, incl, o);
+            if (lane >= o) incl += y;
+          }
+          const uint32_t excl = incl - (above + tie);
+          const uint32_t total = __shfl_sync(FULL, incl, 31);
+          for (uint32_t k0 = 0; k0 < total; k0 += 32) {  // every lane runs every round (shuffles)
+            const uint32_t k = k0 + lane;
+            uint32_t j = 0;  // last lane whose children begin at or before k
+#pragma unroll
+            for (int step = 16; step > 0; step >>= 1) {
+              const uint32_t oc = __shfl_sync(FULL, excl, (j + step) & 31);
+              if (j + step < 32 && oc <= k) j += step;
+            }
+            const uint32_t r = k - __shfl_sync(FULL, excl, j);
+            const int32_t part = __shfl_sync(FULL, nd.x, j);
+            const uint32_t code = static_cast<uint32_t>(__shfl_sync(FULL, nd.y, j));
+            bool same = false;
+            if (k < total) {
+              const uint32_t cc = code * kSeedAA + W.res[d][r];
+              const uint32_t at = n_out + k;
+              if (leaf) {
+                if (at < n_kmers) seeds[o0 + at] = SeedSeed{cc, wi};
+                same = cc == exact;
+              } else if (at < Q.cap) {
+                nxt[at] = make_int2(part + W.sc[d][r], static_cast<int>(cc));
+              }
+            }
+            if (leaf) have_exact |= __any_sync(FULL, same);
+          }
+          n_out += total;
+        }
+        __syncwarp();
+        int2* x = cur;
+        cur = nxt;
+        nxt = x;
+        n_cur = min(n_out, Q.cap);
+        n = n_out;
+      }
+      n_err += n != n_kmers;
+      n_gen += n;
+      __syncwarp();  // the shared rows and nodes are free for the next window
+    }
+    if (Q.exact) {
+      if (lane == 0) seeds[o0 + n_kmers] = SeedSeed{have_exact ? kSeedNone : exact, wi};
+      n_exact += have_exact ? 0 : 1;
+      n_gen += have_exact ? 0 : 1;
+    }
+  }
+  if (lane == 0) {
+    if (n_gen) atomicAdd(&st->kmers_generated, n_gen);
+    if (n_exact) atomicAdd(&st->exact_seeds_added, n_exact);
+    if (n_err) atomicAdd(&st->errors, n_err);
+  }
+}
+
+// The kept k-mers of each window in rank-lexicographic depth-first order, one thread per window: for caps whose levels
+// do not fit shared memory (seed_emit_warp_kernel).
 __global__ void __launch_bounds__(128) seed_emit_kernel(SeedQ Q, SeedPat P, const uint32_t* soff, const SeedWin* win,
                                                         SeedSeed* seeds, SeedStatsDev* st) {
   unsigned long long n_gen = 0, n_exact = 0, n_err = 0;
