@@ -32,11 +32,11 @@
 //            inside equal scores; per-query cut to max_candidates; gather
 #pragma once
 #include "st_common.cuh"
+#include "st_ungapped.cuh"
 
 namespace st {
 
 constexpr int kGateMaxDiags = 16;  // jobs per target (src/prefilter.rs:1459, top.iter().take(16))
-constexpr int kGateChunk = 1024;   // jobs per CTA chunk of the segment kernel
 
 struct GateCandidate {  // the layout of st_candidate
   uint32_t query;
@@ -109,6 +109,22 @@ __device__ __forceinline__ int32_t gate_key_diag(uint64_t k, const GateConf& g) 
 __device__ __forceinline__ void gate_flush(unsigned long long* ctr, unsigned long long v) {
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xFFFFFFFFu, v, o);
   if ((threadIdx.x & 31) == 0 && v) atomicAdd(ctr, v);
+}
+
+// The same with one atomic a block, for short even loops whose every warp has a
+// count: a counter is a single address, which takes about one atomic a
+// nanosecond (seed_post_count_kernel of 38,000 warps 187 -> 128 us).  Kernels of
+// uneven warps keep the form above: the barrier holds their early warps' places
+// (gate_count_kernel 108 -> 147 us with this one).
+__device__ __forceinline__ void gate_flush_block(unsigned long long* ctr, unsigned long long v) {
+  __shared__ unsigned long long s_sum;
+  if (threadIdx.x == 0) s_sum = 0;
+  __syncthreads();
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xFFFFFFFFu, v, o);
+  if ((threadIdx.x & 31) == 0 && v) atomicAdd(&s_sum, v);
+  __syncthreads();
+  if (threadIdx.x == 0 && s_sum) atomicAdd(ctr, s_sum);
+  __syncthreads();  // before the next counter of the block
 }
 
 __global__ void __launch_bounds__(256) gate_keys_kernel(const GateSeedHit* hits, uint64_t n, DeviceDb db,
@@ -276,43 +292,28 @@ struct GateSegParams {
   const uint32_t* joff;  // total jobs at joff[n_groups]
   int32_t* score;
   uint32_t max_m_pad;
+  uint32_t chunk;  // jobs per CTA
 };
 
-// Byte mask of a 16-byte vector: 0xFF for the bytes i with lo <= i < hi.
-__device__ __forceinline__ void gate_window_mask(int32_t lo, int32_t hi, uint32_t m[4]) {
-  const uint32_t bits = ((1u << hi) - 1u) & ~((1u << lo) - 1u);  // 0 <= lo < hi <= 16
-#pragma unroll
-  for (int j = 0; j < 4; ++j) m[j] = (((bits >> (4 * j)) & 0xFu) * 0x00204081u & 0x01010101u) * 0xFFu;
-}
-
-// kadane_score (src/ungapped.rs:53-62) of each job over its window.  A CTA
-// takes a chunk of jobs; per run of one query inside it the query's int8
-// profile is staged in shared memory and every thread keeps one job in flight,
-// one 16-byte target vector per step, taking the run's next job (shared
-// counter) as soon as its own is done, so lanes stay busy whatever the window
-// lengths.  The first and last vectors of a window have their bytes outside
-// the window replaced by the sentinel code, whose profile row is zero: zero
-// cells at the ends of a window change no Kadane maximum, so the cell loop has
-// no window test.  Profiles outside int8 read int32 rows from global memory
-// with an explicit test.
+// kadane_score (src/ungapped.rs:53-62) of each job over its window: a CTA takes a chunk of jobs and scores each run of
+// one query inside it with diag_score_run.
 __global__ void __launch_bounds__(256) gate_score_kernel(const GateSegParams prm) {
   extern __shared__ __align__(16) int8_t smem[];
   __shared__ uint32_t s_run_end, s_next;
   const uint32_t n = prm.joff[*prm.n_groups];
   const uint32_t stride = prm.max_m_pad;
-  int8_t* base = smem + 16;
-  const uint32_t c0 = blockIdx.x * kGateChunk;
+  const uint64_t c0 = static_cast<uint64_t>(blockIdx.x) * prm.chunk;
   if (c0 >= n) return;
-  const uint32_t c1 = min(n, c0 + kGateChunk);
-  uint32_t a = c0;
-  while (a < c1) {
-    const uint32_t q = prm.jobs[a].query;
+  const uint32_t nc = min(n - static_cast<uint32_t>(c0), prm.chunk);
+  const GateJob* chunk = prm.jobs + c0;
+  uint32_t a = 0;
+  while (a < nc) {
+    const uint32_t q = chunk[a].query;
     if (threadIdx.x < 32) {
       uint32_t e = a;
       for (;;) {
         const uint32_t k = e + threadIdx.x;
-        const bool same = (k < c1) && (prm.jobs[k].query == q);
-        const uint32_t ball = __ballot_sync(0xFFFFFFFFu, same);
+        const uint32_t ball = __ballot_sync(0xFFFFFFFFu, k < nc && chunk[k].query == q);
         if (ball != 0xFFFFFFFFu) {
           e += __ffs(~ball) - 1;
           break;
@@ -321,85 +322,20 @@ __global__ void __launch_bounds__(256) gate_score_kernel(const GateSegParams prm
       }
       if (threadIdx.x == 0) {
         s_run_end = e;
-        s_next = a + blockDim.x;
+        s_next = blockDim.x;
       }
     }
-    const uint32_t pstride = prm.prof.stride8[q];
-    const int8_t* src = prm.prof.p8[q];
-    for (uint32_t idx = threadIdx.x; idx < kProfRows * (stride / 16); idx += blockDim.x) {
-      const uint32_t r = idx / (stride / 16);
-      const uint32_t i = (idx - r * (stride / 16)) * 16;
-      uint4 v = make_uint4(0, 0, 0, 0);
-      if (i < pstride) v = *reinterpret_cast<const uint4*>(src + static_cast<size_t>(r) * pstride + i);
-      *reinterpret_cast<uint4*>(base + static_cast<size_t>(r) * stride + i) = v;
-    }
-    if (threadIdx.x < 16) smem[threadIdx.x] = 0;
+    diag_stage(prm.prof, q, stride, smem);
     __syncthreads();
     const uint32_t b = s_run_end;
-    const bool narrow = prm.prof.fits8[q] != 0;
-    const int32_t* p32 = prm.prof.p32[q];
-    const int32_t s32 = static_cast<int32_t>(prm.prof.stride32[q]);
-    const int32_t last_row = static_cast<int32_t>(prm.prof.qlen[q]) - 1;
-    // per lane: job k, target base, diagonal, window [p0, p1) in target positions, next vector pa
-    uint32_t k = a + threadIdx.x;
-    const uint8_t* tp = nullptr;
-    int32_t d = 0, p0 = 0, p1 = 0, pa = 0, cur = 0, best = 0;
-    bool live = false;
-    auto take = [&](uint32_t j) {
-      k = j;
-      live = j < b;
-      if (live) {
-        const GateJob jb = prm.jobs[j];
-        tp = prm.db.arena + prm.db.offset[jb.target];
-        d = jb.diag;
-        p0 = static_cast<int32_t>(jb.lo) + d;
-        p1 = static_cast<int32_t>(jb.hi) + d;
-        pa = jb.hi > jb.lo ? (p0 & ~15) : p1;  // an empty window is done at once (p0 may be negative)
-        cur = 0;
-        best = 0;
-      }
-    };
-    take(k);
-    while (__any_sync(0xFFFFFFFFu, live)) {
-      if (live) {
-        if (pa < p1) {
-          const uint4 v = *reinterpret_cast<const uint4*>(tp + pa);
-          uint32_t w[4] = {v.x, v.y, v.z, v.w};
-          const int32_t qa = pa - d;
-          if (narrow) {
-            if (pa < p0 || pa + 16 > p1) {  // a window end inside this vector
-              uint32_t m[4];
-              gate_window_mask(max(p0 - pa, 0), min(p1 - pa, 16), m);
-#pragma unroll
-              for (int j = 0; j < 4; ++j) w[j] = (w[j] & m[j]) | (0x15151515u & ~m[j]);
-            }
-            const int8_t* rowbase = base + qa;
-#pragma unroll
-            for (int bb = 0; bb < 16; ++bb) {
-              const uint32_t r = (w[bb >> 2] >> ((bb & 3) * 8)) & 0xFFu;
-              cur = wadd(max(cur, 0), static_cast<int32_t>(rowbase[static_cast<int32_t>(r * stride) + bb]));
-              best = max(best, cur);
-            }
-          } else {
-#pragma unroll
-            for (int bb = 0; bb < 16; ++bb) {
-              const uint32_t r = (w[bb >> 2] >> ((bb & 3) * 8)) & 0xFFu;
-              const int32_t p = pa + bb;
-              const int32_t row = min(max(qa + bb, 0), last_row);
-              const int32_t sc = (p >= p0 && p < p1) ? __ldg(p32 + static_cast<int32_t>(r) * s32 + row) : 0;
-              cur = wadd(max(cur, 0), sc);
-              best = max(best, cur);
-            }
-          }
-          pa += 16;
-        }
-        if (pa >= p1) {  // done (or an empty window)
-          prm.score[k] = best;
-          take(atomicAdd(&s_next, 1u));
-        }
-      }
-    }
-    __syncthreads();
+    const GateJob* run = chunk + a;
+    diag_score_run<true>(
+        smem + 16, stride, prm.prof.fits8[q] != 0, prm.prof.p32[q], static_cast<int32_t>(prm.prof.stride32[q]),
+        static_cast<int32_t>(prm.prof.qlen[q]) - 1, b - a, &s_next, prm.score + c0 + a, [&](uint32_t j) {
+          const GateJob jb = run[j];
+          return DiagWindow{prm.db.arena + prm.db.offset[jb.target], jb.diag, static_cast<int32_t>(jb.lo) + jb.diag,
+                            static_cast<int32_t>(jb.hi) + jb.diag};
+        });
     a = b;
   }
 }
@@ -459,13 +395,48 @@ __device__ __forceinline__ int32_t gate_gap_cost(int32_t open, int32_t ext, uint
 // Groups that may pass the gate: every group with more than one diagonal or
 // with its one diagonal at or above the gate goes to a work list (the order of
 // the list does not matter: each group writes its own slot).  Groups left out
-// keep the zero flag written before.
+// keep the zero flag written before.  A CTA takes the places of its tile of
+// groups with one atomic: one a warp on the one counter was 280 us for 14 M
+// windows' groups.
+constexpr uint32_t kScreenTile = 2048;
 __global__ void __launch_bounds__(256) gate_screen_kernel(GateGroups G, GateConf g, const uint32_t* joff,
                                                           const int32_t* score, uint32_t* work, uint32_t* n_work) {
+  constexpr uint32_t kPer = kScreenTile / 256;
+  __shared__ uint32_t s_warp[8], s_base;
   const uint32_t ng = *G.n_groups;
-  for (uint32_t gi = blockIdx.x * blockDim.x + threadIdx.x; gi < ng; gi += gridDim.x * blockDim.x) {
-    const uint32_t j0 = joff[gi], nsg = joff[gi + 1] - j0;
-    if (nsg > 0 && !(nsg == 1 && score[j0] < g.min_score)) work[atomicAdd(n_work, 1u)] = gi;
+  const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  for (uint32_t t0 = blockIdx.x * kScreenTile; t0 < ng; t0 += gridDim.x * kScreenTile) {
+    uint32_t bits = 0;  // this thread's groups t0 + 256 i + threadIdx.x that may pass
+#pragma unroll
+    for (uint32_t i = 0; i < kPer; ++i) {
+      const uint32_t gi = t0 + 256 * i + threadIdx.x;
+      if (gi < ng) {
+        const uint32_t j0 = joff[gi], nsg = joff[gi + 1] - j0;
+        if (nsg > 1 || (nsg == 1 && score[j0] >= g.min_score)) bits |= 1u << i;
+      }
+    }
+    const uint32_t cnt = __popc(bits);
+    uint32_t incl = cnt;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, incl, o);
+      if (lane >= o) incl += y;
+    }
+    if (lane == 31) s_warp[warp] = incl;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      uint32_t sum = 0;
+      for (int w = 0; w < 8; ++w) {
+        const uint32_t x = s_warp[w];
+        s_warp[w] = sum;
+        sum += x;
+      }
+      s_base = sum ? atomicAdd(n_work, sum) : 0u;
+    }
+    __syncthreads();
+    uint32_t at = s_base + s_warp[warp] + incl - cnt;
+    for (uint32_t b = bits; b; b &= b - 1) work[at++] = t0 + 256 * (__ffs(b) - 1) + threadIdx.x;
+    __syncthreads();
   }
 }
 

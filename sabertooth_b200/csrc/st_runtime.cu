@@ -3192,6 +3192,12 @@ extern "C" int st_sw_score(st_ctx* c, uint32_t profile, const uint8_t* target, u
 // ---------------------------------------------------------------------------
 static uint32_t ung_stride(st_ctx* c) { return static_cast<uint32_t>(up16(c->max_m) + 32); }
 
+// Windows per CTA of the diagonal kernels: 1,024 (more lengthen the kernel's tail: 2,048, 4,096 and 8,192 measured
+// slower on 2x10^7 hits), 256 where a small call would otherwise leave SMs without a CTA.
+static uint32_t diag_chunk(st_ctx* c, uint64_t n) {
+  return n / kUngChunk >= 2ull * c->sms ? static_cast<uint32_t>(kUngChunk) : 256u;
+}
+
 // max_m: the longest query the jobs refer to (0: any live profile), which sizes
 // the staged profile rows and so the CTAs that fit on an SM.
 static int launch_ungapped(st_ctx* c, bool hits, const void* d_jobs, uint64_t n, int32_t* d_out, uint32_t max_m = 0) {
@@ -3214,9 +3220,10 @@ static int launch_ungapped(st_ctx* c, bool hits, const void* d_jobs, uint64_t n,
   const bool split = env_u64("ST_UNGAPPED_SPLIT", 0) != 0;
   if (hits && split && smem <= static_cast<size_t>(g_ung_split_smem))
     ungapped_hits_split_kernel<<<static_cast<uint32_t>(grid), kUngSplitLanes, smem, c->stream>>>(prm);
-  else if (hits)
-    ungapped_hits_refill_kernel<<<static_cast<uint32_t>(grid), 256, smem, c->stream>>>(prm);
-  else
+  else if (hits) {
+    prm.chunk = diag_chunk(c, n);
+    ungapped_hits_refill_kernel<<<static_cast<uint32_t>((n + prm.chunk - 1) / prm.chunk), 256, smem, c->stream>>>(prm);
+  } else
     ungapped_kernel<false><<<static_cast<uint32_t>(grid), 256, smem, c->stream>>>(prm);
   ++c->launches;
   ST_CUDA(cudaGetLastError());
@@ -3618,10 +3625,9 @@ static int gate_pipeline(st_ctx* c, const GateSeedHit* d_hits, uint32_t n, const
   else
     gate_emit_kernel<kGateMaxDiags><<<grid_for(n, 128), 128, 0, s>>>(G, g, db, pv.qlen, ns, joff, jobs);
   // window scores
-  GateSegParams sp{db, pv, jobs, ng, joff, sc, g.stride};
+  GateSegParams sp{db, pv, jobs, ng, joff, sc, g.stride, diag_chunk(c, n)};
   const size_t smem = 16 + static_cast<size_t>(kProfRows) * sp.max_m_pad + 16;
-  gate_score_kernel<<<static_cast<uint32_t>((static_cast<uint64_t>(n) + kGateChunk - 1) / kGateChunk), 256, smem, s>>>(
-      sp);
+  gate_score_kernel<<<static_cast<uint32_t>((static_cast<uint64_t>(n) + sp.chunk - 1) / sp.chunk), 256, smem, s>>>(sp);
   // chain, gate, compaction
   ST_CUDA(cudaMemsetAsync(flag, 0, n, s));
   ST_CUDA(cudaMemsetAsync(n_work, 0, 4, s));

@@ -508,10 +508,10 @@ __global__ void __launch_bounds__(256) seed_post_count_kernel(const SeedSeed* se
     }
     cnt[i] = len;
   }
-  gate_flush(&st->seeds, n_seed);
-  gate_flush(&st->postings_visited, n_post);
-  gate_flush(&st->seeds_over_occ_cap, n_over);
-  gate_flush(&st->postings_skipped_occ, n_skip);
+  gate_flush_block(&st->seeds, n_seed);
+  gate_flush_block(&st->postings_visited, n_post);
+  gate_flush_block(&st->seeds_over_occ_cap, n_over);
+  gate_flush_block(&st->postings_skipped_occ, n_skip);
 }
 
 // One hit per posting.  A warp takes 32 consecutive seeds, whose hits are one

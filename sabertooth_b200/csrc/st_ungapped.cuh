@@ -39,6 +39,7 @@ struct UngappedParams {
   uint64_t n;
   int32_t* out;
   uint32_t max_m_pad;  // row stride of the staged profile (>= every query length + 32)
+  uint32_t chunk;      // hits per CTA (ungapped_hits_refill_kernel)
 };
 
 constexpr int kUngChunk = 1024;  // jobs per CTA chunk
@@ -183,32 +184,141 @@ __global__ void __launch_bounds__(256) ungapped_kernel(const UngappedParams prm)
   }
 }
 
-// Hits (whole-diagonal windows, diag_range) with one hit per lane: per run of
-// one query inside the CTA's chunk the profile is staged as above, then every
-// lane keeps a hit in flight, one 16-byte target vector per step, and takes the
-// run's next hit from a shared counter as soon as its own is done, so lanes
-// stay busy whatever the diagonal lengths.  On int8 profiles no cell needs a
-// test (the argument of the whole-diagonal path of ungapped_kernel); rows
-// outside int8 read the int32 profile with an explicit window test.
+// ---- diagonals of one query, one window per lane with refill ----
+// A run of one query's diagonal windows inside a CTA's chunk, against the query's int8 profile staged in shared memory:
+// every lane keeps a window in flight, one 16-byte target vector per step, and takes the run's next window from a
+// shared counter as soon as its own is done, so lanes stay busy whatever the window lengths.  What bounds it is the
+// shared-memory pipe (80-89 % busy): a cell is one byte lookup, and the lookups of 20 active lanes at unrelated query
+// rows take 2.2 wavefronts.  Sorting a run's windows into 32 bins by the bank their first lookup falls on, and
+// giving each lane only windows whose banks no other lane of the step uses, removed a third of the conflicts but
+// halved the active lanes (11 of 32: most windows start at the query's first rows, so lanes wait for their turn):
+// 8 M hits 0.70 -> 1.29 ms, so windows are taken in order.
+//
+// Cells outside a window score 0 and so change no Kadane maximum: guard bytes and padding of the staged rows,
+// sentinel residues past a target; with MASK the first and last vectors' bytes outside the window are replaced by
+// the sentinel.  u = max(cur, 0) is carried instead of cur: u' = max(u + s, 0) is one operation, and
+// max(best, cur) = max(best, u) since best >= 0; int8 scores over at most 2^20 rows cannot overflow, so the
+// unwrapped add equals the reference's wrapping one.  Rows outside int8 read the int32 profile with a window test.
+struct DiagWindow {
+  const uint8_t* target;
+  int32_t diag;
+  int32_t p0, p1;  // target positions; empty when p1 <= p0
+};
+
+// Byte mask of a 16-byte vector: 0xFF for the bytes i with lo <= i < hi.
+__device__ __forceinline__ void diag_window_mask(int32_t lo, int32_t hi, uint32_t m[4]) {
+  const uint32_t bits = ((1u << hi) - 1u) & ~((1u << lo) - 1u);  // 0 <= lo < hi <= 16
+#pragma unroll
+  for (int j = 0; j < 4; ++j) m[j] = (((bits >> (4 * j)) & 0xFu) * 0x00204081u & 0x01010101u) * 0xFFu;
+}
+
+// Scores windows 0 .. nb-1 of the run into out[]; window(j): the window.  Called by the whole CTA with *next =
+// blockDim.x; base = the staged profile (16 guard bytes before it).
+template <bool MASK, class Window>
+__device__ __forceinline__ void diag_score_run(const int8_t* base, uint32_t stride, bool narrow, const int32_t* p32,
+                                               int32_t s32, int32_t last_row, uint32_t nb, uint32_t* next,
+                                               int32_t* out, Window&& window) {
+  uint32_t k = 0;
+  DiagWindow w{nullptr, 0, 0, 0};
+  int32_t pa = 0, cur = 0, best = 0;
+  uint4 vnext = make_uint4(0, 0, 0, 0);  // the lane's next target vector, requested a step ahead
+  bool live = false;
+  auto take = [&](uint32_t j) {
+    k = j;
+    live = j < nb;
+    if (live) {
+      w = window(j);
+      cur = 0;
+      best = 0;
+      pa = w.p0 & ~15;
+      if (w.p1 > w.p0)
+        vnext = *reinterpret_cast<const uint4*>(w.target + pa);
+      else
+        pa = w.p1;  // empty: done at once
+    }
+  };
+  take(threadIdx.x);
+  while (__any_sync(0xFFFFFFFFu, live)) {
+    if (live) {
+      if (pa < w.p1) {
+        // the vector loaded one step ago; the next one is requested before this one is scored
+        const uint4 v = vnext;
+        if (pa + 16 < w.p1) vnext = *reinterpret_cast<const uint4*>(w.target + pa + 16);
+        uint32_t t[4] = {v.x, v.y, v.z, v.w};
+        const int32_t qa = pa - w.diag;
+        if (narrow) {
+          if (MASK && (pa < w.p0 || pa + 16 > w.p1)) {  // a window end inside this vector
+            uint32_t m[4];
+            diag_window_mask(max(w.p0 - pa, 0), min(w.p1 - pa, 16), m);
+#pragma unroll
+            for (int j = 0; j < 4; ++j) t[j] = (t[j] & m[j]) | (0x15151515u & ~m[j]);
+          }
+          const int8_t* rowbase = base + qa;
+#pragma unroll
+          for (int b = 0; b < 16; b += 2) {
+            const uint32_t r0 = (t[b >> 2] >> ((b & 3) * 8)) & 0xFFu;
+            const uint32_t r1 = (t[b >> 2] >> (((b + 1) & 3) * 8)) & 0xFFu;
+            const int32_t u0 =
+                __viaddmax_s32_relu(cur, static_cast<int32_t>(rowbase[static_cast<int32_t>(r0 * stride) + b]), 0);
+            cur = __viaddmax_s32_relu(u0, static_cast<int32_t>(rowbase[static_cast<int32_t>(r1 * stride) + b + 1]), 0);
+            best = __vimax3_s32(best, u0, cur);
+          }
+        } else {
+#pragma unroll
+          for (int b = 0; b < 16; ++b) {
+            const uint32_t r = (t[b >> 2] >> ((b & 3) * 8)) & 0xFFu;
+            const int32_t p = pa + b;
+            const int32_t row = min(max(qa + b, 0), last_row);
+            const int32_t sc = (p >= w.p0 && p < w.p1) ? __ldg(p32 + static_cast<int32_t>(r) * s32 + row) : 0;
+            cur = wadd(max(cur, 0), sc);
+            best = max(best, cur);
+          }
+        }
+        pa += 16;
+      }
+      if (pa >= w.p1) {
+        out[k] = best;
+        take(atomicAdd(next, 1u));
+      }
+    }
+  }
+  __syncthreads();
+}
+
+// Stages query q's int8 profile: rows 0..21 of `stride` bytes at smem + 16, zero past the stored rows, and the guard
+// bytes before row 0.  Called by the whole CTA; the caller synchronises.
+__device__ __forceinline__ void diag_stage(const DeviceProfiles& prof, uint32_t q, uint32_t stride, int8_t* smem) {
+  const uint32_t pstride = prof.stride8[q];
+  const int8_t* src = prof.p8[q];
+  for (uint32_t idx = threadIdx.x; idx < kProfRows * (stride / 16); idx += blockDim.x) {
+    const uint32_t r = idx / (stride / 16);
+    const uint32_t i = (idx - r * (stride / 16)) * 16;
+    uint4 v = make_uint4(0, 0, 0, 0);
+    if (i < pstride) v = *reinterpret_cast<const uint4*>(src + static_cast<size_t>(r) * pstride + i);
+    *reinterpret_cast<uint4*>(smem + 16 + static_cast<size_t>(r) * stride + i) = v;
+  }
+  if (threadIdx.x < 16) smem[threadIdx.x] = 0;
+}
+
+// Hits (whole-diagonal windows, diag_range): a CTA takes a chunk of hits, sorted by query as the prefilter produces
+// them, and scores each run of one query inside it with diag_score_run.
 __global__ void __launch_bounds__(256) ungapped_hits_refill_kernel(const UngappedParams prm) {
   extern __shared__ __align__(16) int8_t smem[];
-  __shared__ unsigned long long s_run_end;
-  __shared__ uint32_t s_next;
+  __shared__ uint32_t s_run_end, s_next;
   const HitRec* hits = reinterpret_cast<const HitRec*>(prm.jobs);
   const uint32_t stride = prm.max_m_pad;
-  int8_t* base = smem + 16;
-  const uint64_t c0 = static_cast<uint64_t>(blockIdx.x) * kUngChunk;
+  const uint64_t c0 = static_cast<uint64_t>(blockIdx.x) * prm.chunk;
   if (c0 >= prm.n) return;
-  const uint64_t c1 = u64min(prm.n, c0 + kUngChunk);
-  uint64_t a = c0;
-  while (a < c1) {
-    const uint32_t q = hits[a].query;
+  const uint32_t nc = static_cast<uint32_t>(u64min(prm.n - c0, prm.chunk));
+  const HitRec* chunk = hits + c0;
+  uint32_t a = 0;
+  while (a < nc) {
+    const uint32_t q = chunk[a].query;
     if (threadIdx.x < 32) {
-      uint64_t e = a;
+      uint32_t e = a;
       for (;;) {
-        const uint64_t k = e + threadIdx.x;
-        const bool same = (k < c1) && (hits[k].query == q);
-        const uint32_t ball = __ballot_sync(0xFFFFFFFFu, same);
+        const uint32_t k = e + threadIdx.x;
+        const uint32_t ball = __ballot_sync(0xFFFFFFFFu, k < nc && chunk[k].query == q);
         if (ball != 0xFFFFFFFFu) {
           e += __ffs(~ball) - 1;
           break;
@@ -220,100 +330,28 @@ __global__ void __launch_bounds__(256) ungapped_hits_refill_kernel(const Ungappe
         s_next = blockDim.x;
       }
     }
-    const uint32_t m = prm.prof.qlen[q];
-    const uint32_t pstride = prm.prof.stride8[q];
-    const int8_t* src = prm.prof.p8[q];
-    for (uint32_t idx = threadIdx.x; idx < kProfRows * (stride / 16); idx += blockDim.x) {
-      const uint32_t r = idx / (stride / 16);
-      const uint32_t i = (idx - r * (stride / 16)) * 16;
-      uint4 v = make_uint4(0, 0, 0, 0);
-      if (i < pstride) v = *reinterpret_cast<const uint4*>(src + static_cast<size_t>(r) * pstride + i);
-      *reinterpret_cast<uint4*>(base + static_cast<size_t>(r) * stride + i) = v;
-    }
-    if (threadIdx.x < 16) smem[threadIdx.x] = 0;
+    diag_stage(prm.prof, q, stride, smem);
     __syncthreads();
-    const uint64_t b = s_run_end;
-    const uint32_t nb = static_cast<uint32_t>(b - a);  // hits of the run, indexed from a
-    const HitRec* run = hits + a;
-    const bool narrow = prm.prof.fits8[q] != 0;
-    const int32_t* p32 = prm.prof.p32[q];
-    const int32_t s32 = static_cast<int32_t>(prm.prof.stride32[q]);
-    const int32_t last_row = static_cast<int32_t>(m) - 1;
-    uint32_t k = threadIdx.x;
-    const uint8_t* tp = nullptr;
-    int32_t d = 0, p0 = 0, p1 = 0, pa = 0, cur = 0, best = 0;
-    uint4 vnext = make_uint4(0, 0, 0, 0);  // the lane's next target vector, requested a step ahead
-    bool live = false;
-    auto take = [&](uint32_t j) {
-      k = j;
-      live = j < nb;
-      if (live) {
-        const HitRec h = run[j];
-        const int64_t n = prm.db.length[h.target];
-        d = h.diag;
-        // diag_range, src/ungapped.rs:38-46
-        const int64_t lo = i64max(-static_cast<int64_t>(d), 0), hi = i64min(m, n - d);
-        tp = prm.db.arena + prm.db.offset[h.target];
-        if (hi > lo) {
-          p0 = static_cast<int32_t>(lo) + d;
-          p1 = static_cast<int32_t>(hi) + d;
-          pa = p0 & ~15;
-          vnext = *reinterpret_cast<const uint4*>(tp + pa);
-        } else {
-          p0 = p1 = pa = 0;  // empty: done at once
-        }
-        cur = 0;
-        best = 0;
-      }
-    };
-    take(k);
-    while (__any_sync(0xFFFFFFFFu, live)) {
-      if (live) {
-        if (pa < p1) {
-          // the vector loaded one step ago; the next one is requested before this one is scored
-          const uint4 v = vnext;
-          if (pa + 16 < p1) vnext = *reinterpret_cast<const uint4*>(tp + pa + 16);
-          const uint32_t w[4] = {v.x, v.y, v.z, v.w};
-          const int32_t qa = pa - d;
-          if (narrow) {
-            // u = max(cur, 0) carried instead of cur: u' = max(u + s, 0) is one DPX op, and
-            // max(best, cur) = max(best, u) since best >= 0; int8 scores over at most 2^20 rows
-            // cannot overflow, so the unwrapped add equals the reference's wrapping one
-            const int8_t* rowbase = base + qa;
-#pragma unroll
-            for (int bb = 0; bb < 16; bb += 2) {
-              const uint32_t r0 = (w[bb >> 2] >> ((bb & 3) * 8)) & 0xFFu;
-              const uint32_t r1 = (w[bb >> 2] >> (((bb + 1) & 3) * 8)) & 0xFFu;
-              const int32_t u0 =
-                  __viaddmax_s32_relu(cur, static_cast<int32_t>(rowbase[static_cast<int32_t>(r0 * stride) + bb]), 0);
-              cur = __viaddmax_s32_relu(u0, static_cast<int32_t>(rowbase[static_cast<int32_t>(r1 * stride) + bb + 1]),
-                                        0);
-              best = __vimax3_s32(best, u0, cur);
-            }
-          } else {
-#pragma unroll
-            for (int bb = 0; bb < 16; ++bb) {
-              const uint32_t r = (w[bb >> 2] >> ((bb & 3) * 8)) & 0xFFu;
-              const int32_t p = pa + bb;
-              const int32_t row = min(max(qa + bb, 0), last_row);
-              const int32_t sc = (p >= p0 && p < p1) ? __ldg(p32 + static_cast<int32_t>(r) * s32 + row) : 0;
-              cur = wadd(max(cur, 0), sc);
-              best = max(best, cur);
-            }
+    const uint32_t b = s_run_end;
+    const HitRec* run = chunk + a;
+    const int32_t m = static_cast<int32_t>(prm.prof.qlen[q]);
+    diag_score_run<false>(
+        smem + 16, stride, prm.prof.fits8[q] != 0, prm.prof.p32[q], static_cast<int32_t>(prm.prof.stride32[q]), m - 1,
+        b - a, &s_next, prm.out + c0 + a, [&](uint32_t j) {
+          const HitRec h = run[j];
+          const int64_t n = prm.db.length[h.target];
+          // diag_range, src/ungapped.rs:38-46
+          const int64_t lo = i64max(-static_cast<int64_t>(h.diag), 0), hi = i64min(m, n - h.diag);
+          DiagWindow w{prm.db.arena + prm.db.offset[h.target], h.diag, 0, 0};
+          if (hi > lo) {
+            w.p0 = static_cast<int32_t>(lo) + h.diag;
+            w.p1 = static_cast<int32_t>(hi) + h.diag;
           }
-          pa += 16;
-        }
-        if (pa >= p1) {
-          prm.out[a + k] = best;
-          take(atomicAdd(&s_next, 1u));
-        }
-      }
-    }
-    __syncthreads();
+          return w;
+        });
     a = b;
   }
 }
-
 
 // Hits with the work of a query run split evenly over the CTA's lanes.
 //
