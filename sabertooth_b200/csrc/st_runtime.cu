@@ -6,6 +6,7 @@
 #include <omp.h>
 
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstdarg>
 #include <cstdio>
@@ -329,7 +330,7 @@ struct st_ctx {
   cudaStream_t plan_s = nullptr;  // profile builds and the device planner, beside kernels still queued
   cudaEvent_t plan_ev = nullptr;  // the end of a device plan's preparation on plan_s
   std::recursive_mutex mu;
-  uint64_t launches = 0;
+  std::atomic<uint64_t> launches{0};
   // database
   DevMem db_arena, db_off, db_len;
   std::vector<uint32_t> h_db_len;
@@ -373,7 +374,7 @@ struct st_ctx {
   // st_sw_score calls in flight: slots handed out under call_mu (not the context lock)
   static constexpr size_t kMaxCallSlots = 32;
   std::mutex call_mu;
-  std::shared_mutex call_rw;  // held shared by per-call scorings from their checks to their launches
+  std::shared_mutex call_rw;  // held shared by per-call scorings from their checks to their results
   uint64_t prof_epoch = 1;    // changes whenever profile layouts or tables are (re)written on the streams
   std::condition_variable call_cv;
   std::vector<std::unique_ptr<CallSlot>> call_slots;
@@ -2974,9 +2975,9 @@ extern "C" int st_sw_align_span_pairs(st_ctx* c, const st_pair* pairs, uint64_t 
 // checks, the profile tables, the sizes, the slot's buffers (device memory is accounted to the context) and,
 // when profiles changed since the slot's last call, the event that orders the call after the context
 // stream's work so far.  sw_score_launch runs outside it, on the slot's own stream: the staged inputs, the
-// copy and the launches.  Between the two the call holds the context's call lock shared, so the profile
-// tables it captured cannot be reallocated under it (table growth takes that lock exclusively, then waits
-// for the calls' streams).
+// copy and the launches.  From its checks to its result the call holds the context's call lock shared, so the
+// profile tables it captured cannot be reallocated under it (table growth takes that lock exclusively; it holds
+// the context lock then, so no further call begins meanwhile).
 struct SwCall {
   uint32_t profile = 0, n = 0, k = 0, P = 1, rows = 0, ncols = 0, sstride = 0;
   int32_t open = 0, ext = 0;
@@ -3056,8 +3057,39 @@ static int sw_score_prepare(st_ctx* c, CallSlot* sl, uint32_t profile, uint32_t 
     ST_CUDA(cudaEventRecord(sl->ev_in, c->stream));
     sl->epoch = c->prof_epoch;
   }
-  c->launches += w->use16 ? 2 : 1;
+  ++c->launches;
   *launch = true;
+  return ST_OK;
+}
+
+// The call's pair on the exact 32-bit kernel, on the slot's stream behind whatever was launched for it: a pair that is
+// not 16-bit eligible, or one that the packed kernel found above its headroom and put into the list (it then left the
+// kernel tag unwritten).  Launched for those only: an empty launch behind every packed one was 4 us of a call's 67.
+static int sw_score_launch32(CallSlot* sl, const SwCall& w) {
+  char* d = sl->stage.as<char>();
+  uint32_t* d_cnt = reinterpret_cast<uint32_t*>(d + w.o_cnt);
+  int32_t* h_res = sl->pin.as<int32_t>(w.total);
+  Sw32Params p32;
+  p32.db.arena = reinterpret_cast<const uint8_t*>(d);
+  p32.db.offset = reinterpret_cast<const uint64_t*>(d + w.o_off);
+  p32.db.length = reinterpret_cast<const uint32_t*>(d + w.o_len);
+  p32.db.n_seqs = 1;
+  p32.prof = w.pv;
+  p32.list = reinterpret_cast<const uint32_t*>(d + w.o_list);
+  p32.list_count = d_cnt + kNumClasses + 1;
+  p32.pair_query = reinterpret_cast<const uint32_t*>(d + w.o_pq);
+  p32.pair_target = reinterpret_cast<const uint32_t*>(d + w.o_pt);
+  p32.pair_center = reinterpret_cast<const int32_t*>(d + w.o_pc);
+  p32.pair_radius = reinterpret_cast<const int32_t*>(d + w.o_pr);
+  p32.scores = h_res;
+  p32.kernels = reinterpret_cast<uint32_t*>(h_res + 1);
+  p32.work_counter = d_cnt + kNumClasses;
+  p32.scratch = reinterpret_cast<int2*>(sl->scratch.p);
+  p32.scratch_stride = static_cast<uint32_t>(up16(w.n) + 32);
+  p32.open = w.open;
+  p32.ext = w.ext;
+  sw32_kernel<kWarps32><<<1, kWarps32 * 32, 0, sl->s>>>(p32);
+  ST_CUDA(cudaGetLastError());
   return ST_OK;
 }
 
@@ -3094,11 +3126,6 @@ static int sw_score_launch(CallSlot* sl, const uint8_t* target, const SwCall& w,
   cudaStream_t st = sl->s;
   if (w.wait) ST_CUDA(cudaStreamWaitEvent(st, sl->ev_in, 0));
   ST_CUDA(cudaMemcpyAsync(d, h, w.total, cudaMemcpyHostToDevice, st));
-  DeviceDb db;
-  db.arena = reinterpret_cast<const uint8_t*>(d);
-  db.offset = reinterpret_cast<const uint64_t*>(d + w.o_off);
-  db.length = reinterpret_cast<const uint32_t*>(d + w.o_len);
-  db.n_seqs = 1;
   uint32_t* d_cnt = reinterpret_cast<uint32_t*>(d + w.o_cnt);
   int32_t* d_score = h_res;
   uint32_t* d_kern = reinterpret_cast<uint32_t*>(h_res + 1);
@@ -3122,24 +3149,7 @@ static int sw_score_launch(CallSlot* sl, const uint8_t* target, const SwCall& w,
     prm.ext = w.ext;
     kClasses[w.k].fn<<<1, kClasses[w.k].W * 32, kProfRows * w.P * w.rows, st>>>(prm);
   }
-  // the 32-bit kernel scores the pair only when it is in the list (headroom reached, or not 16-bit eligible)
-  Sw32Params p32;
-  p32.db = db;
-  p32.prof = w.pv;
-  p32.list = d_list;
-  p32.list_count = d_cnt + kNumClasses + 1;
-  p32.pair_query = reinterpret_cast<const uint32_t*>(d + w.o_pq);
-  p32.pair_target = reinterpret_cast<const uint32_t*>(d + w.o_pt);
-  p32.pair_center = reinterpret_cast<const int32_t*>(d + w.o_pc);
-  p32.pair_radius = reinterpret_cast<const int32_t*>(d + w.o_pr);
-  p32.scores = d_score;
-  p32.kernels = d_kern;
-  p32.work_counter = d_cnt + kNumClasses;
-  p32.scratch = reinterpret_cast<int2*>(sl->scratch.p);
-  p32.scratch_stride = static_cast<uint32_t>(up16(n) + 32);
-  p32.open = w.open;
-  p32.ext = w.ext;
-  sw32_kernel<kWarps32><<<1, kWarps32 * 32, 0, st>>>(p32);
+  if (!w.use16) ST_TRY(sw_score_launch32(sl, w));
   ST_CUDA(cudaGetLastError());
   ST_CUDA(cudaEventRecord(sl->ev_done, st));
   return ST_OK;
@@ -3157,7 +3167,7 @@ extern "C" int st_sw_score(st_ctx* c, uint32_t profile, const uint8_t* target, u
   bool launch = false, queued = false;
   size_t res_off = 0;
   int rc;
-  std::shared_lock<std::shared_mutex> tables;  // the profile tables stay while this call's work is enqueued
+  std::shared_lock<std::shared_mutex> tables;  // the profile tables stay while this call runs
   {
     std::lock_guard<std::recursive_mutex> lk(c->mu);
     rc = cudaSetDevice(c->device) == cudaSuccess ? ST_OK : fail(ST_ECUDA, "cudaSetDevice(%d) failed", c->device);
@@ -3168,10 +3178,17 @@ extern "C" int st_sw_score(st_ctx* c, uint32_t profile, const uint8_t* target, u
     rc = sw_score_launch(sl, target, w, &res_off);
     queued = rc == ST_OK;
   }
-  if (tables.owns_lock()) tables.unlock();
   if (queued) {
-    const cudaError_t e = cudaEventSynchronize(sl->ev_done);
-    if (e != cudaSuccess) {
+    cudaError_t e = cudaEventSynchronize(sl->ev_done);
+    if (e == cudaSuccess && w.use16 && sl->pin.as<int32_t>(res_off)[1] == ST_KERNEL_NONE) {
+      // the packed kernel left the pair to the 32-bit one
+      ++c->launches;
+      rc = sw_score_launch32(sl, w);
+      e = cudaStreamSynchronize(sl->s);
+    }
+    if (rc != ST_OK) {
+      sl->epoch = 0;
+    } else if (e != cudaSuccess) {
       rc = fail(ST_ECUDA, "st_sw_score: %s", cudaGetErrorString(e));
     } else {
       const int32_t* res = sl->pin.as<int32_t>(res_off);
@@ -3183,6 +3200,7 @@ extern "C" int st_sw_score(st_ctx* c, uint32_t profile, const uint8_t* target, u
     cudaGetLastError();
     sl->epoch = 0;  // its stream may not have waited for the context stream: the next call waits again
   }
+  if (tables.owns_lock()) tables.unlock();  // held to here: a rescore launches with the same tables
   call_release(c, sl);
   return rc;
 }
