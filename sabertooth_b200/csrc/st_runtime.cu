@@ -1203,8 +1203,14 @@ struct ClassPlan {
   uint32_t scratch_stride = 0;
   uint64_t cells = 0;     // sum of m*n over this class's pairs
   uint64_t streamed = 0;  // cells the wavefront streams (padded rows x padded columns x slots)
+  double crit = 0;        // its longest critical path, picoseconds (tune_crit_ps)
   Sw16Params prm;
 };
+
+static double class_crit(int cls, uint32_t m_pad, uint32_t ncols) {
+  const Sw16Class& k = kClasses[cls];
+  return tune_crit_ps(k.G, k.R, k.C, m_pad / (k.G * k.R), ncols, k.team ? k.W : 1);
+}
 
 struct st_plan {
   st_ctx* ctx = nullptr;
@@ -1221,6 +1227,7 @@ struct st_plan {
   uint64_t cells = 0;
   uint64_t cells32 = 0;  // cells of pairs sent to the 32-bit kernel at plan time (band cells for bands)
   uint64_t streamed = 0;  // cells streamed by the 16-bit classes
+  double batch_ps = 0;    // the chip's time for them, every query in its cheapest class
   uint32_t kernels_per_run = 0;
   Sw32Params p32;
   cudaGraph_t graph = nullptr;
@@ -1295,8 +1302,14 @@ static int plan_enqueue(st_plan* p, cudaStream_t st, st_ctx::ForkSet* fs, bool g
     if (graph) {
       std::stable_partition(order, order + nc, [&](size_t i) { return i != big; });
     } else {
-      std::stable_sort(order, order + nc,
-                       [&](size_t a, size_t b) { return p->classes[a].cells > p->classes[b].cells; });
+      // a small batch waits for its longest wavefront: the class with the longest first
+      double crit = 0;
+      for (const auto& cp : p->classes) crit = std::max(crit, cp.crit);
+      const bool small = 3.0 * crit > p->batch_ps;
+      std::stable_sort(order, order + nc, [&](size_t a, size_t b) {
+        const ClassPlan &x = p->classes[a], &y = p->classes[b];
+        return small ? x.crit > y.crit : x.cells > y.cells;
+      });
       big = order[0];
     }
     if (cudaEventRecord(fs->ev[0], st) != cudaSuccess) return ST_ECUDA;
@@ -1544,6 +1557,7 @@ static int plan_build(st_ctx* c, const st_pair* pairs, uint64_t n, int32_t open,
                                 class_mask(ends));
   }
   int toolong = -1;
+  double class_path[kNumClasses] = {};
   for (size_t k = 0; k < qlist.size(); ++k) {
     const uint32_t q = qlist[k];
     const uint32_t m = c->profs[q].m;
@@ -1556,7 +1570,9 @@ static int plan_build(st_ctx* c, const st_pair* pairs, uint64_t n, int32_t open,
     if (static_cast<uint64_t>(kProfRows) * P * rows > static_cast<uint64_t>(g_class_smem[cls]))
       toolong = static_cast<int>(m);
     qclass[k] = cls;
+    class_path[cls] = std::max(class_path[cls], class_crit(cls, P * rows, std::max<uint32_t>(32, up4(tlen[byq[qstart[q]]]))));
   }
+  plan->batch_ps = batch_ps;
   if (toolong >= 0) return fail(ST_EINVAL, "query of %d rows does not fit the shared-memory profile", toolong);
   tc.lap("sort+pick");
   std::vector<ClassPlan> cps(kNumClasses);
@@ -1838,6 +1854,7 @@ static int plan_build(st_ctx* c, const st_pair* pairs, uint64_t n, int32_t open,
       kept.scratch_stride = cp.scratch_stride;
       kept.cells = cp.cells;
       kept.streamed = cp.streamed;
+      kept.crit = class_path[cp.cls];
       kept.o_cta = cp.o_cta;
       kept.o_wt = cp.o_wt;
       kept.o_slots = cp.o_slots;
@@ -2283,10 +2300,12 @@ static int dplan_build(st_ctx* c, const st_pair* pairs, uint64_t n, int32_t open
     ST_TRY(occupancy_grid(c, reinterpret_cast<const void*>(kClasses[k].fn), kClasses[k].W * 32, cp.smem,
                           tot.n_cta[k], &cp.grid));
     cp.scratch_stride = tot.max_cols_multi[k];
+    cp.crit = class_crit(k, tot.max_mpad[k], tot.max_cols[k]);
     plan->classes.push_back(std::move(cp));
   }
   plan->scratch32_stride = max_m > static_cast<uint32_t>(kSw32Rows) ? max_len : 0;
   plan->n_static32 = n_list32;
+  plan->batch_ps = static_cast<double>(tot.batch_ps);
   ST_TRY(grid_sw32(c, n_list32, n, plan->scratch32_stride, &plan->grid32));
   size_t t_lpt = 0;
   {
