@@ -4183,7 +4183,12 @@ static void swap_db(st_ctx* c, DbState& s) {
 }
 
 // fit_gumbel_ml and gumbel_mu_given_lambda (src/evalue.rs:129-182) in binary64
-// with the reference's summation order (index order).
+// with the reference's summation order (index order).  The bisection needs only
+// the sign of the likelihood's derivative: away from the root it is taken from
+// sums over the distinct scores (a few hundred integers at most, against
+// thousands of samples, each an exponential), and only where that value is
+// within reach of rounding from the index-order sums, so every step decides as
+// they do.
 static double gumbel_mu_given_lambda(const std::vector<double>& xs, double lambda) {
   double xmin = INFINITY;
   for (double x : xs) xmin = std::fmin(xmin, x);
@@ -4192,7 +4197,11 @@ static double gumbel_mu_given_lambda(const std::vector<double>& xs, double lambd
   return xmin - std::log(s / static_cast<double>(xs.size())) / lambda;
 }
 
-static bool fit_gumbel_ml(const std::vector<double>& xs, double* lambda, double* mu) {
+struct ScoreCounts {
+  std::vector<double> x, c;  // ascending scores, how often each occurs
+};
+
+static bool fit_gumbel_ml(const std::vector<double>& xs, const ScoreCounts& d, double* lambda, double* mu) {
   const size_t n = xs.size();
   if (n < 10) return false;
   double sum = 0.0;
@@ -4202,10 +4211,18 @@ static bool fit_gumbel_ml(const std::vector<double>& xs, double* lambda, double*
   for (double x : xs) ss += (x - mean) * (x - mean);
   const double var = ss / (static_cast<double>(n) - 1.0);
   if (std::isnan(var) || var <= 0.0) return false;
-  double xmin = INFINITY;
-  for (double x : xs) xmin = std::fmin(xmin, x);
+  const double xmin = d.x[0];
   auto g = [&](double lam) {
     double s0 = 0.0, s1 = 0.0;
+    for (size_t i = 0; i < d.x.size(); ++i) {
+      const double w = d.c[i] * std::exp(-lam * (d.x[i] - xmin));
+      s0 += w;
+      s1 += d.x[i] * w;
+    }
+    const double near = 1.0 / lam - mean + s1 / s0;
+    // both forms' rounding is some 1e-15 of their largest term (n terms of one sign a sum)
+    if (std::fabs(near) > 1e-9 * (1.0 / lam + std::fabs(mean) + std::fabs(s1 / s0))) return near;
+    s0 = s1 = 0.0;
     for (double x : xs) {
       const double w = std::exp(-lam * (x - xmin));
       s0 += w;
@@ -4280,10 +4297,20 @@ extern "C" int st_calibrate_profiles(st_ctx* c, const uint32_t* profiles, uint32
   cal.n_seqs = samples;
   cal.has = true;
   const size_t arena_bytes = total + 32;
-  ST_TRY(dev_alloc(&c->mt, cal.arena, arena_bytes));
-  ST_TRY(dev_alloc(&c->mt, cal.off, off.size() * 8));
-  ST_TRY(dev_alloc(&c->mt, cal.len, static_cast<size_t>(samples) * 4));
+  // the samples' database and streams from the pool (an allocation and a release on every call otherwise)
   DevMem st_dev;
+  struct Back {  // every exit has waited for the stream or queued nothing
+    st_ctx* c;
+    DbState* db;
+    DevMem* st;
+    ~Back() {
+      for (DevMem* m : {&db->arena, &db->off, &db->len, st})
+        if (m->p) pool_put_after(c, std::move(*m), c->stream);
+    }
+  } back{c, &cal, &st_dev};
+  ST_TRY(pool_get(c, arena_bytes, cal.arena));
+  ST_TRY(pool_get(c, off.size() * 8, cal.off));
+  ST_TRY(pool_get(c, static_cast<size_t>(samples) * 4, cal.len));
   ST_TRY(pool_get(c, static_cast<size_t>(samples) * 8, st_dev));
   ST_CUDA(cudaMemsetAsync(cal.arena.p, kSentinel, arena_bytes, c->stream));
   ST_CUDA(cudaMemcpyAsync(cal.off.p, off.data(), off.size() * 8, cudaMemcpyHostToDevice, c->stream));
@@ -4315,11 +4342,25 @@ extern "C" int st_calibrate_profiles(st_ctx* c, const uint32_t* profiles, uint32
   auto fit_rows = [&](size_t r0, size_t r1) {
 #pragma omp parallel for schedule(dynamic, 1)
     for (int64_t r = static_cast<int64_t>(r0); r < static_cast<int64_t>(r1); ++r) {
-      std::vector<double> xs(samples);
-      for (uint32_t i = 0; i < samples; ++i) xs[i] = static_cast<double>(sc[static_cast<size_t>(r) * samples + i]);
+      thread_local std::vector<int32_t> sorted;
+      thread_local std::vector<double> xs;
+      thread_local ScoreCounts counts;
+      const int32_t* x = sc.data() + static_cast<size_t>(r) * samples;
+      xs.assign(x, x + samples);
+      sorted.assign(x, x + samples);
+      std::sort(sorted.begin(), sorted.end());
+      counts.x.clear();
+      counts.c.clear();
+      for (uint32_t i = 0; i < samples;) {
+        uint32_t j = i;
+        while (j < samples && sorted[j] == sorted[i]) ++j;
+        counts.x.push_back(sorted[i]);
+        counts.c.push_back(j - i);
+        i = j;
+      }
       double lambda = 0.0, mu = 0.0;
       st_calibration& o = out[row[r]];
-      if (fit_gumbel_ml(xs, &lambda, &mu)) {
+      if (fit_gumbel_ml(xs, counts, &lambda, &mu)) {
         o.lambda = lambda;
         o.mu = mu;
         o.k = std::exp(lambda * (mu + 0.5)) / (static_cast<double>(m[row[r]]) * mean_len);
@@ -4354,7 +4395,6 @@ extern "C" int st_calibrate_profiles(st_ctx* c, const uint32_t* profiles, uint32
     if (h) st_batch_wait(h);
   swap_db(c, cal);
   ST_CUDA(cudaStreamSynchronize(c->stream));
-  pool_put(c, std::move(st_dev));
   if (rc != ST_OK) return rc;
   if (scores) {
     memset(scores, 0, static_cast<size_t>(n_profiles) * samples * 4);
