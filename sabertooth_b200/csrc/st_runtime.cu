@@ -3548,6 +3548,9 @@ static int gate_conf(st_ctx* c, const st_prefilter_params* p, GateConf& g, int& 
   if (qbits + static_cast<int>(g.tbits + g.dbits) > 64 || qbits > 32)
     return fail(ST_EINVAL, "seed-hit key needs %d bits (query %d, target %u, diagonal %u); at most 64",
                 qbits + static_cast<int>(g.tbits + g.dbits), qbits, g.tbits, g.dbits);
+  // a hit's query position is below the longest query's length; it rides in the key where there is room
+  const int pbits = bits_for(c->max_m ? c->max_m - 1 : 0);
+  g.pbits = qbits + static_cast<int>(g.tbits + g.dbits) + pbits <= 64 ? static_cast<uint32_t>(pbits) : 0u;
   g.stride = ung_stride(c);
   if (16 + static_cast<size_t>(kProfRows) * g.stride + 16 > static_cast<size_t>(g_gate_smem))
     return fail(ST_EINVAL, "query too long for the prefilter segment kernel (%u rows)", c->max_m);
@@ -3579,7 +3582,10 @@ static int gate_pipeline(st_ctx* c, const GateSeedHit* d_hits, uint32_t n, const
   {
     cub::DoubleBuffer<uint64_t> kb(nullptr, nullptr);
     cub::DoubleBuffer<uint32_t> vb(nullptr, nullptr);
-    ST_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, t, kb, vb, n, 0, key_bits, c->stream));
+    if (g.pbits)
+      ST_CUDA(cub::DeviceRadixSort::SortKeys(nullptr, t, kb, n, g.pbits, g.pbits + key_bits, c->stream));
+    else
+      ST_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, t, kb, vb, n, 0, key_bits, c->stream));
     t_max = std::max(t_max, t);
     ST_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, t, kb, vb, n, 0, 31 + qbits, c->stream));
     t_max = std::max(t_max, t);
@@ -3644,12 +3650,15 @@ static int gate_pipeline(st_ctx* c, const GateSeedHit* d_hits, uint32_t n, const
   cub::DoubleBuffer<uint64_t> kb(k0, k1);
   cub::DoubleBuffer<uint32_t> vb(v0, v1);
   t = t_max;
-  ST_CUDA(cub::DeviceRadixSort::SortPairs(tmp, t, kb, vb, n, 0, key_bits, s));
+  if (g.pbits)
+    ST_CUDA(cub::DeviceRadixSort::SortKeys(tmp, t, kb, n, g.pbits, g.pbits + key_bits, s));
+  else
+    ST_CUDA(cub::DeviceRadixSort::SortPairs(tmp, t, kb, vb, n, 0, key_bits, s));
   GateGroups G{kb.Current(), vb.Current(), start, ng, n};
   {
     cub::CountingInputIterator<uint32_t> it(0);
     cub::TransformInputIterator<bool, GateHeadFlag, cub::CountingInputIterator<uint32_t>> heads(
-        it, GateHeadFlag{kb.Current(), g.dbits});
+        it, GateHeadFlag{kb.Current(), g.dbits + g.pbits});
     t = t_max;
     ST_CUDA(cub::DeviceSelect::Flagged(tmp, t, it, heads, start, ng, n, s));
   }
