@@ -111,6 +111,13 @@ __device__ __forceinline__ int32_t gate_key_diag(uint64_t k, const GateConf& g) 
   return static_cast<int32_t>(static_cast<int64_t>((k >> g.pbits) & ((1ull << g.dbits) - 1)) - g.doff);
 }
 
+__device__ __forceinline__ uint64_t gate_key(uint32_t query, uint32_t target, int32_t diag, uint32_t qpos,
+                                             const GateConf& g) {
+  const uint64_t k = (static_cast<uint64_t>(query) << (g.tbits + g.dbits)) | (static_cast<uint64_t>(target) << g.dbits) |
+                     static_cast<uint64_t>(static_cast<int64_t>(diag) + g.doff);
+  return g.pbits ? (k << g.pbits) | qpos : k;
+}
+
 // Adds each thread's count to a counter; called by every thread of the block
 // once, after its loop (all 32 lanes of each warp present).
 __device__ __forceinline__ void gate_flush(unsigned long long* ctr, unsigned long long v) {
@@ -147,17 +154,8 @@ __global__ void __launch_bounds__(256) gate_keys_kernel(const GateSeedHit* hits,
       const int64_t tpos = static_cast<int64_t>(h.qpos) + h.diag;
       ok = h.qpos < qlen[h.query] && tpos >= 0 && tpos < static_cast<int64_t>(db.length[h.target]);
     }
-    uint64_t k = bad;
-    if (ok)
-      k = ((static_cast<uint64_t>(h.query) << (g.tbits + g.dbits)) | (static_cast<uint64_t>(h.target) << g.dbits) |
-           static_cast<uint64_t>(static_cast<int64_t>(h.diag) + g.doff))
-          << g.pbits;
-    if (g.pbits)
-      keys[i] = ok ? k | h.qpos : k;
-    else {
-      keys[i] = k;
-      vals[i] = h.qpos;
-    }
+    keys[i] = ok ? gate_key(h.query, h.target, h.diag, h.qpos, g) : bad;
+    if (!g.pbits) vals[i] = h.qpos;
     rejected += ok ? 0 : 1;
   }
   gate_flush(&st->hits_rejected, rejected);

@@ -3559,9 +3559,11 @@ static int gate_conf(st_ctx* c, const st_prefilter_params* p, GateConf& g, int& 
 
 // The whole pipeline on the context stream, one host synchronisation (the
 // number of candidates, which sizes the ranking sort) and a final one for the
-// counts.  Ranked candidates go to d_out (room for n entries).
-static int gate_pipeline(st_ctx* c, const GateSeedHit* d_hits, uint32_t n, const GateConf& g, int qbits,
-                         GateCandidate* d_out, uint64_t* n_out, GateStats* h_stats) {
+// counts.  Ranked candidates go to d_out (room for n entries).  Without d_hits
+// the hits come as their keys (positions inside) in d_keys, which is sort scratch
+// from then on.
+static int gate_pipeline(st_ctx* c, const GateSeedHit* d_hits, uint64_t* d_keys, uint32_t n, const GateConf& g,
+                         int qbits, GateCandidate* d_out, uint64_t* n_out, GateStats* h_stats) {
   const int key_bits = qbits + static_cast<int>(g.tbits + g.dbits);
   const size_t P = static_cast<size_t>(g.n_prof) + 1;
   size_t o = 0;
@@ -3570,7 +3572,7 @@ static int gate_pipeline(st_ctx* c, const GateSeedHit* d_hits, uint32_t n, const
     o += up256(std::max<size_t>(bytes, 1));
     return r;
   };
-  const size_t o_k0 = take(8ull * n), o_k1 = take(8ull * n), o_v0 = take(4ull * n), o_v1 = take(4ull * n);
+  const size_t o_k0 = take(d_hits ? 8ull * n : 0), o_k1 = take(8ull * n), o_v0 = take(4ull * n), o_v1 = take(4ull * n);
   const size_t o_start = take(4ull * n), o_ng = take(4), o_ns = take(4ull * (n + 1)), o_joff = take(4ull * (n + 1));
   const size_t o_jobs = take(sizeof(GateJob) * n), o_sc = take(4ull * n);
   const size_t o_cand = take(sizeof(GateCandidate) * n), o_flag = take(n), o_sel = take(4ull * n), o_nc = take(4);
@@ -3613,7 +3615,7 @@ static int gate_pipeline(st_ctx* c, const GateSeedHit* d_hits, uint32_t n, const
   } back{c, &mem};
   char* b = mem.as<char>();
   auto at = [&](size_t off) { return static_cast<void*>(b + off); };
-  uint64_t* k0 = static_cast<uint64_t*>(at(o_k0));
+  uint64_t* k0 = d_hits ? static_cast<uint64_t*>(at(o_k0)) : d_keys;
   uint64_t* k1 = static_cast<uint64_t*>(at(o_k1));
   uint32_t* v0 = static_cast<uint32_t*>(at(o_v0));
   uint32_t* v1 = static_cast<uint32_t*>(at(o_v1));
@@ -3646,7 +3648,10 @@ static int gate_pipeline(st_ctx* c, const GateSeedHit* d_hits, uint32_t n, const
   // keys, sort, groups
   DeviceDb db = db_view(c);
   DeviceProfiles pv = prof_view(c);
-  gate_keys_kernel<<<grid_for(n, 256), 256, 0, s>>>(d_hits, n, db, pv.qlen, g, k0, v0, st);
+  if (d_hits) {
+    gate_keys_kernel<<<grid_for(n, 256), 256, 0, s>>>(d_hits, n, db, pv.qlen, g, k0, v0, st);
+    ++c->launches;
+  }
   cub::DoubleBuffer<uint64_t> kb(k0, k1);
   cub::DoubleBuffer<uint32_t> vb(v0, v1);
   t = t_max;
@@ -3684,7 +3689,7 @@ static int gate_pipeline(st_ctx* c, const GateSeedHit* d_hits, uint32_t n, const
     t = t_max;
     ST_CUDA(cub::DeviceSelect::Flagged(tmp, t, it, flag, sel, nc, n, s));
   }
-  c->launches += 8;
+  c->launches += 7;
   ST_CUDA(cudaGetLastError());
   ST_TRY(c->pin.reserve(64));
   uint32_t* h_nc = c->pin.as<uint32_t>();
@@ -3751,7 +3756,7 @@ extern "C" int st_prefilter_gate_device(st_ctx* c, const st_seed_hit* d_hits, ui
   GateStats st{};
   *n_out = 0;
   if (n)
-    ST_TRY(gate_pipeline(c, reinterpret_cast<const GateSeedHit*>(d_hits), static_cast<uint32_t>(n), g, qbits,
+    ST_TRY(gate_pipeline(c, reinterpret_cast<const GateSeedHit*>(d_hits), nullptr, static_cast<uint32_t>(n), g, qbits,
                          reinterpret_cast<GateCandidate*>(d_out), n_out, &st));
   return gate_result(st, stats);
 }
@@ -3778,7 +3783,7 @@ extern "C" int st_prefilter_gate(st_ctx* c, const st_seed_hit* hits, uint64_t n,
     char* d = buf.as<char>();
     ST_TRY(upload_host(c, d, hits, n * sizeof(st_seed_hit), c->stream));
     GateCandidate* d_out = reinterpret_cast<GateCandidate*>(d + hb);
-    ST_TRY(gate_pipeline(c, reinterpret_cast<const GateSeedHit*>(d), static_cast<uint32_t>(n), g, qbits, d_out,
+    ST_TRY(gate_pipeline(c, reinterpret_cast<const GateSeedHit*>(d), nullptr, static_cast<uint32_t>(n), g, qbits, d_out,
                          n_out, &st));
     const uint64_t k = std::min<uint64_t>(cap, *n_out);
     if (k) {
@@ -3853,10 +3858,11 @@ extern "C" int st_seed_index_build(st_ctx* c, const char* mask) {
 
 // The seed stage for a batch of queries: hits (device, pooled in `hits`), their
 // count and the counters.  Two host synchronisations (seed slots, hits) size
-// the buffers.
+// the buffers.  With a gate configuration whose keys hold the positions the
+// hits are written as its keys.
 static int seed_stage(st_ctx* c, const uint32_t* profiles, uint32_t n_q, const uint8_t* residues,
                       const uint64_t* res_off, const st_seed_params* sp, DevMem& hits, uint32_t* n_hits,
-                      st_seed_stats* stats) {
+                      st_seed_stats* stats, const GateConf* keys = nullptr) {
   if (!sp) return fail(ST_EINVAL, "null seed parameters");
   if (sp->max_kmers_per_pos == 0) return fail(ST_EINVAL, "max_kmers_per_pos must be at least 1");
   if (!c->has_db) return fail(ST_ESTATE, "no target database uploaded (st_db_upload)");
@@ -4001,11 +4007,17 @@ static int seed_stage(st_ctx* c, const uint32_t* profiles, uint32_t n_q, const u
     return fail(ST_EINVAL, "%llu windows have a score range above %d histogram bins (rows too wide for the "
                 "device seed generator)", sd.errors, kSeedMaxBins);
   if (sd.postings_visited >= 0x7FFFFFFFull) return fail(ST_EINVAL, "too many seed hits in one call");
-  ST_TRY(pool_get(c, std::max<uint64_t>(nh, 1) * sizeof(GateSeedHit), hits));
+  const bool as_keys = keys && keys->pbits;
+  ST_TRY(pool_get(c, std::max<uint64_t>(nh, 1) * (as_keys ? sizeof(uint64_t) : sizeof(GateSeedHit)), hits));
   if (nh) {
-    seed_hits_kernel<<<grid_for(ns, 256), 256, 0, s>>>(Q, seeds, static_cast<uint32_t>(ns), cnt, hoff,
-                                                       c->seed_off.as<uint32_t>(), c->seed_post.as<SeedPost>(),
-                                                       hits.as<GateSeedHit>());
+    if (as_keys)
+      seed_hits_kernel<<<grid_for(ns, 256), 256, 0, s>>>(Q, seeds, static_cast<uint32_t>(ns), cnt, hoff,
+                                                         c->seed_off.as<uint32_t>(), c->seed_post.as<SeedPost>(),
+                                                         SeedHitKeys{hits.as<uint64_t>(), *keys});
+    else
+      seed_hits_kernel<<<grid_for(ns, 256), 256, 0, s>>>(Q, seeds, static_cast<uint32_t>(ns), cnt, hoff,
+                                                         c->seed_off.as<uint32_t>(), c->seed_post.as<SeedPost>(),
+                                                         SeedHitRecs{hits.as<GateSeedHit>()});
     ++c->launches;
     ST_CUDA(cudaGetLastError());
   }
@@ -4096,7 +4108,7 @@ extern "C" int st_prefilter_queries(st_ctx* c, const uint32_t* profiles, uint32_
     uint32_t nh = 0;
     st_seed_stats sst{};
     ST_TRY(seed_stage(c, cp.data(), q1 - q0, residues ? cres.data() : nullptr, residues ? coff.data() : nullptr,
-                      seed_params, hits, &nh, &sst));
+                      seed_params, hits, &nh, &sst, &gc));
     stot.windows += sst.windows;
     stot.windows_skipped += sst.windows_skipped;
     stot.kmers_generated += sst.kmers_generated;
@@ -4113,7 +4125,8 @@ extern "C" int st_prefilter_queries(st_ctx* c, const uint32_t* profiles, uint32_
       tc.lap("candidate buffer");
       GateStats st{};
       uint64_t nc = 0;
-      ST_TRY(gate_pipeline(c, hits.as<GateSeedHit>(), nh, gc, qbits, cm.as<GateCandidate>(), &nc, &st));
+      ST_TRY(gate_pipeline(c, gc.pbits ? nullptr : hits.as<GateSeedHit>(), hits.as<uint64_t>(), nh, gc, qbits,
+                           cm.as<GateCandidate>(), &nc, &st));
       tc.lap("gate");
       const size_t at = all.size();
       all.resize(at + nc);

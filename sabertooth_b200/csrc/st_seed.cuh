@@ -518,10 +518,26 @@ __global__ void __launch_bounds__(256) seed_post_count_kernel(const SeedSeed* se
 // contiguous range of the output; lane k writes output positions k, k + 32, ...
 // and finds the seed of each by a binary search over the 32 seeds' offsets held
 // in the lanes, so reads of the postings and writes of the hits are coalesced
-// whatever the list lengths.
+// whatever the list lengths.  Hits that only the evidence stage reads are
+// written as its sort keys: 8 bytes for 16, and no pass that makes keys of them
+// (a posting lies inside its target, so none is rejected).
+struct SeedHitRecs {
+  GateSeedHit* hits;
+  __device__ __forceinline__ void put(uint32_t k, uint32_t query, uint32_t target, int32_t diag, uint32_t qpos) const {
+    hits[k] = GateSeedHit{query, target, diag, qpos};
+  }
+};
+struct SeedHitKeys {
+  uint64_t* keys;
+  GateConf g;
+  __device__ __forceinline__ void put(uint32_t k, uint32_t query, uint32_t target, int32_t diag, uint32_t qpos) const {
+    keys[k] = gate_key(query, target, diag, qpos, g);
+  }
+};
+template <typename OUT>
 __global__ void __launch_bounds__(256) seed_hits_kernel(SeedQ Q, const SeedSeed* seeds, uint32_t n_seeds,
                                                         const uint32_t* cnt, const uint32_t* hoff, const uint32_t* off,
-                                                        const SeedPost* post, GateSeedHit* hits) {
+                                                        const SeedPost* post, const OUT out) {
   const uint32_t lane = threadIdx.x & 31;
   const uint32_t n_groups = (n_seeds + 31) / 32;
   for (uint32_t g = (blockIdx.x * blockDim.x + threadIdx.x) / 32; g < n_groups; g += (gridDim.x * blockDim.x) / 32) {
@@ -558,7 +574,7 @@ __global__ void __launch_bounds__(256) seed_hits_kernel(SeedQ Q, const SeedSeed*
       const uint32_t sj = __shfl_sync(0xFFFFFFFFu, start, j);
       if (live) {
         const SeedPost ps = post[pj + (k - oj)];
-        hits[k] = GateSeedHit{qj, ps.target, static_cast<int32_t>(ps.tpos) - static_cast<int32_t>(sj), sj};
+        out.put(k, qj, ps.target, static_cast<int32_t>(ps.tpos) - static_cast<int32_t>(sj), sj);
       }
     }
   }

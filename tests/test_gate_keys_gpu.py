@@ -9,7 +9,7 @@ import numpy as np
 import pytest
 
 from sabertooth_b200._lib import SEED_HIT_DTYPE
-from sabertooth_b200 import blosum62
+from sabertooth_b200 import PrefilterParams, blosum62
 from tests.seedhits import default_params
 from tests.test_gate_gpu import _check
 
@@ -65,3 +65,31 @@ def test_keys_with_and_without_positions(ctx, n_short, m_long, n_targets, t_long
     p["diag_window"] = window
     got, _ = _check(ctx, rows, targets, hits, p)
     assert len(got)
+
+
+@pytest.mark.parametrize("n_short,m_long,n_targets,t_long", [(299, 8300, 70000, 1 << 24), (3, 600, 500, 30000)])
+def test_search_from_records_and_from_keys(ctx, n_short, m_long, n_targets, t_long):
+    # the prefilter of a batch of queries equals its seed hits through the evidence call, whichever form the hits take
+    rng = np.random.default_rng(n_targets)
+    rows, targets, _ = _case(rng, n_short, m_long, n_targets, t_long)
+    m = blosum62()
+    pick = [0, 1, 2, n_short]
+    qs = [rng.integers(0, 20, len(rows[i])).astype(np.uint8) for i in pick[:-1]]
+    at = t_long - m_long
+    qs.append(targets[-1][at:at + m_long].copy())  # the long query is the far end of the long target
+    for i, q in zip(pick, qs):
+        rows[i] = m.sequence_rows(q)
+    ctx.upload_db_list(targets)
+    ids = ctx.create_profiles(rows)
+    try:
+        ctx.seed_index_build("111001101")
+        p = PrefilterParams(min_diag_score=43, span=9)
+        sel = ids[pick]
+        found, evidence, _ = ctx.prefilter_queries(sel, qs, p)
+        hits, _ = ctx.seed_hits(sel, qs, p)
+        want, counters = ctx.prefilter_gate(hits, p)
+        assert len(want) and len(hits) > len(want)
+        assert np.array_equal(found, want[np.argsort(want["query"], kind="stable")])
+        assert evidence == counters
+    finally:
+        ctx.free_profiles(ids)
