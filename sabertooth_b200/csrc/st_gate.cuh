@@ -31,7 +31,7 @@
 //            work list
 //   chain    one thread per listed group: best segment, best chain, gate,
 //            region, candidate slot + flag; kadane_segment positions only for
-//            the jobs a chain test or a region reads (the reference's pos_of)
+//            the jobs a chain test or a region may read (the reference's pos_of)
 //   compact  candidates in (query, target) order (CUB select)
 //   rank     stable radix sort by (query, 2^31 - 1 - score) keeps target order
 //            inside equal scores; per-query cut to max_candidates; gather
@@ -462,87 +462,137 @@ __global__ void __launch_bounds__(256) gate_screen_kernel(GateGroups G, GateConf
 // Best single segment (first maximum in job order) or best chain x -> y of two
 // co-linear segments (first maximum in (x, y) order), the gate and the region
 // (src/prefilter.rs:1577-1657, region :1269-1278), one thread per listed group.
-__global__ void __launch_bounds__(128) gate_chain_kernel(GateGroups G, GateConf g, DeviceDb db, DeviceProfiles prof,
-                                                         const uint32_t* joff, const GateJob* jobs,
-                                                         const int32_t* score, const uint32_t* work,
-                                                         const uint32_t* n_work, GateCandidate* cand, uint8_t* flag,
-                                                         GateStats* st) {
+// Segment positions decide only the pairs whose chain would beat the best single
+// segment, and the region: each thread marks the jobs it needs, the CTA packs
+// them and walks them one a thread, so that a warp walks 32 windows where the
+// threads' own few left most of its lanes waiting, and the scores and diagonals
+// of a group are read at once (14 M windows of 150 queries: 545 -> 275 us).
+template <int KMAX>
+constexpr int kChainThreads = KMAX <= 4 ? 256 : 128;  // 12 or 24 KB of shared memory a CTA
+template <int KMAX>
+__global__ void __launch_bounds__(kChainThreads<KMAX>) gate_chain_kernel(
+    GateGroups G, GateConf g, DeviceDb db, DeviceProfiles prof, const uint32_t* joff, const GateJob* jobs,
+    const int32_t* score, const uint32_t* work, const uint32_t* n_work, GateCandidate* cand, uint8_t* flag,
+    GateStats* st) {
+  constexpr uint32_t T = kChainThreads<KMAX>;
+  __shared__ uint32_t s_job[T * KMAX], s_warp[T / 32];
+  __shared__ int2 s_pos[T * KMAX];  // query positions of the first and last cell of the job's best segment
   const uint32_t ng = *G.n_groups;
   const uint32_t nw = *n_work;
+  const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   unsigned long long n_chained = 0;
-  for (uint32_t w = blockIdx.x * blockDim.x + threadIdx.x; w < nw; w += gridDim.x * blockDim.x) {
-    const uint32_t gi = work[w];
-    const uint32_t j0 = joff[gi], nsg = joff[gi + 1] - j0;
+  for (uint32_t w0 = blockIdx.x * T; w0 < nw; w0 += gridDim.x * T) {
+    const bool on = w0 + threadIdx.x < nw;
+    uint32_t gi = 0, j0 = 0, nsg = 0, bi = 0, need = 0;
     int32_t best = 0;
-    uint32_t bi = 0;
-    for (uint32_t k = 0; k < nsg; ++k) {
-      const int32_t sk = score[j0 + k];
-      if (sk > best) {
-        best = sk;
-        bi = k;
-      }
-    }
-    // segment positions, computed where a chain or a region needs them (as the reference's pos_of)
-    int32_t pqs[kGateMaxDiags], pqe[kGateMaxDiags];
-    uint32_t have = 0;
-    auto pos_of = [&](uint32_t x) {
-      if (!(have & (1u << x))) {
-        gate_kadane_segment(prof, db, jobs[j0 + x], pqs[x], pqe[x]);
-        have |= 1u << x;
-      }
-    };
-    int32_t chain = INT32_MIN;
-    uint32_t cx = 0, cy = 0;
-    if (nsg > 1) {
-      for (uint32_t x = 0; x < nsg; ++x) {
-        const int32_t sx = score[j0 + x];
+    int32_t seg[KMAX], dg[KMAX];  // the group's segment scores (0 past its last) and diagonals
+#pragma unroll
+    for (int k = 0; k < KMAX; ++k) seg[k] = dg[k] = 0;
+    // pair(x, y, c, dx, dy) for the ordered pairs whose chain score beats the best single segment
+    auto pairs = [&](auto&& pair) {
+#pragma unroll(KMAX <= 4 ? KMAX : 1)
+      for (uint32_t x = 0; x < KMAX; ++x) {
+        const int32_t sx = seg[x], dx = dg[x];
         if (sx <= 0) continue;
-        const int32_t dx = jobs[j0 + x].diag;
-        for (uint32_t y = 0; y < nsg; ++y) {
+#pragma unroll(KMAX <= 4 ? KMAX : 1)
+        for (uint32_t y = 0; y < KMAX; ++y) {
           if (x == y) continue;
-          const int32_t sy = score[j0 + y], dy = jobs[j0 + y].diag;
+          const int32_t sy = seg[y], dy = dg[y];
           if (sy <= 0 || dx == dy) continue;
           const uint32_t len = static_cast<uint32_t>(dy > dx ? dy - dx : dx - dy);
           const int32_t c = wsub(wadd(sx, sy), gate_gap_cost(g.open, g.ext, len));
-          if (c <= best || c <= chain) continue;
-          pos_of(x);
-          pos_of(y);
-          const int32_t qex = pqe[x], qsy = pqs[y];
+          if (c > best) pair(x, y, c, dx, dy);
+        }
+      }
+    };
+    if (on) {
+      gi = work[w0 + threadIdx.x];
+      j0 = joff[gi];
+      nsg = joff[gi + 1] - j0;
+#pragma unroll
+      for (uint32_t k = 0; k < KMAX; ++k)
+        if (k < nsg) {
+          seg[k] = score[j0 + k];
+          dg[k] = jobs[j0 + k].diag;
+        }
+#pragma unroll
+      for (uint32_t k = 0; k < KMAX; ++k)
+        if (seg[k] > best) {
+          best = seg[k];
+          bi = k;
+        }
+      if (nsg > 1) pairs([&](uint32_t x, uint32_t y, int32_t, int32_t, int32_t) { need |= 1u << x | 1u << y; });
+      if (g.regions && best >= g.min_score) need |= 1u << bi;
+    }
+    const uint32_t cnt = __popc(need);
+    uint32_t incl = cnt;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t v = __shfl_up_sync(0xFFFFFFFFu, incl, o);
+      if (lane >= o) incl += v;
+    }
+    if (lane == 31) s_warp[warp] = incl;
+    __syncthreads();
+    uint32_t base = incl - cnt, total = 0;
+#pragma unroll
+    for (uint32_t v = 0; v < T / 32; ++v) {
+      base += v < warp ? s_warp[v] : 0u;
+      total += s_warp[v];
+    }
+    {
+      uint32_t at = base;
+      for (uint32_t m = need; m; m &= m - 1) s_job[at++] = j0 + (__ffs(m) - 1);
+    }
+    __syncthreads();
+    for (uint32_t i = threadIdx.x; i < total; i += T) {
+      int32_t a, b;
+      gate_kadane_segment(prof, db, jobs[s_job[i]], a, b);
+      s_pos[i] = make_int2(a, b);
+    }
+    __syncthreads();
+    auto pos = [&](uint32_t x) { return s_pos[base + __popc(need & ((1u << x) - 1u))]; };
+    if (on) {
+      int32_t chain = INT32_MIN;
+      uint32_t cx = 0, cy = 0;
+      if (need && nsg > 1)
+        pairs([&](uint32_t x, uint32_t y, int32_t c, int32_t dx, int32_t dy) {
+          if (c <= chain) return;
+          const int32_t qex = pos(x).y, qsy = pos(y).x;
           if (qex < qsy && static_cast<int64_t>(qex) + dx < static_cast<int64_t>(qsy) + dy) {
             chain = c;
             cx = x;
             cy = y;
           }
+        });
+      int32_t sum;
+      uint32_t u0, u1;
+      if (chain > best) {
+        ++n_chained;
+        sum = chain;
+        u0 = cx;
+        u1 = cy;
+      } else {
+        sum = best;
+        u0 = u1 = bi;
+      }
+      if (sum >= g.min_score) {
+        uint32_t s, e;
+        gate_group_range(G, gi, ng, s, e);
+        uint32_t rlo = 0, rhi = 0xFFFFFFFFu;
+        if (g.regions) {
+          const int2 p0 = pos(u0), p1 = pos(u1);
+          const int64_t d0 = jobs[j0 + u0].diag, d1 = jobs[j0 + u1].diag;
+          const int64_t a0 = i64max(p0.x + d0, 0), b0 = i64max(p0.y + d0, 0);
+          const int64_t a1 = i64max(p1.x + d1, 0), b1 = i64max(p1.y + d1, 0);
+          rlo = static_cast<uint32_t>(i64min(a0, a1));
+          rhi = static_cast<uint32_t>(i64max(b0, b1));
         }
+        const GateJob jb = jobs[j0];
+        cand[gi] = GateCandidate{jb.query, jb.target, e - s, sum, static_cast<int64_t>(jobs[j0 + bi].diag), rlo, rhi};
+        flag[gi] = 1;
       }
     }
-    int32_t total;
-    uint32_t u0, u1;
-    if (chain > best) {
-      ++n_chained;
-      total = chain;
-      u0 = cx;
-      u1 = cy;
-    } else {
-      total = best;
-      u0 = u1 = bi;
-    }
-    if (total < g.min_score) continue;
-    uint32_t s, e;
-    gate_group_range(G, gi, ng, s, e);
-    uint32_t rlo = 0, rhi = 0xFFFFFFFFu;
-    if (g.regions) {
-      pos_of(u0);
-      pos_of(u1);
-      const int64_t d0 = jobs[j0 + u0].diag, d1 = jobs[j0 + u1].diag;
-      const int64_t a0 = i64max(pqs[u0] + d0, 0), b0 = i64max(pqe[u0] + d0, 0);
-      const int64_t a1 = i64max(pqs[u1] + d1, 0), b1 = i64max(pqe[u1] + d1, 0);
-      rlo = static_cast<uint32_t>(i64min(a0, a1));
-      rhi = static_cast<uint32_t>(i64max(b0, b1));
-    }
-    const GateJob jb = jobs[j0];
-    cand[gi] = GateCandidate{jb.query, jb.target, e - s, total, static_cast<int64_t>(jobs[j0 + bi].diag), rlo, rhi};
-    flag[gi] = 1;
+    __syncthreads();  // the shared lists are written again in the next round
   }
   gate_flush(&st->chains_used, n_chained);
 }

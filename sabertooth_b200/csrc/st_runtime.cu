@@ -3683,7 +3683,13 @@ static int gate_pipeline(st_ctx* c, const GateSeedHit* d_hits, uint64_t* d_keys,
   ST_CUDA(cudaMemsetAsync(flag, 0, n, s));
   ST_CUDA(cudaMemsetAsync(n_work, 0, 4, s));
   gate_screen_kernel<<<grid_for(n, 256), 256, 0, s>>>(G, g, joff, sc, work, n_work);
-  gate_chain_kernel<<<grid_for(n, 128), 128, 0, s>>>(G, g, db, pv, joff, jobs, sc, work, n_work, cand, flag, st);
+  if (g.kmax <= 4)
+    gate_chain_kernel<4><<<grid_for(n, kChainThreads<4>), kChainThreads<4>, 0, s>>>(
+        G, g, db, pv, joff, jobs, sc, work, n_work, cand, flag, st);
+  else
+    gate_chain_kernel<kGateMaxDiags><<<grid_for(n, kChainThreads<kGateMaxDiags>),
+                                       kChainThreads<kGateMaxDiags>, 0, s>>>(
+        G, g, db, pv, joff, jobs, sc, work, n_work, cand, flag, st);
   {
     cub::CountingInputIterator<uint32_t> it(0);
     t = t_max;
