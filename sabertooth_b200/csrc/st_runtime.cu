@@ -456,7 +456,13 @@ static int pool_get(st_ctx* c, size_t bytes, DevMem& out) {
       want = q * k;
       break;
     }
-  return dev_alloc(&c->mt, out, std::max(want, bytes));
+  const int rc = dev_alloc(&c->mt, out, std::max(want, bytes));
+  if (rc != ST_ENOMEM) return rc;
+  // near the budget: exactly what is asked for, with the unused arenas given back (freeing one waits for the device)
+  for (auto& e : c->pool)
+    if (e.ready) c->spare_events.push_back(e.ready);
+  c->pool.clear();
+  return dev_alloc(&c->mt, out, bytes);
 }
 
 static void pool_trim(st_ctx* c) {
