@@ -646,7 +646,7 @@ def main():
                                    "ms_parts": e2e_parts}},
             "plain": {"value": round(plain_gcups, 3), "unit": UNIT, "pairs": int(len(sample)),
                       "matches_batched": bool(plain_ok),
-                      "how": "one st_sw_score call per pair (host target, 2 launches, blocking)"},
+                      "how": "one st_sw_score call per pair (host target, one launch, blocking)"},
             "plain_concurrent": plain_conc,
             "batched_vs_plain": round(gcups / world / plain_gcups, 1),
             "clocks": clocks,

@@ -10,7 +10,7 @@
 // owns query rows [pass*256 + 8l, +8), the columns of both pairs' band windows
 // stream through the warp as a wavefront, and a query of more than 256 rows
 // is scored in passes whose bottom row goes through the warp's scratch line.
-// The recurrence is the packed one of the tile classes (six DPX operations and
+// The recurrence is the literal one in packed cells (six DPX operations and
 // a prmt per cell pair); a per-cell band mask, built per lane and step from
 // the band rows of the lane's eight rows, sets out-of-band cells to H = 0 and
 // their successors' E and F to -open, as the 32-bit kernel does.
