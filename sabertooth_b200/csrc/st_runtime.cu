@@ -458,9 +458,13 @@ static int pool_get(st_ctx* c, size_t bytes, DevMem& out) {
     }
   const int rc = dev_alloc(&c->mt, out, std::max(want, bytes));
   if (rc != ST_ENOMEM) return rc;
-  // near the budget: exactly what is asked for, with the unused arenas given back (freeing one waits for the device)
+  // near the budget: exactly what is asked for, with the pooled arenas given back once their last work is done
   for (auto& e : c->pool)
-    if (e.ready) c->spare_events.push_back(e.ready);
+    if (e.ready) {
+      ST_CUDA(cudaEventSynchronize(e.ready));
+      c->spare_events.push_back(e.ready);
+      e.ready = nullptr;
+    }
   c->pool.clear();
   return dev_alloc(&c->mt, out, bytes);
 }
