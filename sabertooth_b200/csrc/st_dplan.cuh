@@ -33,12 +33,14 @@ namespace st {
 constexpr int kDpMaxClasses = 32;
 constexpr uint32_t kDpNoClass = 63;  // sort key of a query with no 16-bit pairs
 
+static_assert(kTuneMaxPasses <= kMaxPasses16, "a pass number has to fit the packed kernel's control word");
+
 struct DpClass {
   uint32_t G, R, C, W;
   uint32_t team;      // a CTA's warps share each warp task's passes
   uint32_t rows;      // G * R
   uint32_t S;         // targets per warp task, 64 / G
-  uint32_t max_mpad;  // the largest staged row count that fits the class's shared memory
+  uint32_t max_mpad;  // the largest staged row count of the class (tune_max_rows)
   float rate;         // streamed cells per second / 1e12 (0: not considered)
 };
 

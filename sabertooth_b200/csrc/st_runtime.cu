@@ -1388,15 +1388,13 @@ static int plan_build(st_ctx* c, const st_pair* pairs, uint64_t n, int32_t open,
   plan->d_scores = d_scores;
   plan->d_kernels = d_kernels;
   const bool g16 = gaps16_ok(open, ext);
-  // the longest query whose int8 profile fits the shared memory of some 16-bit class;
-  // longer ones take the 32-bit kernel
+  // the longest query that some 16-bit class stages; longer ones take the 32-bit kernel
   const uint32_t max_n16 = ends ? kEndMaxLen : UINT32_MAX;
   uint32_t max_m16 = 0;
   for (int k = 0; k < kNumClasses; ++k) {
     if (ends && !end_fns(k)) continue;
     const uint32_t rows = static_cast<uint32_t>(kClasses[k].G * kClasses[k].R);
-    const uint32_t smem = static_cast<uint32_t>(std::min<int>(g_class_smem[k], 216 * 1024));  // the models' limit
-    max_m16 = std::max(max_m16, smem / kProfRows / rows * rows);
+    max_m16 = std::max(max_m16, tune_max_rows(rows, static_cast<uint32_t>(g_class_smem[k])));
   }
   TraceClock tc("plan");
 
@@ -2147,8 +2145,7 @@ static int dplan_build(st_ctx* c, const st_pair* pairs, uint64_t n, int32_t open
     d.team = kClasses[k].team ? 1u : 0u;
     d.rows = d.G * d.R;
     d.S = 64 / d.G;
-    const uint32_t smem = static_cast<uint32_t>(std::min<int>(g_class_smem[k], 216 * 1024));
-    d.max_mpad = ends && !end_fns(k) ? 0u : smem / kProfRows / d.rows * d.rows;
+    d.max_mpad = ends && !end_fns(k) ? 0u : tune_max_rows(d.rows, static_cast<uint32_t>(g_class_smem[k]));
     d.rate = c->tuning.rate[k];
     max_m16 = std::max(max_m16, d.max_mpad);
   }
@@ -4532,11 +4529,11 @@ extern "C" int st_autotune(st_ctx* c, const st_pair* pairs, uint64_t n, int32_t 
   ST_TRY(sync_profiles(c));
   if (classes_calibrated) *classes_calibrated = 0;
   if (!gaps16_ok(open, ext)) return ST_OK;  // nothing runs on the 16-bit kernel
-  // queries that every class can stage (the models' shared-memory limit)
+  // queries that every class can stage
   uint32_t max_m = UINT32_MAX;
   for (int k = 0; k < kNumClasses; ++k) {
     const uint32_t rows = static_cast<uint32_t>(kClasses[k].G * kClasses[k].R);
-    max_m = std::min(max_m, static_cast<uint32_t>(216 * 1024) / kProfRows / rows * rows);
+    max_m = std::min(max_m, tune_max_rows(rows));
   }
   std::vector<std::vector<uint32_t>> byq(c->profs.size());
   for (uint64_t i = 0; i < n; ++i) {

@@ -128,6 +128,7 @@ constexpr uint32_t kNoPair = 0xFFFFFFFFu;
 constexpr uint32_t kCtlLast = 1u << 27;   // last step of the task
 constexpr uint32_t kCtlFirst = 1u << 28;  // first step of a pass
 constexpr uint32_t kCtlMore = 1u << 29;   // a pass that is not the last: its bottom row is kept
+constexpr uint32_t kMaxPasses16 = 256;    // passes that bits 16-23 can name; the planners admit no more
 constexpr int kSlotRing = 8;
 constexpr uint32_t kTeamSpins = 1u << 22;  // polls of a producer's count before a team gives its pair up
 

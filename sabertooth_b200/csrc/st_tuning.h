@@ -24,6 +24,16 @@ constexpr int kTuneMBins = 10;  // query length: <=32, <=64, ..., <=8192, >8192
 constexpr int kTuneNBins = 8;   // mean target length: <=64, <=128, ..., <=4096, >4096
 constexpr int kMaxTileClasses = 32;
 
+// The queries that the packed kernel stages: 22 int8 rows of the query padded to whole passes in shared memory, and a
+// pass number that fits the eight bits it has in the kernel's control word (only <4,8> would need more, past 8,192 rows).
+constexpr uint32_t kTuneStageBytes = 216 * 1024;
+constexpr uint32_t kTuneMaxPasses = 256;
+
+// The longest staged query, padded to whole passes of `rows` rows.
+inline uint32_t tune_max_rows(uint32_t rows, uint32_t smem = kTuneStageBytes) {
+  return std::min(std::min(smem, kTuneStageBytes) / 22 / rows, kTuneMaxPasses) * rows;
+}
+
 struct Tuning {
   int table[kTuneMBins][kTuneNBins];  // class index, -1 = rate model
   float rate[kMaxTileClasses];        // streamed cells per second / 1e12, per class; 0 = not used
@@ -104,7 +114,7 @@ inline double tune_streamed(int c, uint32_t m, const uint32_t* tlen_desc, size_t
   st_tuning_class_shape(c, &G, &R, &C);
   const uint32_t rows = static_cast<uint32_t>(G * R);
   const uint32_t P = (m + rows - 1) / rows;
-  if (22.0 * P * rows > 216.0 * 1024) return 1e300;  // profile does not fit shared memory
+  if (P * rows > tune_max_rows(rows)) return 1e300;  // the class does not stage this query
   const uint32_t S = static_cast<uint32_t>(64 / G);
   uint32_t minc = 32;
   if (P > 1) minc = std::max<uint32_t>(minc, (static_cast<uint32_t>(C * G) + 15) & ~15u);
@@ -196,7 +206,7 @@ inline int tuning_pick_single(const Tuning*, uint32_t m, uint32_t n) {
     int G, R, C;
     st_tuning_class_shape(c, &G, &R, &C);
     const uint32_t rows = static_cast<uint32_t>(G * R), P = (m + rows - 1) / rows;
-    if (22.0 * P * rows > 216.0 * 1024) continue;  // profile does not fit shared memory
+    if (P * rows > tune_max_rows(rows)) continue;  // the class does not stage this query
     uint32_t ncols = std::max<uint32_t>(32, (n + 3) & ~3u);
     if (P > 1) ncols = std::max<uint32_t>(ncols, (static_cast<uint32_t>(C * G) + 15) & ~15u);
     const double v = tune_crit_ps(G, R, C, P, ncols, st_tuning_class_team(c) ? st_tuning_class_warps(c) : 1);
