@@ -55,11 +55,15 @@ static int fail(int code, const char* fmt, ...) {
   return code;
 }
 
+// An error is reported once: the runtime's record of it is cleared, as the checks after launches
+// (cudaGetLastError) would report it again for work that went well.  (One that ends the context stays.)
 #define ST_CUDA(call)                                                                              \
   do {                                                                                             \
     cudaError_t e_ = (call);                                                                       \
-    if (e_ != cudaSuccess) return fail(ST_ECUDA, "%s: %s (%s:%d)", #call, cudaGetErrorString(e_), \
-                                       __FILE__, __LINE__);                                        \
+    if (e_ != cudaSuccess) {                                                                       \
+      cudaGetLastError();                                                                          \
+      return fail(ST_ECUDA, "%s: %s (%s:%d)", #call, cudaGetErrorString(e_), __FILE__, __LINE__); \
+    }                                                                                              \
   } while (0)
 
 #define ST_TRY(expr)          \
@@ -120,7 +124,8 @@ __attribute__((visibility("hidden"))) void st_internal_set_error(const char* msg
 // ---------------------------------------------------------------------------
 struct MemTracker {
   size_t used = 0;
-  size_t budget = 0;  // 0 = unlimited
+  size_t budget = 0;           // 0 = unlimited
+  size_t fail_above = SIZE_MAX;  // a larger allocation is made to fail in the driver (ST_ALLOC_FAIL_ABOVE, for tests)
 };
 
 struct DevMem {
@@ -167,9 +172,10 @@ static int dev_alloc(MemTracker* mt, DevMem& m, size_t bytes) {
   cudaError_t e;
   {
     SlowCall sc("cudaMalloc", bytes);
-    e = cudaMalloc(&m.p, bytes);
+    e = cudaMalloc(&m.p, bytes > mt->fail_above ? size_t{1} << 46 : bytes);
   }
   if (e != cudaSuccess) {
+    cudaGetLastError();  // the caller may do without, or try less: no later check is to find it
     m.p = nullptr;
     return fail(ST_ENOMEM, "cudaMalloc(%zu): %s", bytes, cudaGetErrorString(e));
   }
@@ -458,7 +464,8 @@ static int pool_get(st_ctx* c, size_t bytes, DevMem& out) {
     }
   const int rc = dev_alloc(&c->mt, out, std::max(want, bytes));
   if (rc != ST_ENOMEM) return rc;
-  // near the budget: exactly what is asked for, with the pooled arenas given back once their last work is done
+  // near the budget or the device's memory: exactly what is asked for, with the pooled arenas given back once their
+  // last work is done
   for (auto& e : c->pool)
     if (e.ready) {
       ST_CUDA(cudaEventSynchronize(e.ready));
@@ -713,6 +720,7 @@ extern "C" st_ctx* st_init(int device, size_t hbm_budget_bytes) {
   c->device = device;
   c->sms = prop.multiProcessorCount;
   c->mt.budget = hbm_budget_bytes;
+  c->mt.fail_above = env_u64("ST_ALLOC_FAIL_ABOVE", SIZE_MAX);
   if (cudaStreamCreateWithFlags(&c->own, cudaStreamNonBlocking) != cudaSuccess) {
     fail(ST_ECUDA, "cudaStreamCreate failed");
     return nullptr;
