@@ -23,7 +23,7 @@
 // past a window's columns or on a half's idle passes score 0 and cannot raise
 // the maximum (open, extend >= 0).
 //
-// Work: warps claim four entries of the 32-bit list's static part at a time;
+// Work: warps claim two entries of the 32-bit list's static part at a time;
 // entries that are not banded pairs with int8 rows are left to the 32-bit
 // kernel, which skips exactly the entries taken here (band16_takes).  Bands of
 // radius up to 140 take band16_ring, wider ones the whole-warp passes of
@@ -515,46 +515,94 @@ __device__ __forceinline__ void band16_ring(const Sw32Params& prm, uint32_t pA, 
   }
 }
 
-// Warps claim four entries of the list at a time; the widest band among them says how they are scored.
+// A couple of wide bands out of line: inlined beside the rings it took the kernel's registers with it (2,000 pairs of
+// radius 64: 854 us inlined, 660 us so).
+__device__ __noinline__ void band16_couple_call(const Sw32Params& prm, uint32_t pA, uint32_t pB, int2* bnd) {
+  band16_couple(prm, pA, pB, bnd);
+}
+
+// Entries w and w + 1 of the list where they are scored here (kBandNone where not); returns their widest radius, -1
+// for none.
+__device__ __forceinline__ int32_t band16_entries(const Sw32Params& prm, uint32_t w, uint32_t& a, uint32_t& b) {
+  int32_t widest = -1;
+  a = b = kBandNone;
+  if (w < prm.n_static) {
+    const uint32_t e = prm.list[w];
+    if (band16_takes(prm, e)) {
+      a = e;
+      widest = prm.pair_radius[e];
+    }
+  }
+  if (w + 1 < prm.n_static) {
+    const uint32_t e = prm.list[w + 1];
+    if (band16_takes(prm, e)) {
+      b = e;
+      widest = max(widest, prm.pair_radius[e]);
+    }
+  }
+  return widest;
+}
+
+// Warps claim two entries of the list at a time, the most that is scored at once where a radius is above a ring of 16
+// lanes' (68): a couple more behind them would wait for the whole of the first while warps beside stay empty (with
+// claims of four, lists of 4 to 8,000 pairs of radius 100 or 300 took 1.2 to 2.1 times as long).  A couple of narrower
+// bands fills half a warp, so another is claimed beside it.
 template <int WARPS>
 __global__ void __launch_bounds__(WARPS * 32) sw16_band_kernel(const Sw32Params prm) {
+  const int warp = threadIdx.x >> 5;
+  const int lane = threadIdx.x & 31;
+  int2* bnd = prm.scratch + static_cast<size_t>(blockIdx.x * WARPS + warp) * prm.scratch_stride;
+  for (;;) {
+    uint32_t w = 0;
+    if (lane == 0) w = atomicAdd(prm.work_counter, 2u);
+    w = __shfl_sync(0xFFFFFFFFu, w, 0);
+    if (w >= prm.n_static) break;
+    uint32_t a, b;
+    int32_t widest = band16_entries(prm, w, a, b);
+    if (widest < 0) continue;
+    if (widest <= band_ring_radius(16)) {
+      if (lane == 0) w = atomicAdd(prm.work_counter, 2u);
+      w = __shfl_sync(0xFFFFFFFFu, w, 0);
+      uint32_t c, d;
+      const int32_t beside = band16_entries(prm, w, c, d);
+      const bool pack = beside <= band_ring_radius(16);  // none at all included
+      if (lane >= 16) {
+        a = pack ? c : kBandNone;
+        b = pack ? d : kBandNone;
+      }
+      band16_ring<16>(prm, a, b, bnd);
+      if (pack) continue;
+      a = c;  // wider ones after all
+      b = d;
+      widest = beside;
+    }
+    if (widest <= band_ring_radius(32))
+      band16_ring<32>(prm, a, b, bnd);
+    else
+      band16_couple_call(prm, a, b, bnd);
+  }
+}
+
+// The same for a list without a band that a ring takes (every radius above 140): whole-warp passes alone, in 95
+// registers instead of 126, which leaves room for five CTAs an SM instead of four (8,000 pairs of radius 300: 7.06
+// against 8.00 ms; 2 pairs: 2.40 against 2.46).
+template <int WARPS>
+__global__ void __launch_bounds__(WARPS * 32) sw16_band_wide_kernel(const Sw32Params prm) {
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
   int2* bnd = prm.scratch + static_cast<size_t>(blockIdx.x * WARPS + warp) * prm.scratch_stride;
   const uint32_t n = prm.n_static;
   for (;;) {
     uint32_t w = 0;
-    if (lane == 0) w = atomicAdd(prm.work_counter, 4u);
+    if (lane == 0) w = atomicAdd(prm.work_counter, 2u);
     w = __shfl_sync(0xFFFFFFFFu, w, 0);
     if (w >= n) break;
-    uint32_t p[4];
-    int32_t widest = -1;
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      p[k] = kBandNone;
-      if (w + k < n) {
-        const uint32_t e = prm.list[w + k];
-        if (band16_takes(prm, e)) {
-          p[k] = e;
-          widest = max(widest, prm.pair_radius[e]);
-        }
-      }
-    }
-    if (widest < 0) continue;
-    if (widest <= band_ring_radius(16)) {
-      const bool upper = lane >= 16;
-      band16_ring<16>(prm, upper ? p[2] : p[0], upper ? p[3] : p[1], bnd);
-    } else {
-#pragma unroll 1
-      for (int k = 0; k < 4; k += 2) {
-        const uint32_t a = k ? p[2] : p[0], b = k ? p[3] : p[1];
-        if (a == kBandNone && b == kBandNone) continue;
-        if (widest <= band_ring_radius(32))
-          band16_ring<32>(prm, a, b, bnd);
-        else
-          band16_couple(prm, a, b, bnd);
-      }
-    }
+    const uint32_t a = prm.list[w];
+    const uint32_t b = w + 1 < n ? prm.list[w + 1] : kBandNone;
+    const uint32_t pA = band16_takes(prm, a) ? a : kBandNone;
+    const uint32_t pB = (b != kBandNone && band16_takes(prm, b)) ? b : kBandNone;
+    if (pA == kBandNone && pB == kBandNone) continue;
+    band16_couple(prm, pA, pB, bnd);
   }
 }
 

@@ -1248,6 +1248,7 @@ struct st_plan {
   double batch_ps = 0;    // the chip's time for them, every query in its cheapest class
   uint32_t kernels_per_run = 0;
   Sw32Params p32;
+  bool band_wide = false;  // no band of the list is one that the rings take
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t exec = nullptr;
 };
@@ -1279,6 +1280,12 @@ static int occupancy_grid(st_ctx* c, const void* fn, int threads, size_t smem, u
   return ST_OK;
 }
 
+// The packed kernel of the list's banded pairs.
+static void launch_band(const st_plan* p, cudaStream_t s) {
+  const auto fn = p->band_wide ? sw16_band_wide_kernel<kWarps32> : sw16_band_kernel<kWarps32>;
+  fn<<<p->grid32, kWarps32 * 32, 0, s>>>(p->p32);
+}
+
 // The launches of one run, in stream order: clear outputs, reset counters,
 // every 16-bit class, then the 32-bit kernel over the static list plus the
 // pairs the 16-bit classes flagged.
@@ -1297,7 +1304,7 @@ static int plan_enqueue(st_plan* p, cudaStream_t st, st_ctx::ForkSet* fs, bool g
   const bool band16 = p->p32.band16 != 0;
   if (!fs || nc + (band16 ? 1 : 0) <= 1) {
     for (auto& cp : p->classes) kClasses[cp.cls].fn<<<cp.grid, kClasses[cp.cls].W * 32, cp.smem, st>>>(cp.prm);
-    if (band16) sw16_band_kernel<kWarps32><<<p->grid32, kWarps32 * 32, 0, st>>>(p->p32);
+    if (band16) launch_band(p, st);
   } else {
     // The classes run side by side: the costliest on the launching stream, the
     // others on forks joined before sw32. The launch order matters, as the block
@@ -1353,7 +1360,7 @@ static int plan_enqueue(st_plan* p, cudaStream_t st, st_ctx::ForkSet* fs, bool g
         used[j] = true;
         s = fs->s[j];
       }
-      sw16_band_kernel<kWarps32><<<p->grid32, kWarps32 * 32, 0, s>>>(p->p32);
+      launch_band(p, s);
       if (cudaGetLastError() != cudaSuccess) return ST_ECUDA;
     }
     for (int j = 0; j < st_ctx::ForkSet::kForks; ++j) {
@@ -1423,8 +1430,10 @@ static int plan_build(st_ctx* c, const st_pair* pairs, uint64_t n, int32_t open,
   int64_t bad = -1;
   uint64_t cells = 0, cells32 = 0;
   uint32_t max_len = 0, max_m32 = 0;
+  int32_t min_radius = INT32_MAX;
   // classify every pair (validation, route, cells), in parallel
-#pragma omp parallel for schedule(static) reduction(+ : cells, cells32) reduction(max : max_len, max_m32)
+#pragma omp parallel for schedule(static) reduction(+ : cells, cells32) reduction(max : max_len, max_m32) \
+    reduction(min : min_radius)
   for (int64_t i = 0; i < static_cast<int64_t>(n); ++i) {
     const st_pair& p = pairs[i];
     if (p.profile >= n_prof || !c->profs[p.profile].live || p.target >= c->n_seqs) {
@@ -1446,6 +1455,7 @@ static int plan_build(st_ctx* c, const st_pair* pairs, uint64_t n, int32_t open,
     max_len = std::max(max_len, tl);
     max_m32 = std::max(max_m32, pm.m);  // every 16-bit pair may be rescored in 32 bits
     if (p.band_radius >= 0) {
+      min_radius = std::min(min_radius, p.band_radius);
       const uint64_t bc = band_cells(pm.m, tl, p.band_center, p.band_radius);
       cells += bc;
       cells32 += bc;
@@ -1470,6 +1480,7 @@ static int plan_build(st_ctx* c, const st_pair* pairs, uint64_t n, int32_t open,
   }
   plan->cells = cells;
   plan->cells32 = cells32;
+  plan->band_wide = min_radius > band_ring_radius(32);
   tc.lap("classify");
   // 32-bit list in pair order; 16-bit pairs grouped by query, in pair order
   // within a query: a counting sort with one histogram per thread over
@@ -2023,7 +2034,7 @@ extern "C" int st_plan_profile(st_plan* p, uint32_t cap, int32_t* classes, uint6
       cells[i] = cp.cells;
     } else if (nb && i + 1 < n) {
       // the banded pairs of the static list (their cells are counted with the 32-bit list's)
-      sw16_band_kernel<kWarps32><<<p->grid32, kWarps32 * 32, 0, c->stream>>>(p->p32);
+      launch_band(p, c->stream);
       ST_CUDA(cudaMemsetAsync(p->p32.work_counter, 0, 4, c->stream));
       classes[i] = -2;
       cells[i] = 0;
@@ -2079,18 +2090,21 @@ static int pipeline_streams() {
 
 // Checks every pair (profile id live, target in the database) in parallel;
 // reports the first bad one. Also the longest target and query of the batch
-// (the 32-bit kernel's scratch).
-static int validate_pairs(st_ctx* c, const st_pair* pairs, uint64_t n, uint32_t* max_len, uint32_t* max_m) {
+// (the 32-bit kernel's scratch), and its narrowest band (INT32_MAX: none).
+static int validate_pairs(st_ctx* c, const st_pair* pairs, uint64_t n, uint32_t* max_len, uint32_t* max_m,
+                          int32_t* min_radius) {
   const uint32_t n_prof = static_cast<uint32_t>(c->profs.size());
   int64_t bad = INT64_MAX;
   uint32_t ml = 0, mm = 0;
-#pragma omp parallel for schedule(static) reduction(min : bad) reduction(max : ml, mm)
+  int32_t nr = INT32_MAX;
+#pragma omp parallel for schedule(static) reduction(min : bad, nr) reduction(max : ml, mm)
   for (int64_t i = 0; i < static_cast<int64_t>(n); ++i) {
     const st_pair& p = pairs[i];
     if (p.profile >= n_prof || !c->profs[p.profile].live || p.target >= c->n_seqs) {
       bad = std::min<int64_t>(bad, i);
       continue;
     }
+    if (p.band_radius >= 0) nr = std::min(nr, p.band_radius);
     const uint32_t tl = c->h_db_len[p.target];
     const uint32_t m = c->profs[p.profile].m;
     if (tl && m) {
@@ -2105,8 +2119,9 @@ static int validate_pairs(st_ctx* c, const st_pair* pairs, uint64_t n, uint32_t*
     return fail(ST_EINVAL, "pair %lld: target %u outside the database (%u sequences)", static_cast<long long>(bad),
                 p.target, c->n_seqs);
   }
-  if (max_len) *max_len = ml;
-  if (max_m) *max_m = mm;
+  *max_len = ml;
+  *max_m = mm;
+  *min_radius = nr;
   return ST_OK;
 }
 
@@ -2126,8 +2141,8 @@ static int bits_for(uint64_t x) {
 static int upload_host(st_ctx* c, void* dst, const void* src, size_t bytes, cudaStream_t s);
 
 static int dplan_build(st_ctx* c, const st_pair* pairs, uint64_t n, int32_t open, int32_t ext, int32_t* d_scores,
-                       uint32_t* d_kernels, uint32_t max_len, uint32_t max_m, DevMem& work, st_plan** out,
-                       bool ends = false) {
+                       uint32_t* d_kernels, uint32_t max_len, uint32_t max_m, int32_t min_radius, DevMem& work,
+                       st_plan** out, bool ends = false) {
   cudaStream_t st = c->stream;
   TraceClock tc("dplan");
   const uint32_t n_prof = static_cast<uint32_t>(c->profs.size());
@@ -2320,6 +2335,7 @@ static int dplan_build(st_ctx* c, const st_pair* pairs, uint64_t n, int32_t open
   }
   plan->scratch32_stride = max_m > static_cast<uint32_t>(kSw32Rows) ? max_len : 0;
   plan->n_static32 = n_list32;
+  plan->band_wide = min_radius > band_ring_radius(32);
   plan->batch_ps = static_cast<double>(tot.batch_ps);
   ST_TRY(grid_sw32(c, n_list32, n, plan->scratch32_stride, &plan->grid32));
   size_t t_lpt = 0;
@@ -2526,10 +2542,11 @@ static int batch_begin(st_ctx* c, const st_pair* pairs, uint64_t n, int32_t open
   }
   if (use_device_plan(n)) {
     uint32_t max_len = 0, max_m = 0;
-    ST_TRY(validate_pairs(c, pairs, n, &max_len, &max_m));
+    int32_t min_radius = 0;
+    ST_TRY(validate_pairs(c, pairs, n, &max_len, &max_m, &min_radius));
     ST_TRY(sync_profiles(c));
     tc.lap("validate");
-    ST_TRY(dplan_build(c, pairs, n, open, ext, d_scores, d_kern, max_len, max_m, b->work, &b->plan));
+    ST_TRY(dplan_build(c, pairs, n, open, ext, d_scores, d_kern, max_len, max_m, min_radius, b->work, &b->plan));
   } else {
     ST_TRY(plan_build(c, pairs, n, open, ext, d_scores, d_kern, &b->plan, false, c->stream, 0));
     tc.lap("plan");
@@ -2861,7 +2878,8 @@ static int end_pairs_entry(st_ctx* c, const st_pair* pairs, uint64_t n, int32_t 
   if (n && (!pairs || !scores || !ends || (span && !starts))) return fail(ST_EINVAL, "null argument");
   if (!c->has_db) return fail(ST_ESTATE, "no target database uploaded (st_db_upload)");
   uint32_t max_len = 0, max_m = 0;
-  ST_TRY(validate_pairs(c, pairs, n, &max_len, &max_m));
+  int32_t min_radius = 0;
+  ST_TRY(validate_pairs(c, pairs, n, &max_len, &max_m, &min_radius));
   int64_t banded = INT64_MAX;
 #pragma omp parallel for schedule(static) reduction(min : banded) if (n > 65536)
   for (int64_t i = 0; i < static_cast<int64_t>(n); ++i)
@@ -2896,7 +2914,7 @@ static int end_pairs_entry(st_ctx* c, const st_pair* pairs, uint64_t n, int32_t 
   int32_t* d = out.as<int32_t>();
   int32_t *d_s = d, *d_eq = d + n, *d_et = d + 2 * n, *d_rs = d + 3 * n, *d_sq = d + 4 * n, *d_st = d + 5 * n;
   if (use_device_plan(n))
-    ST_TRY(dplan_build(c, pairs, n, open, ext, d_s, nullptr, max_len, max_m, work, &plan, true));
+    ST_TRY(dplan_build(c, pairs, n, open, ext, d_s, nullptr, max_len, max_m, min_radius, work, &plan, true));
   else
     ST_TRY(plan_build(c, pairs, n, open, ext, d_s, nullptr, &plan, false, c->stream, 0, true));
   cudaStream_t st = c->stream;
