@@ -386,6 +386,7 @@ struct st_ctx {
   std::vector<std::unique_ptr<CallSlot>> call_slots;
   std::vector<CallSlot*> call_idle;
   Tuning tuning;
+  uint32_t end_ready[2] = {};  // end-cell kernels (forward, reverse) whose shared memory is set, a bit per tile class
   // seed index over the database (st_seed_index_build): offsets of the 20^w codes, postings
   DevMem seed_off, seed_post;
   SeedPat seed_pat{};
@@ -650,6 +651,8 @@ static int g_ung_smem = 0;              // dynamic shared memory the ungapped ke
 static int g_ung_split_smem = 0;        // the same for ungapped_hits_split_kernel (more static shared memory)
 static int g_gate_smem = 0;             // dynamic shared memory of the prefilter segment kernel
 
+// For every context: the kernels whose limits the planners and the checks need.  The end-cell kernels and the seed
+// kernel get theirs where they are launched, so that a context pays for what it uses.
 static int set_smem_limits(int device) {
   int optin = 0;
   ST_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device));
@@ -659,19 +662,10 @@ static int set_smem_limits(int device) {
     g_class_smem[i] = std::min<int>(kMaxSmem, optin - static_cast<int>(fa.sharedSizeBytes));
     ST_CUDA(cudaFuncSetAttribute(kClasses[i].fn, cudaFuncAttributeMaxDynamicSharedMemorySize, g_class_smem[i]));
   }
-  for (const auto& f : kEndFns)
-    for (Sw16Fn fn : {f.fwd, f.rev}) {
-      cudaFuncAttributes fa;
-      ST_CUDA(cudaFuncGetAttributes(&fa, reinterpret_cast<const void*>(fn)));
-      ST_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   std::min<int>(kMaxSmem, optin - static_cast<int>(fa.sharedSizeBytes))));
-    }
-  cudaFuncAttributes fa_t, fa_f;
-  ST_CUDA(cudaFuncGetAttributes(&fa_t, reinterpret_cast<const void*>(ungapped_kernel<true>)));
-  ST_CUDA(cudaFuncGetAttributes(&fa_f, reinterpret_cast<const void*>(ungapped_kernel<false>)));
-  g_ung_smem = std::min<int>(kMaxSmem, optin - static_cast<int>(std::max(fa_t.sharedSizeBytes, fa_f.sharedSizeBytes)));
-  ST_CUDA(cudaFuncSetAttribute(ungapped_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, g_ung_smem));
-  ST_CUDA(cudaFuncSetAttribute(ungapped_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, g_ung_smem));
+  cudaFuncAttributes fa_l;
+  ST_CUDA(cudaFuncGetAttributes(&fa_l, reinterpret_cast<const void*>(ungapped_kernel)));
+  g_ung_smem = std::min<int>(kMaxSmem, optin - static_cast<int>(fa_l.sharedSizeBytes));
+  ST_CUDA(cudaFuncSetAttribute(ungapped_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, g_ung_smem));
   cudaFuncAttributes fa_r;
   ST_CUDA(cudaFuncGetAttributes(&fa_r, reinterpret_cast<const void*>(ungapped_hits_refill_kernel)));
   g_ung_smem = std::min<int>(g_ung_smem, optin - static_cast<int>(fa_r.sharedSizeBytes));
@@ -681,8 +675,6 @@ static int set_smem_limits(int device) {
   g_ung_split_smem = std::min<int>(kMaxSmem, optin - static_cast<int>(fa_s.sharedSizeBytes));
   ST_CUDA(cudaFuncSetAttribute(ungapped_hits_split_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                g_ung_split_smem));
-  ST_CUDA(cudaFuncSetAttribute(seed_emit_warp_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               2 * kSeedWarpCap * static_cast<int>(sizeof(int2))));
   cudaFuncAttributes fa_g;
   ST_CUDA(cudaFuncGetAttributes(&fa_g, reinterpret_cast<const void*>(gate_score_kernel)));
   g_gate_smem = std::min<int>(kMaxSmem, optin - static_cast<int>(fa_g.sharedSizeBytes));
@@ -2828,6 +2820,18 @@ static int end_single_run(st_ctx* c, const DeviceDb& db, uint32_t profile, uint3
   return ST_OK;
 }
 
+// A class's end-cell kernel, ready for the longest query that the classes stage (beside its 10 KB of static shared
+// memory that is within an SM's).
+static int end_kernel(st_ctx* c, int cls, bool rev, Sw16Fn* fn) {
+  const Sw16EndFns* f = end_fns(cls);
+  *fn = rev ? f->rev : f->fwd;
+  uint32_t& ready = c->end_ready[rev ? 1 : 0];
+  if (ready >> cls & 1u) return ST_OK;
+  ST_CUDA(cudaFuncSetAttribute(*fn, cudaFuncAttributeMaxDynamicSharedMemorySize, kTuneStageBytes));
+  ready |= 1u << cls;
+  return ST_OK;
+}
+
 // One end-cell pass of a plan: every 16-bit class (side by side on the fork set), then the exact 32-bit kernel over
 // its list, which holds the pairs that are not eligible for 16 bits and those the forward pass found above the
 // headroom.
@@ -2852,8 +2856,9 @@ static int end_pass(st_plan* p, st_ctx::ForkSet* fs, cudaStream_t st, bool rev, 
     prm.rev_q = arrays.rev_q;
     prm.rev_t = arrays.rev_t;
     prm.rev_score = arrays.rev_score;
-    const Sw16EndFns* f = end_fns(cp.cls);
-    (rev ? f->rev : f->fwd)<<<cp.grid, kClasses[cp.cls].W * 32, cp.smem, s>>>(prm);
+    Sw16Fn fn = nullptr;
+    ST_TRY(end_kernel(p->ctx, cp.cls, rev, &fn));
+    fn<<<cp.grid, kClasses[cp.cls].W * 32, cp.smem, s>>>(prm);
     ST_CUDA(cudaGetLastError());
   }
   for (size_t i = 1; i < order.size(); ++i) {
@@ -3294,7 +3299,7 @@ static int launch_ungapped(st_ctx* c, bool hits, const void* d_jobs, uint64_t n,
     prm.chunk = diag_chunk(c, n);
     ungapped_hits_refill_kernel<<<static_cast<uint32_t>((n + prm.chunk - 1) / prm.chunk), 256, smem, c->stream>>>(prm);
   } else
-    ungapped_kernel<false><<<static_cast<uint32_t>(grid), 256, smem, c->stream>>>(prm);
+    ungapped_kernel<<<static_cast<uint32_t>(grid), 256, smem, c->stream>>>(prm);
   ++c->launches;
   ST_CUDA(cudaGetLastError());
   return ST_OK;
@@ -4013,8 +4018,12 @@ static int seed_stage(st_ctx* c, const uint32_t* profiles, uint32_t n_q, const u
   SeedSeed* seeds = reinterpret_cast<SeedSeed*>(b2 + o_seeds);
   uint32_t* cnt = reinterpret_cast<uint32_t*>(b2 + o_cnt);
   uint32_t* hoff = reinterpret_cast<uint32_t*>(b2 + o_hoff);
+  const uint32_t emit_smem = 2 * Q.cap * static_cast<uint32_t>(sizeof(int2));
+  if (Q.cap <= kSeedWarpCap && emit_smem > 40 * 1024)  // past what a launch may have without asking
+    ST_CUDA(cudaFuncSetAttribute(seed_emit_warp_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 2 * kSeedWarpCap * static_cast<int>(sizeof(int2))));
   if (ns && Q.cap <= kSeedWarpCap)
-    seed_emit_warp_kernel<<<win_ctas, 32, 2 * Q.cap * sizeof(int2), s>>>(Q, P, soff, win, seeds, st);
+    seed_emit_warp_kernel<<<win_ctas, 32, emit_smem, s>>>(Q, P, soff, win, seeds, st);
   else if (ns)
     seed_emit_kernel<<<grid_for(nw, 128), 128, 0, s>>>(Q, P, soff, win, seeds, st);
   seed_post_count_kernel<<<grid_for(ns + 1, 256), 256, 0, s>>>(seeds, static_cast<uint32_t>(ns),

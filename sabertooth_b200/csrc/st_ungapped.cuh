@@ -44,42 +44,10 @@ struct UngappedParams {
 
 constexpr int kUngChunk = 1024;  // jobs per CTA chunk
 
-template <bool HITS>
-__device__ __forceinline__ void ung_job(const UngappedParams& prm, uint64_t k, uint32_t& q, uint32_t& t,
-                                        int32_t& d, int64_t& lo, int64_t& hi) {
-  if constexpr (HITS) {
-    const HitRec h = reinterpret_cast<const HitRec*>(prm.jobs)[k];
-    q = h.query;
-    t = h.target;
-    d = h.diag;
-    const int64_t m = prm.prof.qlen[q];
-    const int64_t n = prm.db.length[t];
-    // diag_range, src/ungapped.rs:38-46
-    lo = i64max(-static_cast<int64_t>(d), 0);
-    hi = i64min(m, n - d);
-    if (hi <= lo) lo = hi = 0;
-  } else {
-    const UngappedJob j = reinterpret_cast<const UngappedJob*>(prm.jobs)[k];
-    q = j.query;
-    t = j.target;
-    d = j.diag;
-    lo = j.lo;
-    hi = j.hi;
-  }
-}
-
-template <bool HITS>
-__device__ __forceinline__ uint32_t ung_query(const UngappedParams& prm, uint64_t k) {
-  if constexpr (HITS)
-    return reinterpret_cast<const HitRec*>(prm.jobs)[k].query;
-  else
-    return reinterpret_cast<const UngappedJob*>(prm.jobs)[k].query;
-}
-
-template <bool HITS>
 __global__ void __launch_bounds__(256) ungapped_kernel(const UngappedParams prm) {
   extern __shared__ __align__(16) int8_t smem[];
   __shared__ uint32_t s_run_end;
+  const UngappedJob* jobs = reinterpret_cast<const UngappedJob*>(prm.jobs);
   const uint32_t stride = prm.max_m_pad;
   int8_t* base = smem + 16;  // 16 guard bytes before row 0
   const uint64_t c0 = static_cast<uint64_t>(blockIdx.x) * kUngChunk;
@@ -87,13 +55,13 @@ __global__ void __launch_bounds__(256) ungapped_kernel(const UngappedParams prm)
   const uint64_t c1 = u64min(prm.n, c0 + kUngChunk);
   uint64_t a = c0;
   while (a < c1) {
-    const uint32_t q = ung_query<HITS>(prm, a);
+    const uint32_t q = jobs[a].query;
     // end of this query's run inside the chunk (warp 0 scans 32 jobs at a time)
     if (threadIdx.x < 32) {
       uint64_t e = a;
       for (;;) {
         const uint64_t k = e + threadIdx.x;
-        const bool same = (k < c1) && (ung_query<HITS>(prm, k) == q);
+        const bool same = (k < c1) && (jobs[k].query == q);
         const uint32_t ball = __ballot_sync(0xFFFFFFFFu, same);
         if (ball != 0xFFFFFFFFu) {
           e += __ffs(~ball) - 1;
@@ -125,32 +93,12 @@ __global__ void __launch_bounds__(256) ungapped_kernel(const UngappedParams prm)
     const int32_t s32 = static_cast<int32_t>(prm.prof.stride32[q]);
     const int32_t last_row = static_cast<int32_t>(m) - 1;
     for (uint64_t k = a + threadIdx.x; k < b; k += blockDim.x) {
-      uint32_t qq, tt;
-      int32_t d;
-      int64_t lo, hi;
-      ung_job<HITS>(prm, k, qq, tt, d, lo, hi);
+      const UngappedJob j = jobs[k];
+      const int32_t d = j.diag;
+      const int64_t lo = j.lo, hi = j.hi;
       int32_t best = 0, cur = 0;
-      if (HITS && hi > lo && narrow) {
-        // Whole-diagonal windows (hits) on int8 profiles: every cell of a vector outside [lo, hi) scores
-        // 0 on its own: query rows before 0 or from m read the zero guard bytes and padding of the staged
-        // rows, target positions from n hold the sentinel code, whose row is zero. Zero cells at either
-        // end of the window cannot change Kadane's maximum, so whole vectors are scored without a test.
-        const uint8_t* tp = prm.db.arena + prm.db.offset[tt];
-        const int32_t p0 = static_cast<int32_t>(lo) + d, p1 = static_cast<int32_t>(hi) + d;
-        for (int32_t pa = p0 & ~15; pa < p1; pa += 16) {
-          const uint4 v = *reinterpret_cast<const uint4*>(tp + pa);
-          const uint32_t w[4] = {v.x, v.y, v.z, v.w};
-          const int8_t* rowbase = base + (pa - d);
-#pragma unroll
-          for (int bb = 0; bb < 16; ++bb) {
-            const uint32_t r = (w[bb >> 2] >> ((bb & 3) * 8)) & 0xFFu;
-            const int32_t sc = rowbase[static_cast<int32_t>(r * stride) + bb];
-            cur = wadd(max(cur, 0), sc);
-            best = max(best, cur);
-          }
-        }
-      } else if (hi > lo) {
-        const uint8_t* tp = prm.db.arena + prm.db.offset[tt];
+      if (hi > lo) {
+        const uint8_t* tp = prm.db.arena + prm.db.offset[j.target];
         // target positions [p0, p1); sequences are shorter than 2^31
         const int32_t p0 = static_cast<int32_t>(lo) + d, p1 = static_cast<int32_t>(hi) + d;
         int32_t pa = p0 & ~15;
