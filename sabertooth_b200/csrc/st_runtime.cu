@@ -283,6 +283,7 @@ static const Sw16EndFns* end_fns(int cls) {
   return nullptr;
 }
 constexpr uint32_t kEndMaxLen = 65535;  // an end cell's column travels in 16 bits
+constexpr int kEndOutputs = 6;          // words a pair that come back from a span call
 
 static_assert(kNumClasses <= kMaxTileClasses, "tile classes exceed the tuning arrays");
 
@@ -1367,12 +1368,20 @@ static int plan_enqueue(st_plan* p, cudaStream_t st, st_ctx::ForkSet* fs, bool g
   return cudaGetLastError() == cudaSuccess ? ST_OK : ST_ECUDA;
 }
 
-static int fork_set(st_ctx* c, int i, st_ctx::ForkSet** out) {
+// The fork streams that a plan's launches use beside the launching one.
+static int plan_forks(const st_plan* p) {
+  const int n = static_cast<int>(p->classes.size()) + (p->p32.band16 ? 1 : 0) - 1;
+  return std::max(0, std::min(n, st_ctx::ForkSet::kForks));
+}
+
+// Fork set i with at least `n` streams, each made when a launch first needs it (a whole set is most of a
+// millisecond of a context's first call).
+static int fork_set(st_ctx* c, int i, int n, st_ctx::ForkSet** out) {
   st_ctx::ForkSet& f = c->forks[i];
-  for (auto& s : f.s)
-    if (!s) ST_CUDA(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
-  for (auto& e : f.ev)
-    if (!e) ST_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+  for (int k = 0; k < n; ++k)
+    if (!f.s[k]) ST_CUDA(cudaStreamCreateWithFlags(&f.s[k], cudaStreamNonBlocking));
+  for (int k = 0; n && k <= n; ++k)
+    if (!f.ev[k]) ST_CUDA(cudaEventCreateWithFlags(&f.ev[k], cudaEventDisableTiming));
   *out = &f;
   return ST_OK;
 }
@@ -1380,7 +1389,8 @@ static int fork_set(st_ctx* c, int i, st_ctx::ForkSet** out) {
 // Builds a plan for `n` pairs. Its initialised data is staged in pinned block
 // `slot` of the context's ring and uploaded on `up`; the block is reused only
 // after that copy has finished (an event per block).
-// With `ends` the plan is for the end-cell modes: their tile classes only, targets they can address.
+// With `ends` the plan is for the end-cell modes: their tile classes only, targets they can address, and a caller
+// that waits for the stream before it uses the context's pinned block or returns.
 static int plan_build(st_ctx* c, const st_pair* pairs, uint64_t n, int32_t open, int32_t ext, int32_t* d_scores,
                       uint32_t* d_kernels, st_plan** out, bool capture, cudaStream_t up, int slot,
                       bool ends = false) {
@@ -1819,13 +1829,21 @@ static int plan_build(st_ctx* c, const st_pair* pairs, uint64_t n, int32_t open,
   ST_TRY(pool_get(c, total_bytes, plan->arena));
   tc.lap("arena");
   char* dbase = plan->arena.as<char>();
-  // stage the data region in pinned memory and upload it at once
-  Pinned& pin = c->plan_pin[slot];
-  if (!c->plan_pin_ev[slot]) ST_CUDA(cudaEventCreateWithFlags(&c->plan_pin_ev[slot], cudaEventDisableTiming));
-  if (c->plan_pin_used[slot]) ST_CUDA(cudaEventSynchronize(c->plan_pin_ev[slot]));  // may still feed a copy
-  c->plan_pin_used[slot] = false;
-  ST_TRY(pin.reserve(data_bytes));
-  char* h = pin.as<char>();
+  // stage the data region in pinned memory and upload it at once.  End-cell calls wait for their work before they
+  // return, so where the ring's block would have to grow and the context's own has room, behind the results that come
+  // back through it, they use that (making a pinned block takes 2 ms, three times a small call).
+  const size_t pin_off = ends ? up256(n * 4 * kEndOutputs) : 0;
+  const bool own_pin = ends && c->plan_pin[slot].bytes < data_bytes && c->pin.bytes >= pin_off + data_bytes;
+  Pinned& pin = own_pin ? c->pin : c->plan_pin[slot];
+  if (own_pin) {
+    ST_CUDA(cudaStreamSynchronize(c->stream));  // may still feed a copy
+  } else {
+    if (!c->plan_pin_ev[slot]) ST_CUDA(cudaEventCreateWithFlags(&c->plan_pin_ev[slot], cudaEventDisableTiming));
+    if (c->plan_pin_used[slot]) ST_CUDA(cudaEventSynchronize(c->plan_pin_ev[slot]));  // may still feed a copy
+    c->plan_pin_used[slot] = false;
+    ST_TRY(pin.reserve(data_bytes));
+  }
+  char* h = pin.as<char>(own_pin ? pin_off : 0);
 #pragma omp parallel sections
   {
 #pragma omp section
@@ -1858,8 +1876,10 @@ static int plan_build(st_ctx* c, const st_pair* pairs, uint64_t n, int32_t open,
     }
   }
   ST_CUDA(cudaMemcpyAsync(dbase, h, data_bytes, cudaMemcpyHostToDevice, up));
-  ST_CUDA(cudaEventRecord(c->plan_pin_ev[slot], up));
-  c->plan_pin_used[slot] = true;
+  if (!own_pin) {
+    ST_CUDA(cudaEventRecord(c->plan_pin_ev[slot], up));
+    c->plan_pin_used[slot] = true;
+  }
   tc.lap("stage+upload");
   plan->counters = reinterpret_cast<uint32_t*>(dbase + o_cnt);
   plan->counters_init = reinterpret_cast<const uint32_t*>(dbase + o_cinit);
@@ -1940,7 +1960,7 @@ static int plan_build(st_ctx* c, const st_pair* pairs, uint64_t n, int32_t open,
     ST_CUDA(cudaStreamSynchronize(up));
     ST_CUDA(cudaStreamBeginCapture(c->own, cudaStreamCaptureModeThreadLocal));
     st_ctx::ForkSet* fs = nullptr;
-    ST_TRY(fork_set(c, 0, &fs));
+    ST_TRY(fork_set(c, 0, plan_forks(plan.get()), &fs));
     const int rc = plan_enqueue(plan.get(), c->own, fs, true);
     cudaError_t ce = cudaStreamEndCapture(c->own, &plan->graph);
     if (rc != ST_OK || ce != cudaSuccess)
@@ -1957,7 +1977,7 @@ static int plan_run(st_plan* p) {
     ST_CUDA(cudaGraphLaunch(p->exec, c->stream));
   } else {
     st_ctx::ForkSet* fs = nullptr;
-    ST_TRY(fork_set(c, 0, &fs));
+    ST_TRY(fork_set(c, 0, plan_forks(p), &fs));
     if (plan_enqueue(p, c->stream, fs) != ST_OK)
       return fail(ST_ECUDA, "plan launch failed: %s", cudaGetErrorString(cudaGetLastError()));
   }
@@ -2721,7 +2741,7 @@ extern "C" int st_sw_score_pairs(st_ctx* c, const st_pair* pairs, uint64_t n, in
       plans.emplace_back(p, plan_free);
       if (!tev.empty()) cudaEventRecord(tev[1 + 2 * k], s);
       st_ctx::ForkSet* fs = nullptr;
-      rc = fork_set(c, 1 + static_cast<int>(k % n_side), &fs);
+      rc = fork_set(c, 1 + static_cast<int>(k % n_side), plan_forks(p), &fs);
       if (rc != ST_OK) break;
       if (plan_enqueue(p, s, fs) != ST_OK) {
         rc = fail(ST_ECUDA, "plan launch failed: %s", cudaGetErrorString(cudaGetLastError()));
@@ -2896,7 +2916,7 @@ static int end_pairs_entry(st_ctx* c, const st_pair* pairs, uint64_t n, int32_t 
   if (n > 0xFFFFFFF0ull) return fail(ST_EINVAL, "too many pairs");
   ST_TRY(sync_profiles(c));
   // [scores] [query ends] [target ends] and with spans [reverse scores] [the same of the reverse pass]
-  const int k_out = span ? 6 : 3;
+  const int k_out = span ? kEndOutputs : 3;
   DevMem out, work;
   st_plan* plan = nullptr;
   struct Back {  // on every exit: nothing queued still uses the buffers when they return to the pool
@@ -2924,7 +2944,7 @@ static int end_pairs_entry(st_ctx* c, const st_pair* pairs, uint64_t n, int32_t 
     ST_TRY(plan_build(c, pairs, n, open, ext, d_s, nullptr, &plan, false, c->stream, 0, true));
   cudaStream_t st = c->stream;
   st_ctx::ForkSet* fs = nullptr;
-  ST_TRY(fork_set(c, 0, &fs));
+  ST_TRY(fork_set(c, 0, static_cast<int>(plan->classes.size()) - 1, &fs));
   ST_CUDA(cudaMemsetAsync(d_s, 0, n * 4, st));
   ST_CUDA(cudaMemsetAsync(d_eq, 0xFF, n * 8, st));  // -1: a pair without a positive score has no cells
   ST_CUDA(cudaMemcpyAsync(plan->counters, plan->counters_init, (kNumClasses + 2) * 4, cudaMemcpyDeviceToDevice, st));
