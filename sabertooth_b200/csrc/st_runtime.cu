@@ -1386,6 +1386,9 @@ static int fork_set(st_ctx* c, int i, int n, st_ctx::ForkSet** out) {
   return ST_OK;
 }
 
+// Below this many pairs a planning loop runs on the calling thread: waking a team costs more than it saves.
+constexpr uint64_t kSerialPairs = 2048;
+
 // Builds a plan for `n` pairs. Its initialised data is staged in pinned block
 // `slot` of the context's ring and uploaded on `up`; the block is reused only
 // after that copy has finished (an event per block).
@@ -1435,7 +1438,7 @@ static int plan_build(st_ctx* c, const st_pair* pairs, uint64_t n, int32_t open,
   int32_t min_radius = INT32_MAX;
   // classify every pair (validation, route, cells), in parallel
 #pragma omp parallel for schedule(static) reduction(+ : cells, cells32) reduction(max : max_len, max_m32) \
-    reduction(min : min_radius)
+    reduction(min : min_radius) if (n > kSerialPairs)
   for (int64_t i = 0; i < static_cast<int64_t>(n); ++i) {
     const st_pair& p = pairs[i];
     if (p.profile >= n_prof || !c->profs[p.profile].live || p.target >= c->n_seqs) {
@@ -1515,7 +1518,7 @@ static int plan_build(st_ctx* c, const st_pair* pairs, uint64_t n, int32_t open,
   list32.resize(ps.n32[nt]);
   std::vector<uint32_t>& byq = ps.byq;
   byq.resize(qstart[n_prof]);
-#pragma omp parallel for schedule(static)
+#pragma omp parallel for schedule(static) if (n_prof > kSerialPairs)
   for (int64_t q = 0; q < static_cast<int64_t>(n_prof); ++q) {
     uint64_t o = qstart[q];
     for (int t = 0; t < nt; ++t) {
@@ -1542,7 +1545,7 @@ static int plan_build(st_ctx* c, const st_pair* pairs, uint64_t n, int32_t open,
   // The packed band kernel scores neighbouring entries together, so similar pairs share a warp.
   if (list32.size() > 1) {
     std::vector<std::pair<uint64_t, uint32_t>> ord(list32.size());
-#pragma omp parallel for schedule(static)
+#pragma omp parallel for schedule(static) if (list32.size() > kSerialPairs)
     for (int64_t k = 0; k < static_cast<int64_t>(list32.size()); ++k) {
       const uint32_t i = list32[k];
       const uint64_t m = c->profs[pq[i]].m, tl = tlen[i];
@@ -1568,7 +1571,7 @@ static int plan_build(st_ctx* c, const st_pair* pairs, uint64_t n, int32_t open,
   std::vector<double>& est = ps.est;  // per query and class: the chip's time for it, picoseconds
   est.resize(qlist.size() * kNumClasses);
   double batch_ps = 0.0;              // the batch's time with every query in its cheapest class
-#pragma omp parallel for schedule(dynamic, 8) reduction(+ : batch_ps)
+#pragma omp parallel for schedule(dynamic, 8) reduction(+ : batch_ps) if (qlist.size() > 8)
   for (int64_t k = 0; k < static_cast<int64_t>(qlist.size()); ++k) {
     const uint32_t q = qlist[k];
     uint32_t* v0 = byq.data() + qstart[q];
@@ -1585,21 +1588,27 @@ static int plan_build(st_ctx* c, const st_pair* pairs, uint64_t n, int32_t open,
     batch_ps += tuning_estimate(&c->tuning, c->profs[q].m, tl_desc.data(), tl_desc.size(), &est[k * kNumClasses],
                                 class_mask(ends));
   }
+  // the picks (30 classes a query, some 0.3 us), then what they say of each class
+#pragma omp parallel for schedule(static) if (qlist.size() > 64)
+  for (int64_t k = 0; k < static_cast<int64_t>(qlist.size()); ++k) {
+    const uint32_t q = qlist[k];
+    const uint32_t m = c->profs[q].m;
+    const uint32_t mean_n = static_cast<uint32_t>(qsum[k] / (qstart[q + 1] - qstart[q]));
+    int cls = tuning_pick_batch(&c->tuning, m, tlen[byq[qstart[q]]], mean_n, &est[k * kNumClasses], batch_ps);
+    if (cls < 0) cls = tuning_pick_single(&c->tuning, m, mean_n);  // no class stages it: the wavefront model
+    qclass[k] = cls;
+  }
   int toolong = -1;
   double class_path[kNumClasses] = {};
   for (size_t k = 0; k < qlist.size(); ++k) {
-    const uint32_t q = qlist[k];
-    const uint32_t m = c->profs[q].m;
-    const uint64_t np = qstart[q + 1] - qstart[q];
-    const uint32_t mean_n = static_cast<uint32_t>(qsum[k] / np);
-    int cls = tuning_pick_batch(&c->tuning, m, tlen[byq[qstart[q]]], mean_n, &est[k * kNumClasses], batch_ps);
-    if (cls < 0) cls = tuning_pick_single(&c->tuning, m, mean_n);  // no class stages it: the wavefront model
+    const uint32_t m = c->profs[qlist[k]].m;
+    const int cls = qclass[k];
     const uint32_t rows = kClasses[cls].G * kClasses[cls].R;
     const uint32_t P = (m + rows - 1) / rows;
     if (static_cast<uint64_t>(kProfRows) * P * rows > static_cast<uint64_t>(g_class_smem[cls]))
       toolong = static_cast<int>(m);
-    qclass[k] = cls;
-    class_path[cls] = std::max(class_path[cls], class_crit(cls, P * rows, std::max<uint32_t>(32, up4(tlen[byq[qstart[q]]]))));
+    class_path[cls] = std::max(class_path[cls],
+                               class_crit(cls, P * rows, std::max<uint32_t>(32, up4(tlen[byq[qstart[qlist[k]]]]))));
   }
   plan->batch_ps = batch_ps;
   if (toolong >= 0) return fail(ST_EINVAL, "query of %d rows does not fit the shared-memory profile", toolong);
@@ -1650,7 +1659,7 @@ static int plan_build(st_ctx* c, const st_pair* pairs, uint64_t n, int32_t open,
   auto wt_cost = [&](const QShape& sh, uint32_t ncols) {
     return static_cast<uint64_t>(sh.P) * (ncols / sh.C) * sh.step_cost;
   };
-#pragma omp parallel for schedule(dynamic, 16)
+#pragma omp parallel for schedule(dynamic, 16) if (n > kSerialPairs)
   for (int64_t k = 0; k < static_cast<int64_t>(qlist.size()); ++k) {
     const QShape sh = shape_of(k);
     const uint64_t np = qstart[qlist[k] + 1] - qstart[qlist[k]];
@@ -1693,7 +1702,7 @@ static int plan_build(st_ctx* c, const st_pair* pairs, uint64_t n, int32_t open,
     }
     if (n_wt > w0) f(w0, n_wt, acc - start);
   };
-#pragma omp parallel for schedule(dynamic, 16)
+#pragma omp parallel for schedule(dynamic, 16) if (n > kSerialPairs)
   for (int64_t k = 0; k < static_cast<int64_t>(qlist.size()); ++k) {
     uint32_t n = 0;
     for_each_cta(k, shape_of(k), [&](uint32_t, uint32_t, uint64_t) { ++n; });
@@ -1722,7 +1731,7 @@ static int plan_build(st_ctx* c, const st_pair* pairs, uint64_t n, int32_t open,
     cps[k].cta.resize(n_cta_cls[k]);
     cta_cost[k].resize(n_cta_cls[k]);
   }
-#pragma omp parallel for schedule(dynamic, 16)
+#pragma omp parallel for schedule(dynamic, 16) if (n > kSerialPairs)
   for (int64_t k = 0; k < static_cast<int64_t>(qlist.size()); ++k) {
     const uint32_t q = qlist[k];
     const int cls = qclass[k];
@@ -1844,7 +1853,7 @@ static int plan_build(st_ctx* c, const st_pair* pairs, uint64_t n, int32_t open,
     ST_TRY(pin.reserve(data_bytes));
   }
   char* h = pin.as<char>(own_pin ? pin_off : 0);
-#pragma omp parallel sections
+#pragma omp parallel sections if (n > 4 * kSerialPairs)
   {
 #pragma omp section
     memcpy(h + o_pq, pq.data(), n * 4);
@@ -1869,7 +1878,7 @@ static int plan_build(st_ctx* c, const st_pair* pairs, uint64_t n, int32_t open,
     const size_t ns = cp.slots.size();
     const Sw16Slot* src = cp.slots.data();
     Sw16Slot* dst = reinterpret_cast<Sw16Slot*>(h + cp.o_slots);
-#pragma omp parallel for schedule(static)
+#pragma omp parallel for schedule(static) if (ns > 65536)
     for (int64_t b = 0; b < static_cast<int64_t>((ns + 65535) / 65536); ++b) {
       const size_t a0 = static_cast<size_t>(b) * 65536, a1 = std::min(ns, a0 + 65536);
       memcpy(dst + a0, src + a0, (a1 - a0) * sizeof(Sw16Slot));
