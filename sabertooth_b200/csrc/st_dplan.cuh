@@ -313,9 +313,10 @@ __global__ void __launch_bounds__(256) dp_pick_kernel(const DpIn in, const DpWor
   }
 }
 
-// CTA tasks of one query, by one warp: consecutive warp tasks in units of tune_cta_unit (a team class: one each); a
-// task ends at 128 warp tasks or where the query's running cost passes a multiple of the class's cap (its cost over two CTAs on every
-// SM).  f(t, w0, w1, cost) is called once for each task t by some lane; returns the number of tasks.
+// CTA tasks of one query, by one warp: consecutive warp tasks in units of tune_cta_unit (a team class: one each), a task
+// for each in a small batch (tune_cta_single); else a task ends at 128 warp tasks or at the unit nearest to where the
+// query's running cost passes a multiple of the class's cap (its cost over two CTAs on every SM).
+// f(t, w0, w1, cost) is called once for each task t by some lane; returns the number of tasks.
 template <class F>
 __device__ __forceinline__ uint32_t dp_for_each_cta(const DpClasses& cls, const DpTotals* tot, uint32_t k,
                                                     const DpShape& sh, uint32_t nw, const DpLens& tl, F&& f) {
@@ -325,6 +326,8 @@ __device__ __forceinline__ uint32_t dp_for_each_cta(const DpClasses& cls, const 
   wt_total = dp_warp_sum(wt_total);
   const uint32_t unit = c.team ? 1u : tune_cta_unit(wt_total, cls.sms, c.W);
   const unsigned long long cap = max(1ull, tot->cost[k] / (2ull * cls.sms));
+  const bool single = c.team || tune_cta_single(wt_total, cls.sms, c.W);
+  const unsigned long long half = unit * dp_wt_cost(c, sh, tl(0)) / 2;
   unsigned long long base = 0;         // cost of the warp tasks before this round's
   unsigned long long last_bucket = 0;  // of the last unit of the round before
   unsigned long long open_cost = 0;    // running cost at the start of the open task
@@ -339,10 +342,10 @@ __device__ __forceinline__ uint32_t dp_for_each_cta(const DpClasses& cls, const 
       if (lane >= o) incl += y;
     }
     const unsigned long long excl = base + incl - cw;
-    const unsigned long long bucket = excl / cap;
+    const unsigned long long bucket = (excl + half) / cap;
     unsigned long long before = __shfl_up_sync(0xFFFFFFFFu, bucket, unit);
     if (lane < static_cast<int>(unit)) before = last_bucket;
-    const bool begin = x < nw && x % unit == 0 && (x == 0 || bucket != before || x % 128u == 0 || c.team);
+    const bool begin = x < nw && x % unit == 0 && (x == 0 || single || bucket != before || x % 128u == 0);
     const uint32_t mask = __ballot_sync(0xFFFFFFFFu, begin);
     const uint32_t lower = mask & ((1u << lane) - 1u);
     // the task before mine: begun by the next lower lane of the ballot, or the open one

@@ -1622,8 +1622,9 @@ static int plan_build(st_ctx* c, const st_pair* pairs, uint64_t n, int32_t open,
   }
   // Emission. A query's pairs (sorted by target length, longest first) form
   // warp tasks of S = 64/G pairs; consecutive warp tasks form CTA tasks, in units
-  // of tune_cta_unit warp tasks. A CTA task ends at 128 warp tasks, or where the
-  // query's running cost passes a multiple of the class's cap: one CTA's share of
+  // of tune_cta_unit warp tasks: one each in a small batch (tune_cta_single), else a CTA
+  // task ends at 128 warp tasks, or at the unit nearest to where the query's
+  // running cost passes a multiple of the class's cap: one CTA's share of
   // the class's total cost on a grid of two CTAs per SM. The cap keeps a long
   // query from becoming one CTA task longer than the rest of the launch (the
   // tail); a finer split would pay the ramp, drain and barrier wait of a CTA
@@ -1686,12 +1687,14 @@ static int plan_build(st_ctx* c, const st_pair* pairs, uint64_t n, int32_t open,
     const uint64_t cp = cap[qclass[k]];
     const Sw16Class& kc = kClasses[qclass[k]];
     const uint32_t unit = kc.team ? 1u : tune_cta_unit(wt_total, c->sms, kc.W);
+    const bool single = kc.team || tune_cta_single(wt_total, c->sms, kc.W);
+    const uint64_t half = n_wt ? unit * wt_cost(sh, wt_cols(k, sh, 0)) / 2 : 0;  // of a unit: ends where it is nearest
     uint32_t w0 = 0;
     uint64_t acc = 0, start = 0, bucket = 0;
     for (uint32_t w = 0; w < n_wt; ++w) {
       if (w % unit == 0) {
-        const uint64_t bk = acc / cp;
-        if (w > 0 && (bk != bucket || w % kMaxWtPerCta == 0 || kc.team)) {
+        const uint64_t bk = (acc + half) / cp;
+        if (w > 0 && (single || bk != bucket || w % kMaxWtPerCta == 0)) {
           f(w0, w, acc - start);
           w0 = w;
           start = acc;

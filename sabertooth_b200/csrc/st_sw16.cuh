@@ -348,7 +348,7 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 4 || (R == 8 && MODE == k
         *reinterpret_cast<uint4*>(prof_s + static_cast<size_t>(r) * m_pad + i) = v;
       }
     }
-    if (threadIdx.x == 0) s_next = task.wt_begin;
+    if (threadIdx.x == 0) s_next = task.wt_begin + WARPS;
     if constexpr (TEAM) {
       if (threadIdx.x < WARPS) s_prog[threadIdx.x] = 0;
       if (threadIdx.x == 0) {
@@ -368,13 +368,15 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 4 || (R == 8 && MODE == k
     // neighbour's outputs.
     const bool feeder = gl == G - 1;
     const int src_lane = (lane & ~(G - 1)) | ((lane - 1) & (G - 1));
+    // a warp's first warp task goes by its number, so that a task of few has them on different schedulers and no warp
+    // has two while another has none; the others are claimed
     auto claim = [&]() -> uint32_t {
       uint32_t w = 0;
       if (lane == 0) w = atomicAdd(&s_next, 1u);
       return __shfl_sync(FULL, w, 0);
     };
     // a team's warps share the CTA task's one warp task: warp w takes its passes w, w + WARPS, ...
-    uint32_t w_cur = TEAM ? task.wt_begin : claim();
+    uint32_t w_cur = __shfl_sync(FULL, task.wt_begin + (TEAM ? 0u : static_cast<uint32_t>(warp)), 0);
     bool have = TEAM ? warp < P : w_cur < task.wt_end;
     if (have) {
     auto load_pairs = [&](uint32_t slot_begin) {

@@ -152,12 +152,20 @@ TUNE_HD inline double tune_objective(double est_ps, double crit_ps, double batch
   return est_ps + (over > 0.0 ? 0.1 * over : 0.0);
 }
 
-// Warp tasks per unit of a CTA task: a CTA's warps, fewer (a power of two) when the batch has not that many for
-// two CTAs on every SM, so that a small batch spreads over the chip.
+// Warp tasks per unit of a CTA task: a CTA's warps, fewer (a power of two) while the batch would leave an SM without
+// a unit, so that a small batch spreads over the chip.
 TUNE_HD inline uint32_t tune_cta_unit(uint64_t wt_total, uint32_t sms, uint32_t W) {
   uint32_t u = W;
-  while (u > 1 && static_cast<uint64_t>(u) * 2 * sms > wt_total) u >>= 1;
+  while (u > 1 && static_cast<uint64_t>(u / 2) * sms >= wt_total) u >>= 1;
   return u;
+}
+
+// Whether every unit is a CTA task of its own: the whole batch is no more than the warps that are resident at once
+// (two CTAs of eight warps on an SM, three of four).  A second unit in a task would be a second round of its warps
+// while others have none; in larger batches it saves staging the query again (100 queries x 100 targets of 250 x 300 in
+// <8,32>: 428 us with two units in most tasks, 233 with one; 600 queries x 300 of mixed lengths: 4.75 ms with one, 4.37).
+TUNE_HD inline bool tune_cta_single(uint64_t wt_total, uint32_t sms, uint32_t W) {
+  return wt_total <= static_cast<uint64_t>(sms) * (W < 8 ? 12 : 16);
 }
 
 // est[c] = the chip's time (ps) for the query in class c: streamed cells over the rate; a class without a rate
