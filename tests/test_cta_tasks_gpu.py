@@ -1,6 +1,6 @@
 """How a query's warp tasks are cut into CTA tasks: batches below, at and above what is resident at once, one and many
-queries, target counts around a unit's, several classes, with both planners, against the oracle; and no second round
-of a CTA's warps where a batch fits the chip."""
+queries, target counts around a unit's, several classes, with both planners, against the oracle; and no warp task that
+waits for another where the chip has schedulers for all."""
 import numpy as np
 import pytest
 import torch
@@ -47,24 +47,24 @@ def test_scores(ctx, shape, nq, nt):
     assert np.array_equal(got, want)
 
 
-def test_three_in_turn_take_three_times_as_long(ctx):
-    """100 queries x 100 targets in <8,32> are 1,300 warp tasks on 592 schedulers, three in turn at most, in CTAs of four
-    warps whose cap is 4.4 warp tasks.  Cut into tasks of two units they took two rounds of a CTA each, 4.6 times as
-    long as one warp task a query."""
+def test_fewer_warp_tasks_than_schedulers(ctx):
+    """100 queries x 30 targets in <8,32> are 400 warp tasks, four a query, in CTAs of four warps: with 592 schedulers none
+    waits for another, so they take as long as the 100 of 100 queries x 8 targets.  Units of one warp task, two or
+    three of them in a CTA task by the class's cap, took 1.7 to 2.4 times as long."""
     m = blosum62()
     rng = np.random.default_rng(4)
-    ctx.upload_db_list([rng.integers(0, 20, 300).astype(np.uint8) for _ in range(100)])
+    ctx.upload_db_list([rng.integers(0, 20, 300).astype(np.uint8) for _ in range(30)])
     ids = ctx.create_profiles([m.sequence_rows(rng.integers(0, 20, 250).astype(np.uint8)) for _ in range(100)])
     saved = ctx.tuning_table()
     ms = {}
     try:
         ctx.set_tuning_table(np.full((10, 8), [c[:2] for c in tile_classes()].index((8, 32)), dtype=np.int32))
-        for n in (8, 100):
+        for n in (8, 30):
             d = torch.zeros(n * 100, dtype=torch.int32, device="cuda")
             plan = ctx.plan(all_pairs(ids, n), GapCosts(11, 1), d.data_ptr())
-            ms[n] = min(plan.profile()[0][2] for _ in range(7))
+            ms[n] = np.median([plan.profile()[0][2] for _ in range(9)])
             plan.close()
     finally:
         ctx.set_tuning_table(saved)
         ctx.free_profiles(ids)
-    assert ms[100] < 3.5 * ms[8], ms
+    assert ms[30] < 1.4 * ms[8], ms
