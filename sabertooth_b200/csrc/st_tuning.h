@@ -152,10 +152,14 @@ TUNE_HD inline double tune_objective(double est_ps, double crit_ps, double batch
   return est_ps + (over > 0.0 ? 0.1 * over : 0.0);
 }
 
-// Warp tasks per unit of a CTA task: a CTA's warps, fewer (a power of two) while the batch would leave an SM without
-// a unit, so that a small batch spreads over the chip.
+// Warp tasks per unit of a CTA task: a CTA's warps; one on each scheduler where the batch has not two CTAs of them for
+// every SM; fewer still (a power of two) while it would leave an SM without a unit, so that a small batch spreads over
+// the chip.  Two thousand warp tasks in whole CTAs leave some SMs with two and others with one (4,000 spans 1.25 ms so,
+// 1.09 by fours); one or two of eight warps at work share a scheduler while others idle (16 queries x 60 targets of 1,500 x
+// 300 361 us by twos, 192 by eights).
 TUNE_HD inline uint32_t tune_cta_unit(uint64_t wt_total, uint32_t sms, uint32_t W) {
   uint32_t u = W;
+  if (u > 4 && static_cast<uint64_t>(u) * 2 * sms > wt_total) u = 4;
   while (u > 1 && static_cast<uint64_t>(u / 2) * sms >= wt_total) u >>= 1;
   return u;
 }

@@ -72,4 +72,4 @@ def test_first_span_call_makes_no_pinned_block():
         first_call(work)  # loads the kernels
         ends = [first_call(work) for _ in range(7)]
         scores = [first_call(lambda c: c.sw_score_pairs(pairs, GapCosts(11, 1))) for _ in range(7)]
-        assert np.median(ends) < 0.5 * np.median(scores), (ends, scores)
+        assert min(ends) < 0.5 * min(scores), (ends, scores)  # host timings: a busy machine only adds to them
