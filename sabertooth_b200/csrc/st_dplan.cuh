@@ -11,8 +11,10 @@
 //   sort       radix sort of the keys (stable: equal keys keep pair order)
 //   estimate   per query and class: the chip's time for the query's streamed
 //              cells; the batch's time with every query in its cheapest class
-//   pick       per query: tile class by that time and its critical path
-//              (tune_objective), warp-task count, per-class totals (atomics)
+//   paths      the longest critical path of the queries in their cheapest classes
+//   limits     for each of 32 limits on the paths: what the queries would take
+//   pick       per query: the tile class under the best limit or by its own weight,
+//              warp-task count, per-class totals (atomics)
 //   split      per query: CTA-task count under the class's cost cap
 //   order      queries sorted by class, exclusive scans of slots, warp tasks
 //              and CTA tasks in that order (class segments are contiguous)
@@ -33,6 +35,7 @@ namespace st {
 constexpr int kDpMaxClasses = 32;
 constexpr uint32_t kDpNoClass = 63;  // sort key of a query with no 16-bit pairs
 
+static_assert(kTuneLimits == 32, "a lane for each limit");
 static_assert(kTuneMaxPasses <= kMaxPasses16, "a pass number has to fit the packed kernel's control word");
 
 struct DpClass {
@@ -61,6 +64,10 @@ struct DpTotals {
   uint32_t max_cols_multi[kDpMaxClasses];  // widest warp task of a query with several passes
   unsigned long long cost[kDpMaxClasses];  // sum of warp-task costs (the CTA-task cap)
   unsigned long long batch_ps;             // the batch's time with every query in its cheapest class
+  unsigned long long longest_path, path_sum;  // of the queries in their cheapest classes, picoseconds
+  uint32_t n_queries, n_wait;              // queries with 16-bit pairs, those that wait (tune_waits)
+  // under each limit: cell time, longest path, scheduler rounds
+  unsigned long long cells_ps[kTuneLimits], path_ps[kTuneLimits], rounds[kTuneLimits];
 };
 
 struct DpIn {
@@ -248,7 +255,75 @@ __global__ void __launch_bounds__(256) dp_estimate_kernel(const DpIn in, const D
   }
 }
 
-// ---- pick: one warp per query, a lane per class ----
+// ---- paths, limits and pick: one warp per query, a lane per class ----
+// The lane's class's cost for the query (as tuning_costs).
+__device__ __forceinline__ TuneCost dp_cost(const DpIn& in, const DpWork& w, const DpClasses& cls, uint32_t q,
+                                            uint32_t np, uint32_t longest) {
+  const int lane = threadIdx.x & 31;
+  const TuneCost none{1e300, 1e300, 1e300, 0.0};
+  if (lane >= cls.n) return none;
+  const double est = w.est[static_cast<size_t>(q) * kDpMaxClasses + lane];
+  if (est >= 1e300) return none;
+  const DpClass& c = cls.c[lane];
+  const DpShape sh = dp_shape(c, in.prof.qlen[q]);
+  return tune_cost(c.G, c.R, c.C, c.W, c.team != 0, sh.P, max(sh.minc, dp_up4(longest)), (np + c.S - 1) / c.S, est,
+                   c.rate, static_cast<double>(w.totals->batch_ps), cls.sms);
+}
+
+// The first lane of the least v; -1 when none is below 1e300.
+__device__ __forceinline__ int dp_least(double v) {
+  int k = threadIdx.x & 31;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    const double ov = __shfl_xor_sync(0xFFFFFFFFu, v, o);
+    const int ok = __shfl_xor_sync(0xFFFFFFFFu, k, o);
+    if (ov < v || (ov == v && ok < k)) {
+      v = ov;
+      k = ok;
+    }
+  }
+  return v < 1e300 ? k : -1;
+}
+
+__device__ __forceinline__ bool dp_by_limit(const DpTotals* t) {
+  return tune_alike(static_cast<double>(t->longest_path), static_cast<double>(t->path_sum), t->n_queries, t->n_wait);
+}
+
+__global__ void __launch_bounds__(256) dp_path_kernel(const DpIn in, const DpWork w, const DpClasses cls) {
+  const uint32_t q = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  if (q >= in.n_prof || w.qcnt[q] == 0) return;
+  const TuneCost c = dp_cost(in, w, cls, q, w.qcnt[q], dp_lens(in, w, q)(0));
+  const int k = dp_least(c.ps < 1e140 ? c.ps : 1e300);
+  if ((threadIdx.x & 31) != max(k, 0)) return;
+  atomicAdd(&w.totals->n_queries, 1u);
+  if (k < 0) return;
+  atomicMax(&w.totals->longest_path, static_cast<unsigned long long>(c.path) + 1);
+  atomicAdd(&w.totals->path_sum, static_cast<unsigned long long>(c.path) + 1);
+  if (tune_waits(c.path, static_cast<double>(w.totals->batch_ps))) atomicAdd(&w.totals->n_wait, 1u);
+}
+
+// A lane per limit here, for a batch whose paths are alike (classes forced by the table are not looked at).
+__global__ void __launch_bounds__(256) dp_limit_kernel(const DpIn in, const DpWork w, const DpClasses cls) {
+  const uint32_t q = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  if (q >= in.n_prof || w.qcnt[q] == 0 || !dp_by_limit(w.totals)) return;
+  const int lane = threadIdx.x & 31;
+  const TuneCost c = dp_cost(in, w, cls, q, w.qcnt[q], dp_lens(in, w, q)(0));
+  const double limit = tune_limit(static_cast<double>(w.totals->longest_path), lane);
+  TuneCost best{1e300, 1e300, 1e300, 0.0}, shortest = best;
+  for (int k = 0; k < cls.n; ++k) {
+    const double ps = __shfl_sync(0xFFFFFFFFu, c.ps, k);
+    const TuneCost x{ps, ps, __shfl_sync(0xFFFFFFFFu, c.path, k), __shfl_sync(0xFFFFFFFFu, c.rounds, k)};
+    if (x.ps >= 1e140) continue;
+    if (x.path < shortest.path) shortest = x;
+    if (x.path <= limit && x.ps < best.ps) best = x;
+  }
+  if (best.ps >= 1e140) best = shortest;
+  if (best.ps >= 1e140) return;
+  atomicAdd(&w.totals->cells_ps[lane], static_cast<unsigned long long>(best.ps));
+  atomicMax(&w.totals->path_ps[lane], static_cast<unsigned long long>(best.path));
+  atomicAdd(&w.totals->rounds[lane], static_cast<unsigned long long>(best.rounds));
+}
+
 __global__ void __launch_bounds__(256) dp_pick_kernel(const DpIn in, const DpWork w, const DpClasses cls) {
   const uint32_t q = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
@@ -273,24 +348,19 @@ __global__ void __launch_bounds__(256) dp_pick_kernel(const DpIn in, const DpWor
   if (forced >= 0 && forced < cls.n && est[forced] < 1e300) {
     best = forced;
   } else {
-    double v = 1e300;
-    if (lane < cls.n && est[lane] < 1e300) {
-      const DpClass& c = cls.c[lane];
-      const DpShape sh = dp_shape(c, m);
-      v = tune_objective(est[lane], tune_crit_ps(c.G, c.R, c.C, sh.P, max(sh.minc, dp_up4(tl(0))), c.team ? c.W : 1u),
-                         static_cast<double>(w.totals->batch_ps));
+    const TuneCost c = dp_cost(in, w, cls, q, np, tl(0));
+    const bool rated = c.est < 1e140;
+    if (dp_by_limit(w.totals)) {
+      const double limit =
+          tune_limit(static_cast<double>(w.totals->longest_path),
+                     dp_least(tune_batch_time(static_cast<double>(w.totals->cells_ps[lane]),
+                                              static_cast<double>(w.totals->path_ps[lane]),
+                                              static_cast<double>(w.totals->rounds[lane]), cls.sms)));
+      best = dp_least(rated && c.path <= limit ? c.ps : 1e300);
+      if (best < 0) best = dp_least(rated ? c.path : 1e300);
     }
-    int k = lane;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      const double ov = __shfl_xor_sync(0xFFFFFFFFu, v, o);
-      const int ok = __shfl_xor_sync(0xFFFFFFFFu, k, o);
-      if (ov < v || (ov == v && ok < k)) {
-        v = ov;
-        k = ok;
-      }
-    }
-    if (v < 1e300) best = k;
+    // by its own weight; or no class of the query has a rate
+    if (best < 0) best = dp_least(c.est < 1e300 ? tune_weighed(c, static_cast<double>(w.totals->batch_ps)) : 1e300);
   }
   if (best < 0) return;  // cannot happen: the 16-bit route admits only queries some class stages
   const DpClass& c = cls.c[best];

@@ -427,6 +427,8 @@ struct st_ctx {
     std::vector<uint64_t> qstart, n32;
     std::vector<uint32_t> hist;  // per-thread query histograms of the grouping
     std::vector<double> est;
+    std::vector<TuneCost> cost;
+    std::vector<uint8_t> front;
     std::vector<Sw16Slot> slots[32];
     std::vector<Sw16WarpTask> wt[32];
     std::vector<Sw16CtaTask> cta[32];
@@ -1588,15 +1590,73 @@ static int plan_build(st_ctx* c, const st_pair* pairs, uint64_t n, int32_t open,
     batch_ps += tuning_estimate(&c->tuning, c->profs[q].m, tl_desc.data(), tl_desc.size(), &est[k * kNumClasses],
                                 class_mask(ends));
   }
-  // the picks (30 classes a query, some 0.3 us), then what they say of each class
-#pragma omp parallel for schedule(static) if (qlist.size() > 64)
+  // every class's cost, the limit of the paths (tune_batch_time) and the picks
+  std::vector<TuneCost>& cost = ps.cost;
+  std::vector<uint8_t>& front = ps.front;  // per query: the classes that some limit picks (tuning_front)
+  std::vector<int> n_front(qlist.size());
+  cost.resize(qlist.size() * kNumClasses);
+  front.resize(qlist.size() * kNumClasses);
+  double longest_path = 0.0, path_sum = 0.0;
+  size_t n_wait = 0;
+#pragma omp parallel for schedule(static) reduction(max : longest_path) reduction(+ : path_sum, n_wait) \
+    if (qlist.size() > 64)
   for (int64_t k = 0; k < static_cast<int64_t>(qlist.size()); ++k) {
     const uint32_t q = qlist[k];
-    const uint32_t m = c->profs[q].m;
-    const uint32_t mean_n = static_cast<uint32_t>(qsum[k] / (qstart[q + 1] - qstart[q]));
-    int cls = tuning_pick_batch(&c->tuning, m, tlen[byq[qstart[q]]], mean_n, &est[k * kNumClasses], batch_ps);
-    if (cls < 0) cls = tuning_pick_single(&c->tuning, m, mean_n);  // no class stages it: the wavefront model
-    qclass[k] = cls;
+    const uint64_t np = qstart[q + 1] - qstart[q];
+    const double* ek = &est[k * kNumClasses];
+    TuneCost* ck = &cost[k * kNumClasses];
+    uint8_t* fk = &front[k * kNumClasses];
+    tuning_costs(&c->tuning, c->profs[q].m, tlen[byq[qstart[q]]], np, ek, batch_ps, c->sms, ck);
+    const int forced = tuning_forced(&c->tuning, c->profs[q].m, static_cast<uint32_t>(qsum[k] / np), ek);
+    if (forced >= 0) {
+      fk[0] = static_cast<uint8_t>(forced);
+      n_front[k] = 1;
+    } else {
+      n_front[k] = tuning_front(ck, fk);
+    }
+    if (n_front[k]) {
+      const double path = ck[fk[n_front[k] - 1]].path;
+      longest_path = std::max(longest_path, path);
+      path_sum += path;
+      n_wait += tune_waits(path, batch_ps) ? 1 : 0;
+    }
+  }
+  const bool by_limit = tune_alike(longest_path, path_sum, qlist.size(), n_wait);
+  double limits[kTuneLimits], cells_ps[kTuneLimits] = {}, rounds[kTuneLimits] = {}, path_ps[kTuneLimits] = {};
+  for (int i = 0; i < kTuneLimits; ++i) limits[i] = tune_limit(longest_path, i);
+#pragma omp parallel for schedule(static) reduction(+ : cells_ps[:kTuneLimits], rounds[:kTuneLimits]) \
+    reduction(max : path_ps[:kTuneLimits]) if (qlist.size() > 256)
+  for (int64_t k = 0; k < (by_limit ? static_cast<int64_t>(qlist.size()) : 0); ++k) {
+    const TuneCost* ck = &cost[k * kNumClasses];
+    int n = n_front[k];
+    if (n == 0 || ck[front[k * kNumClasses]].ps >= 1e140) continue;
+    for (int i = 0; i < kTuneLimits; ++i) {
+      n = tuning_under(ck, &front[k * kNumClasses], n, limits[i]) + 1;
+      const TuneCost& x = ck[front[k * kNumClasses + n - 1]];
+      cells_ps[i] += x.ps;
+      rounds[i] += x.rounds;
+      path_ps[i] = std::max(path_ps[i], x.path);
+    }
+  }
+  int limit = 0;
+  double least = 1e300;
+  for (int i = 0; i < kTuneLimits; ++i) {
+    const double t = tune_batch_time(cells_ps[i], path_ps[i], rounds[i], c->sms);
+    if (t < least) {
+      least = t;
+      limit = i;
+    }
+  }
+  for (size_t k = 0; k < qlist.size(); ++k) {
+    const TuneCost* ck = &cost[k * kNumClasses];
+    const uint8_t* fk = &front[k * kNumClasses];
+    if (n_front[k] == 1) {
+      qclass[k] = fk[0];  // forced, or no choice
+    } else if (n_front[k] == 0) {  // no class stages it: the wavefront model
+      qclass[k] = tuning_pick_single(&c->tuning, c->profs[qlist[k]].m, tlen[byq[qstart[qlist[k]]]]);
+    } else {
+      qclass[k] = by_limit ? fk[tuning_under(ck, fk, n_front[k], limits[limit])] : tuning_weighed(ck, batch_ps);
+    }
   }
   int toolong = -1;
   double class_path[kNumClasses] = {};
@@ -2318,6 +2378,8 @@ static int dplan_build(st_ctx* c, const st_pair* pairs, uint64_t n, int32_t open
   const uint32_t gq32 = static_cast<uint32_t>((static_cast<uint64_t>(n_prof) * 32 + 255) / 256);
   const uint32_t gq = static_cast<uint32_t>((np1 + 255) / 256);
   dp_estimate_kernel<<<n_prof, 256, 0, s1>>>(in1, w, cls);
+  dp_path_kernel<<<gq32, 256, 0, s1>>>(in1, w, cls);
+  dp_limit_kernel<<<gq32, 256, 0, s1>>>(in1, w, cls);
   dp_pick_kernel<<<gq32, 256, 0, s1>>>(in1, w, cls);
   dp_split_kernel<<<gq32, 256, 0, s1>>>(in1, w, cls);
   cub::DoubleBuffer<uint32_t> qk(w.qkey, w.qkey_alt), qi(w.qid, w.qid_alt);
@@ -2328,7 +2390,7 @@ static int dplan_build(st_ctx* c, const st_pair* pairs, uint64_t n, int32_t open
   ST_CUDA(cub::DeviceScan::ExclusiveSum(tmp, t_scan, w.a_wt, w.o_wt, static_cast<int>(np1), s1));
   ST_CUDA(cub::DeviceScan::ExclusiveSum(tmp, t_scan, w.a_cta, w.o_cta, static_cast<int>(np1), s1));
   ST_CUDA(cudaGetLastError());
-  c->launches += 6;
+  c->launches += 8;
   DpTotals tot;
   uint32_t n_list32 = 0;  // pairs the classify stage sent to the 32-bit kernel
   ST_CUDA(cudaMemcpyAsync(&tot, w.totals, sizeof(DpTotals), cudaMemcpyDeviceToHost, s1));

@@ -1,12 +1,11 @@
 // Tile-class selection for the packed 16-bit kernel: lanes per alignment (G),
 // query rows per lane (R) and columns per step (C).
 //
-// Batches: each query takes the class with the least estimated cost to the
-// batch: the chip's time for its streamed cells (padded rows x padded columns x
-// slots, from its own target lengths, over the class's measured rate; built-in
-// B200 figures, replaced by st_autotune, 0 = class not considered), plus what its
-// critical path exceeds the whole batch by.  A table entry per (query length,
-// mean target length) bin, set by the caller, forces a class for that bin.
+// Batches: each query's classes are weighed by the chip's time for its streamed
+// cells (padded rows x padded columns x slots, from its own target lengths, over
+// the class's measured rate; built-in B200 figures, replaced by st_autotune, 0 =
+// class not considered) and by their critical paths.  A table entry per (query
+// length, mean target length) bin, set by the caller, forces a class for that bin.
 //
 // Single alignments (the per-call path) take the class of the shortest
 // critical path.
@@ -139,17 +138,69 @@ TUNE_HD inline double tune_crit_ps(uint32_t G, uint32_t R, uint32_t C, uint32_t 
   return (steps + G) * (fixed + 11.8 * (R * C)) * (1e6 / 1965.0);
 }
 
-// What a query costs the batch in a class: the chip's time for its cells, plus a part of what its critical path
-// exceeds the whole batch by (batch_ps: the batch's time with every query in its cheapest class).  Large batches
-// are all cell time and take the classes of few lanes, which pad least; in a small one the chip waits for the
-// longest wavefront, so a query of many rows takes more lanes and fewer passes, or a team.  A path counts three
-// times its lone length (a warp shares its scheduler with up to three others for most of its run), and its excess
-// a tenth (the queries that exceed do so side by side).  Measured over factors 0-5 and weights 0.03-3: 100 PSSM
-// queries x 300 targets 2.30 ms without the term, 1.44 with (1.5, 1), 1.10 with (3, 0.1); 600 queries 4.92, 4.83,
-// 4.70 ms; 64 profiles x 1,000 samples 3.74, 2.42, 2.42 ms.
-TUNE_HD inline double tune_objective(double est_ps, double crit_ps, double batch_ps) {
-  const double over = 3.0 * crit_ps - batch_ps;
-  return est_ps + (over > 0.0 ? 0.1 * over : 0.0);
+// What a class costs a query of a batch: the chip's time for its cells, the length of its critical path, and the turns
+// its warp tasks take of an SM's four schedulers.  A large batch is all cell time and takes the classes of few lanes,
+// which pad least; a small one waits for its longest wavefront, so a query of many rows takes more lanes and fewer
+// passes, or a team.  How the two are weighed depends on how alike the paths are (tune_alike).
+struct TuneCost {
+  double est;     // the streamed cells over the rate; >= 1e140: a class without a rate, 1e300: it does not stage the query
+  double ps;      // the same with what a small batch pays beside
+  double path;
+  double rounds;
+};
+
+// nw: warp tasks, in CTAs of W warps.  A wavefront starts and ends with G - 1 steps of idle lanes, once for the warp
+// tasks that a warp streams one after the other: each in a batch that fits the chip (batch_ps, its cell time in the
+// cheapest classes, below the three and a half paths of a full scheduler), up to sixteen in a large one.  And a CTA holds
+// one query, so many queries of a few warp tasks each take the places of the CTAs that fit the chip, two on an SM or
+// three of four warps or eight rows a lane.
+TUNE_HD inline TuneCost tune_cost(uint32_t G, uint32_t R, uint32_t C, uint32_t W, bool team, uint32_t P,
+                                  uint32_t longest_cols, uint32_t nw, double est_ps, double rate, double batch_ps,
+                                  uint32_t sms) {
+  TuneCost r{est_ps, est_ps, tune_crit_ps(G, R, C, P, longest_cols, team ? W : 1), 0.0};
+  r.rounds = team ? nw * (W / 4) : nw / W * (W / 4) + (nw % W + 3) / 4;
+  if (est_ps < 1e140) {
+    const double streamed = batch_ps / (3.5 * r.path);
+    const double ramp = 64.0 * R * C * (G - 1) * nw / rate;  // a step is 64 R C cells of a warp
+    r.ps += ramp / (streamed < 1.0 ? 1.0 : (streamed > 16.0 ? 16.0 : streamed));
+    const double place = r.path / ((W < 8 || R == 8 ? 3.0 : 2.0) * sms) * (team ? nw : 1u);
+    if ((team || nw < W) && place > r.ps) r.ps = place;
+  }
+  return r;
+}
+
+// Paths of mixed lengths: each query is weighed by itself, the time of its cells and a tenth of what its path exceeds the
+// whole batch by.  A path counts three times its lone length (a warp shares its scheduler with up to three others for
+// most of its run), and a tenth because the queries that exceed do so side by side.  100 PSSM queries x 300 targets 2.30
+// ms without the second term, 1.10 with it; 600 queries 4.92 and 4.70 ms.
+TUNE_HD inline bool tune_waits(double path, double batch_ps) { return 3.0 * path > batch_ps; }
+TUNE_HD inline double tune_weighed(const TuneCost& c, double batch_ps) {
+  return c.est + (tune_waits(c.path, batch_ps) ? 0.1 * (3.0 * c.path - batch_ps) : 0.0);
+}
+
+// Paths much alike, the longest (of the queries in their cheapest classes) within a quarter of the mean, and most of
+// them waited for: that would count one path once for each query.  The batch has one limit for the paths instead: each query
+// takes the class of least time whose path is within it (the shortest path where none is), and the limit is the one of
+// the least estimate of the batch's time, from the sums of its queries' times and rounds and its longest path.  That
+// wavefront shares its scheduler with as many others as there are rounds, up to two more, and a third of what is the
+// shorter of its time and the cells' comes on top.  Microseconds with each query by itself / with a limit: 64 queries x
+// 60 targets of 250 x 300 132 / 101, 100 x 100 303 / 255, 300 x 50 of 100 x 160 162 / 116, 64 x 60 of 600 x 300 274 / 230.
+// With mixed lengths the limit lost as much as it won: 16 x 300 766 / 717, 100 x 300 1,375 / 1,740.
+TUNE_HD inline bool tune_alike(double longest_path, double path_sum, uint64_t n, uint64_t n_wait) {
+  return 2 * n_wait > n && longest_path * n <= 1.25 * path_sum;
+}
+TUNE_HD inline double tune_batch_time(double cells_ps, double path_ps, double rounds, uint32_t sms) {
+  const double load = rounds / sms;
+  const double path = path_ps * (load < 1.0 ? 1.0 : (load > 3.0 ? 3.0 : load));
+  return cells_ps > path ? cells_ps + path / 3.0 : path + cells_ps / 3.0;
+}
+
+// The limits that are compared: the longest path of the queries in their cheapest classes, and down from it in steps of
+// a tenth.
+constexpr int kTuneLimits = 32;
+TUNE_HD inline double tune_limit(double longest, int i) {
+  for (; i > 0; --i) longest *= 0.9;
+  return longest;
 }
 
 // Warp tasks per unit of a CTA task: a CTA's warps; one on each scheduler where the batch has not two CTAs of them for
@@ -186,28 +237,64 @@ inline double tuning_estimate(const Tuning* t, uint32_t m, const uint32_t* tlen_
   return best;
 }
 
-// The class of one query of a batch (longest: its longest target); -1 when none stages it.
-inline int tuning_pick_batch(const Tuning* t, uint32_t m, uint32_t longest, uint32_t mean_n, const double* est,
-                             double batch_ps) {
+// The class that the table forces on a query, -1: none, or it does not stage the query.
+inline int tuning_forced(const Tuning* t, uint32_t m, uint32_t mean_n, const double* est) {
   const int forced = t->table[tune_mbin(m)][tune_nbin(mean_n)];
-  if (forced >= 0 && forced < st_tuning_num_classes() && est[forced] < 1e300) return forced;
-  int best = -1;
-  double bt = 1e300;
+  return forced >= 0 && forced < st_tuning_num_classes() && est[forced] < 1e300 ? forced : -1;
+}
+
+// Every class's cost for a query of m rows, n targets of which the longest has `longest` residues, from its estimates.
+inline void tuning_costs(const Tuning* t, uint32_t m, uint32_t longest, size_t n, const double* est, double batch_ps,
+                         uint32_t sms, TuneCost* cost) {
   for (int c = 0; c < st_tuning_num_classes(); ++c) {
-    if (est[c] >= 1e300) continue;
     int G, R, C;
     st_tuning_class_shape(c, &G, &R, &C);
-    const uint32_t rows = static_cast<uint32_t>(G * R), P = (m + rows - 1) / rows;
+    const uint32_t rows = static_cast<uint32_t>(G * R), P = (m + rows - 1) / rows, S = static_cast<uint32_t>(64 / G);
     const uint32_t minc = P > 1 ? std::max<uint32_t>(32, (static_cast<uint32_t>(C * G) + 15) & ~15u) : 32u;
-    const double crit = tune_crit_ps(G, R, C, P, std::max<uint32_t>(minc, (longest + 3) & ~3u),
-                                     st_tuning_class_team(c) ? st_tuning_class_warps(c) : 1);
-    const double v = tune_objective(est[c], crit, batch_ps);
-    if (v < bt) {
-      bt = v;
-      best = c;
-    }
+    cost[c] = tune_cost(G, R, C, st_tuning_class_warps(c), st_tuning_class_team(c), P,
+                        std::max<uint32_t>(minc, (longest + 3) & ~3u), static_cast<uint32_t>((n + S - 1) / S), est[c],
+                        t->rate[c], batch_ps, sms);
   }
+}
+
+// The classes that some limit picks for a query, shortest path first and each cheaper than those before it: under a limit
+// the query takes the last whose path is within it, or the first.  Without a class that has a rate the cheapest that
+// stages the query alone.  Returns their number (0: none stages it).
+inline int tuning_front(const TuneCost* cost, uint8_t* front) {
+  uint8_t order[kMaxTileClasses];  // the classes with a rate by path, then time
+  int m = 0, unrated = -1;
+  for (int c = 0; c < st_tuning_num_classes(); ++c) {
+    if (cost[c].ps >= 1e140) {
+      if (cost[c].ps < 1e300 && (unrated < 0 || cost[c].ps < cost[unrated].ps)) unrated = c;
+      continue;
+    }
+    int i = m++;
+    for (; i > 0; --i) {
+      const TuneCost& o = cost[order[i - 1]];
+      if (o.path < cost[c].path || (o.path == cost[c].path && o.ps <= cost[c].ps)) break;
+      order[i] = order[i - 1];
+    }
+    order[i] = static_cast<uint8_t>(c);
+  }
+  int n = 0;
+  for (int i = 0; i < m; ++i)
+    if (n == 0 || cost[order[i]].ps < cost[front[n - 1]].ps) front[n++] = order[i];
+  if (n == 0 && unrated >= 0) front[n++] = static_cast<uint8_t>(unrated);
+  return n;
+}
+
+// The class of a query by its own weight (tune_weighed); -1 when none stages it.
+inline int tuning_weighed(const TuneCost* cost, double batch_ps) {
+  int best = -1;
+  for (int c = 0; c < st_tuning_num_classes(); ++c)
+    if (cost[c].est < 1e300 && (best < 0 || tune_weighed(cost[c], batch_ps) < tune_weighed(cost[best], batch_ps))) best = c;
   return best;
+}
+
+// Its place among them under a limit.
+inline int tuning_under(const TuneCost* cost, const uint8_t* front, int n, double limit) {
+  while (n > 1 && cost[front[n - 1]].path > limit) --n;
+  return n - 1;
 }
 
 // The class in which a lone alignment of m rows and n columns is done first.

@@ -43,9 +43,23 @@ int main() {
     for (int i = 0; i < kTuneMBins; ++i)
       for (int j = 0; j < kTuneNBins; ++j) t.table[i][j] = 0;  // the class of the fewest rows, forced
     const double batch = tuning_estimate(&t, m, &len, 1, est, 0xFFFFFFFFu);
-    const int c = tuning_pick_batch(&t, m, len, len, est, batch);
-    if (c < 0 || !passes_ok(c, m)) ++bad;
+    const int c = tuning_forced(&t, m, len, est);
+    if (c >= 0 && !passes_ok(c, m)) ++bad;
     forced += c == 0;
+    TuneCost cost[kN];
+    uint8_t front[kMaxTileClasses];
+    tuning_costs(&t, m, len, 1, est, batch, 148, cost);
+    const int n = tuning_front(cost, front);
+    if (n == 0) ++bad;
+    for (int i = 0; i < n; ++i) {
+      if (!passes_ok(front[i], m)) ++bad;
+      // shorter paths cost more, and a limit picks the cheapest class whose path is within it
+      if (i && !(cost[front[i - 1]].path < cost[front[i]].path && cost[front[i - 1]].ps > cost[front[i]].ps)) ++bad;
+      if (front[tuning_under(cost, front, n, cost[front[i]].path)] != front[i]) ++bad;
+      for (int k = 0; k < kN; ++k)
+        if (cost[k].path <= cost[front[i]].path && cost[k].ps < cost[front[i]].ps) ++bad;
+    }
+    if (n && front[tuning_under(cost, front, n, 0.0)] != front[0]) ++bad;
   }
   std::printf("%%d %%d\n", bad, forced);
 }
