@@ -387,6 +387,7 @@ struct st_ctx {
   std::vector<std::unique_ptr<CallSlot>> call_slots;
   std::vector<CallSlot*> call_idle;
   Tuning tuning;
+  uint32_t team_spins = kTeamSpins;  // ST_TEAM_SPINS, for tests
   uint32_t end_ready[2] = {};  // end-cell kernels (forward, reverse) whose shared memory is set, a bit per tile class
   // seed index over the database (st_seed_index_build): offsets of the 20^w codes, postings
   DevMem seed_off, seed_post;
@@ -716,6 +717,7 @@ extern "C" st_ctx* st_init(int device, size_t hbm_budget_bytes) {
   c->sms = prop.multiProcessorCount;
   c->mt.budget = hbm_budget_bytes;
   c->mt.fail_above = env_u64("ST_ALLOC_FAIL_ABOVE", SIZE_MAX);
+  c->team_spins = static_cast<uint32_t>(std::min<uint64_t>(env_u64("ST_TEAM_SPINS", kTeamSpins), kTeamSpins));
   if (cudaStreamCreateWithFlags(&c->own, cudaStreamNonBlocking) != cudaSuccess) {
     fail(ST_ECUDA, "cudaStreamCreate failed");
     return nullptr;
@@ -2004,6 +2006,7 @@ static int plan_build(st_ctx* c, const st_pair* pairs, uint64_t n, int32_t open,
     prm.scratch_stride = cp.scratch_stride;
     prm.open = open;
     prm.ext = ext;
+    prm.team_spins = c->team_spins;
   }
   {
     Sw32Params& p32 = plan->p32;
@@ -2513,6 +2516,7 @@ static int dplan_build(st_ctx* c, const st_pair* pairs, uint64_t n, int32_t open
     prm.scratch_stride = cp.scratch_stride;
     prm.open = open;
     prm.ext = ext;
+    prm.team_spins = c->team_spins;
   }
   Sw32Params& p32 = plan->p32;
   p32.db = db;
@@ -3132,6 +3136,7 @@ extern "C" int st_sw_align_span_pairs(st_ctx* c, const st_pair* pairs, uint64_t 
 struct SwCall {
   uint32_t profile = 0, n = 0, k = 0, P = 1, rows = 0, ncols = 0, sstride = 0;
   int32_t open = 0, ext = 0;
+  uint32_t team_spins = 0;
   bool use16 = false, wait = false;
   size_t tbytes = 0, o_off = 0, o_len = 0, o_pt = 0, o_pq = 0, o_pc = 0, o_pr = 0, o_cta = 0, o_wt = 0, o_slots = 0,
          o_cnt = 0, o_list = 0, total = 0;
@@ -3158,6 +3163,7 @@ static int sw_score_prepare(st_ctx* c, CallSlot* sl, uint32_t profile, uint32_t 
   w->n = n;
   w->open = open;
   w->ext = ext;
+  w->team_spins = c->team_spins;
   w->tbytes = up16(n) + 32;
   size_t o = w->tbytes;
   w->o_off = o; o += 8;
@@ -3298,6 +3304,7 @@ static int sw_score_launch(CallSlot* sl, const uint8_t* target, const SwCall& w,
     prm.scratch_stride = w.sstride;
     prm.open = w.open;
     prm.ext = w.ext;
+    prm.team_spins = w.team_spins;
     kClasses[w.k].fn<<<1, kClasses[w.k].W * 32, kProfRows * w.P * w.rows, st>>>(prm);
   }
   if (!w.use16) ST_TRY(sw_score_launch32(sl, w));

@@ -108,6 +108,7 @@ struct Sw16Params {
   uint2* scratch;         // pass boundary rows, scratch_stride entries per group
   uint32_t scratch_stride;
   int32_t open, ext;
+  uint32_t team_spins;    // team form: polls of a producer's count before a team gives its pair up
   // end-cell modes: end cell (query, target) of each pair, -1 for a zero score; in the reverse mode the end of
   // the reversed prefix [0, rev_q] x [0, rev_t] whose forward score is rev_score
   int32_t* end_q = nullptr;
@@ -130,7 +131,7 @@ constexpr uint32_t kCtlFirst = 1u << 28;  // first step of a pass
 constexpr uint32_t kCtlMore = 1u << 29;   // a pass that is not the last: its bottom row is kept
 constexpr uint32_t kMaxPasses16 = 256;    // passes that bits 16-23 can name; the planners admit no more
 constexpr int kSlotRing = 8;
-constexpr uint32_t kTeamSpins = 1u << 22;  // polls of a producer's count before a team gives its pair up
+constexpr uint32_t kTeamSpins = 1u << 22;  // the default of Sw16Params::team_spins
 
 template <int G, int R, int C>
 struct Sw16Tile {
@@ -478,7 +479,7 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 4 || (R == 8 && MODE == k
       const uint32_t need = static_cast<uint32_t>((u_pass - 1) / WARPS) * team_cols + u_col + C;
       if (seen < need) {
         for (uint32_t spin = 0; (seen = s_prog[from]) < need && s_fail == 0; ++spin)
-          if (spin >= kTeamSpins) s_fail = 1;
+          if (spin >= prm.team_spins) s_fail = 1;
         __threadfence_block();
       }
       load_bnd<C>(true, prm.scratch + static_cast<size_t>(blockIdx.x * WARPS + from) * prm.scratch_stride + u_col,
