@@ -537,18 +537,6 @@ static int side_stream(st_ctx* c, cudaStream_t* out) {
   return ST_OK;
 }
 
-// Orders the context's stream after the last profile build and, when
-// profiles were created or freed since, refreshes the device tables of
-// profile pointers, strides and lengths. The tables go up on the stream from
-// a ring of pinned blocks, so work already queued keeps reading the old ones.
-// Waits for every per-call scoring in flight (before memory they may read is reallocated).
-static int calls_drain(st_ctx* c) {
-  std::lock_guard<std::mutex> lk(c->call_mu);
-  for (auto& sl : c->call_slots)
-    if (sl->s) ST_CUDA(cudaStreamSynchronize(sl->s));
-  return ST_OK;
-}
-
 static CallSlot* call_acquire(st_ctx* c) {
   std::unique_lock<std::mutex> lk(c->call_mu);
   for (;;) {
@@ -573,6 +561,10 @@ static void call_release(st_ctx* c, CallSlot* sl) {
   c->call_cv.notify_one();
 }
 
+// Orders the context's stream after the last profile build and, when
+// profiles were created or freed since, refreshes the device tables of
+// profile pointers, strides and lengths. The tables go up on the stream from
+// a ring of pinned blocks, so work already queued keeps reading the old ones.
 static int sync_profiles(st_ctx* c) {
   if (c->prof_ev_set) {
     ST_CUDA(cudaStreamWaitEvent(c->stream, c->prof_ev, 0));
@@ -613,10 +605,8 @@ static int sync_profiles(st_ctx* c) {
   auto up = [&](DevMem& d, size_t off, size_t bytes) -> int {
     if (d.bytes < bytes) {
       ST_CUDA(cudaStreamSynchronize(c->stream));  // queued work may read the old table
-      // and so may per-call scorings: none is between its checks and its launches (they hold the call
-      // lock shared), and those launched are waited for
+      // and so may per-call scorings, which hold the call lock shared from their checks to their results
       std::unique_lock<std::shared_mutex> calls(c->call_rw);
-      ST_TRY(calls_drain(c));
       ST_TRY(dev_alloc(&c->mt, d, bytes * 2));
     }
     ST_CUDA(cudaMemcpyAsync(d.p, h + off, bytes, cudaMemcpyHostToDevice, c->stream));
@@ -3124,7 +3114,7 @@ extern "C" int st_sw_align_span_pairs(st_ctx* c, const st_pair* pairs, uint64_t 
 }
 
 // ---------------------------------------------------------------------------
-// plain per-call SW (one pair, one launch of each kernel, blocking)
+// plain per-call SW (one pair, one launch, blocking; a second one for a pair past the 16-bit headroom)
 // ---------------------------------------------------------------------------
 // One per-call scoring on slot `sl`, in two phases.  sw_score_prepare runs under the context lock: the
 // checks, the profile tables, the sizes, the slot's buffers (device memory is accounted to the context) and,

@@ -173,14 +173,12 @@ __device__ __forceinline__ void load_rows8(const int8_t* p, uint32_t (&w)[R / 4]
 // `on`.  A predicated load: the lanes that do not feed the stream pass it without a branch.
 template <int C>
 __device__ __forceinline__ uint32_t load_codes(bool on, const uint8_t* t, uint32_t len16, int c) {
-  uint32_t v = 0x15151515u & (C == 4 ? 0xFFFFFFFFu : (C == 2 ? 0xFFFFu : 0xFFu));
+  uint32_t v = 0x15151515u & (C == 4 ? 0xFFFFFFFFu : 0xFFFFu);
   const uint32_t p = on && static_cast<uint32_t>(c) < len16;
   if constexpr (C == 4)
     asm volatile("{ .reg .pred q; setp.ne.u32 q, %2, 0; @q ld.global.nc.u32 %0, [%1]; }" : "+r"(v) : "l"(t + c), "r"(p));
-  else if constexpr (C == 2)
-    asm volatile("{ .reg .pred q; setp.ne.u32 q, %2, 0; @q ld.global.nc.u16 %0, [%1]; }" : "+r"(v) : "l"(t + c), "r"(p));
   else
-    asm volatile("{ .reg .pred q; setp.ne.u32 q, %2, 0; @q ld.global.nc.u8 %0, [%1]; }" : "+r"(v) : "l"(t + c), "r"(p));
+    asm volatile("{ .reg .pred q; setp.ne.u32 q, %2, 0; @q ld.global.nc.u16 %0, [%1]; }" : "+r"(v) : "l"(t + c), "r"(p));
   return v;
 }
 
@@ -274,7 +272,7 @@ __device__ __forceinline__ uint32_t rows_from(int nz, int v) {
 
 // Persistent kernel: CTAs pull CTA tasks (one query each) from a global
 // counter and stage the query's int8 profile in shared memory; each warp then
-// streams the CTA task's warp tasks, claimed from a shared counter.
+// streams the CTA task's warp tasks, its first by its number and the others claimed from a shared counter.
 //
 // Beside the cells a step costs its 3 + 2C shuffles, the residues' row offsets
 // (one dot product each, dot_byte) and the feeder's loads and stores, which are
