@@ -424,12 +424,13 @@ int st_sw_align_span_pairs(st_ctx* ctx, const st_pair* pairs, uint64_t n, int32_
 /* ---- tile classes and autotuning ----------------------------------------- */
 /* The packed 16-bit kernel runs in tile classes: G lanes per alignment x R
  * query rows per lane x C target columns per wavefront step.  In a batch each
- * query takes the class with the least estimated time: its streamed cells
- * (padded rows x padded columns) over the class's rate (streamed cells per
- * second / 1e12; built-in B200 figures until st_autotune measures them; a rate
- * of 0 leaves the class out).  A per-context table maps (query-length bin,
- * mean target-length bin) to a class that is then forced; -1 entries (the
- * default) use the rates.  Query bins: <=32, <=64, ..., <=8192, >8192 (10);
+ * query's class is picked by its estimated time, its streamed cells (padded
+ * rows x padded columns) over the class's rate (streamed cells per second /
+ * 1e12; built-in B200 figures until st_autotune measures them; a rate of 0
+ * leaves the class out), and by how long the batch would wait for its longest
+ * wavefront.  A per-context table maps (query-length bin, mean target-length
+ * bin) to a class that is then forced, unless it cannot stage the query; -1
+ * entries (the default) use the rates.  Query bins: <=32, <=64, ..., <=8192, >8192 (10);
  * target bins: <=64, <=128, ..., <=4096, >4096 (8); the table is row-major
  * [10][8].  (No reference counterpart: the reference picks SIMD widths at run
  * time, src/simd.rs:59-124.) */
